@@ -40,9 +40,28 @@ enum PassMap : int {
 // 2047 GO; kOut16None marks an empty slot.
 constexpr uint16_t kOut16None = 0xFFFFu;
 constexpr uint32_t kOut16MaxGO = 2047u;
-// GR->GO slot planes the per-tile pass streams when some GR has more synapses
-// (the rest go to per-tile lists).
+// The persistent pass streams every GR->GO slot; it refuses networks with
+// more than this many on some GR.
 constexpr uint32_t kOutInline = 4u;
+
+// Steps in the ring of GR->GO counts: a spike of step t reaches slots t ..
+// t + 31, while the small-cell update of step t reads and clears slot t - 1.
+constexpr uint32_t kGoRing = 64u;
+// Cells of a block of the event lists, an unused entry of a list (a dummy counter
+// behind the block's), an unused item, the items an event CTA lists at a time and
+// its shared memory, and the spiking cells a streaming
+// CTA lists at a time.
+constexpr uint32_t kEvCells = 16384u;
+constexpr uint32_t kEvUnused = kEvCells;
+constexpr uint32_t kEvNone = 0xFFFFFFFFu;
+constexpr uint32_t kEvListCap = 1024u;
+constexpr uint32_t kEvRoleBytes = 128u + 16u + kEvCells + 16u + 4u * kEvListCap;
+constexpr uint32_t kEvCellCap = 256u;
+// Delay field of the last entry of a cell's GR->GO row whose synapses go on in
+// another one.
+constexpr uint32_t kOutMore = 0xFEu;
+// Largest tile of the per-tile pass.
+constexpr uint32_t kEvMaxTile = 16384u;
 
 // A step's MF spike words passed by value to the step's kernels (one
 // network launched a step at a time: the host packs the caller's input and
@@ -94,6 +113,43 @@ CBM_LAYOUT_FN PassLayout passLayout(uint32_t R, uint32_t nMF, uint32_t nGO, uint
 	L.txBase = 6 * row4 + 64u * R * mfS + 64u * R * goS + 32u * outBytes * R * outS + 32u * R + row4 * Z;
 	L.txHist = 256u * R;
 	return L;
+}
+
+// One stage of the per-tile pass: SC cells of the six state arrays (from 0),
+// then every zone's weights, the PF delays and the arrived spikes.
+struct EventLayout {
+	uint32_t w, pfDelay, cnt, bytes;  // region offsets, stage size
+	uint32_t tx;                      // bytes the stage's copies deliver
+};
+CBM_LAYOUT_FN EventLayout eventLayout(uint32_t SC, uint32_t Z)
+{
+	EventLayout L;
+	L.w = 24u * SC;
+	L.pfDelay = L.w + 4u * SC * Z;
+	L.cnt = L.pfDelay + SC;
+	L.bytes = L.tx = L.cnt + SC;  // a multiple of 128
+	return L;
+}
+
+// Its shared memory after 128-byte alignment: barriers, plasticity steps per
+// PC and zone, BC and SC counts, the step's spikes (a bit a cell), a list of
+// spiking cells (u16), the PF->PC outputs, and the stages.
+constexpr uint32_t kEvBarBytes = 128u;
+struct EventSmem {
+	uint32_t step, bc, spk, cells, x, stages, bytes;
+};
+CBM_LAYOUT_FN EventSmem eventSmem(uint32_t S, uint32_t stageBytes, uint32_t TC, uint32_t Z, uint32_t pcs, uint32_t counts)
+{
+	EventSmem M;
+	uint32_t o = kEvBarBytes;
+	M.step = o; o += (4u * pcs * Z + 15u) & ~15u;
+	M.bc = o; o += (4u * counts + 15u) & ~15u;
+	M.spk = o; o += TC / 8u;
+	M.cells = o; o += 2u * kEvCellCap;
+	M.x = o; o += 4u * TC * Z;
+	M.stages = o = align128(o);
+	M.bytes = o + S * stageBytes;
+	return M;
 }
 
 // Values the host may change between steps (setter calls of the reference's
@@ -186,7 +242,6 @@ struct DevNet {
 	uint32_t P, bs, K, J, tilesPerPC;     // PF->PC reduction geometry (kernels.cu:435-470)
 	uint32_t bcShift, scShift, bcLocal, scLocal;
 	uint32_t nMFSlots, nGOSlots, nOutSlots;
-	uint32_t nOutTma;                     // GR->GO slot planes the per-tile TMA pass streams (the rest: ovStart)
 	uint32_t mfWords, goWords;            // spike-bit vectors incl. the always-zero sentinel
 	uint32_t maxnumpMFfromMFtoGO, maxnumpGOCoupInGOGO;
 	uint32_t numpPCfromSCtoPC, numpNCfromPCtoNC, numpNCfromMFtoNC, numpIOfromNCtoIO, numpIOInIOIO;
@@ -226,11 +281,26 @@ struct DevNet {
 	const uint16_t *goIdx;    // [nGOSlots][numGR], sentinel numGO
 	const uint32_t *outCon;   // [nOutSlots][numGR]: (GO << 8) | delay bit, kNoDelay when empty
 	const uint16_t *outCon16; // the same as 16-bit entries (kOut16None when empty), or null (> 2047 GO)
-	// GR->GO synapses in slots >= nOutTma, per TMA-pass tile (null when none):
-	// tile b's are ovEntry[ovStart[b] .. ovStart[b+1]), x = tile-local cell
-	// (row * 32 + lane) | delay bit << 24, y = GO
-	const uint32_t *ovStart;
-	const uint2 *ovEntry;
+	// per-tile pass: a tile is evRows rows of 1 << evWdShift cells of the
+	// [numGR / bs][bs] view, evTilesX tiles side by side; evPCs PCs, evBC BC
+	// and evSC SC blocks in a tile.  While it runs, vGR, gKCaGR, threshGR, gESum,
+	// gISum, apBufGR, historyGR and the zones' w are in tile order (tile by tile,
+	// row by row), as the arrays below always are
+	uint32_t evWdShift, evRows, evTilesX, evTiles, evPCs, evBC, evSC;
+	uint32_t evPerMF, evPerGO;  // items of 64 cells a usual list is cut into
+	// block b's target cells of source s (MF, then GO), by eights (u16):
+	// evEntry[evStart[b (numMF + numGO + 1) + s] .. evStart[.. + s + 1]),
+	// padded with kEvUnused
+	const uint32_t *evStart;
+	const uint4 *evEntry;
+	// a cell's GR->GO synapses, four a row as outCon's entries; a row whose last
+	// entry has delay kOutMore goes on in row (entry >> 8) of outMore
+	const uint4 *outCell, *outMore;
+	const uint8_t *evPfDelay;  // pfDelay
+	uint32_t outNow;           // some GR->GO synapse has delay 0: spikes are delivered in their own step
+	uint32_t *spkBits;         // [2][tiles][cells / 128][4]: spikes of the step of that parity (bit i of word c: cell 4 i + c)
+	uint8_t *evCnt;            // [2][numGR] spikes that arrived in the step of that parity: MF | GO << 4
+	uint64_t evFirst;          // the first step of the pass: gESum, gISum are final before it, later one step behind
 	const uint8_t *pfDelay;   // delay bit of the PF->BC/SC/PC output, kNoDelay when none
 
 	// ---- GO / MF / SC state (innetactivitystate.h)
@@ -251,7 +321,7 @@ struct DevNet {
 	uint64_t *pairStep;  // [2] the step whose PF->PC pair sums each pairSum slot holds (vector GR pass)
 	uint32_t *passClaim; // [3] work counters of the vector GR pass, per step mod 3
 	uint32_t *pcDone;    // [numPC] reduction chunks of the previous step done per PC (vector GR pass)
-	uint32_t *goCount;   // [2][numGO] GR->GO input counts per step parity
+	uint32_t *goCount;   // [kGoRing][numGO] GR->GO input counts per step of arrival
 	uint32_t *bcCount;   // [3][numBC] PF->BC counts
 	uint32_t *scCount;   // [3][numSC] PF->SC counts
 	uint32_t *goBits;    // [2][goWords] GO spikes per step parity

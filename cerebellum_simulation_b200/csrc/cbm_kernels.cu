@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(kPassThreads) grPassKernel(const DevNet *const
 	const float gLeak = N->gLeakGR, eLeak = N->eLeakGR, eGOIn = N->eGOGR;
 	const float threshBase = N->threshRestGR, threshMax = N->threshMaxGR, threshDecay = N->threshDecGR;
 	const float gDecMF = N->gDecMFtoGR, gIncMF = N->gIncMFtoGR, gDecGO = N->gDecGOtoGR, gIncGO = N->gIncGOtoGR;
-	uint32_t *goCount = N->goCount + (size_t)(t & 1) * N->numGO;
+	uint32_t *goCount = N->goCount + (size_t)(t & (kGoRing - 1u)) * N->numGO;
 	const uint32_t bcBase = (pc * P) >> N->bcShift, scBase = (pc * P) >> N->scShift;
 	const bool bcWarpUniform = (1u << N->bcShift) >= J, scWarpUniform = (1u << N->scShift) >= J;
 
@@ -392,15 +392,6 @@ __global__ void __launch_bounds__(kPassThreads) grPassKernel(const DevNet *const
 	}
 }
 
-// ------------------------------------------------------------ GR pass, TMA
-// The same tile and per-cell work as grPassKernel for networks whose
-// reduction width bs is at least 32 (tiles of 32-cell rows), with the tile's
-// input rows streamed by TMA: one producer warp copies R = W*RW rows x 32
-// cells of every GR array per stage into an S-deep ring of shared-memory
-// stages; each of the W consumer warps updates RW rows of a stage, reading
-// its inputs from shared memory and writing the new state straight to global
-// memory.  Waits are bounded (kPassWaitLimitNs); a time-out sets
-// kErrPassWait in the network's error word, which the host reports.
 constexpr uint64_t kPassWaitLimitNs = 2000000000ull;
 
 // Slot loops: MS > 0 compiles them for at most MS synapse slots per cell
@@ -418,384 +409,6 @@ __device__ __forceinline__ int countSpikes(const uint8_t *spikes, const uint16_t
 		for (uint32_t s = 0; s < n; s++) c += spikes[idx[s * stride]];
 	}
 	return c;
-}
-
-// Network shapes the TMA pass can be compiled for: slot counts, zones and
-// whether every 32-cell row feeds a single BC and a single SC become
-// compile-time constants (shared-memory offsets fold into immediates, slot
-// loops lose their predicates).  Shape 0 reads them at run time.
-template <int SH> struct PassShape {
-	static constexpr uint32_t mf = 0, go = 0, out = 0, z = 0;
-	static constexpr bool uniform = false, out16 = false;
-};
-// 4 MF and 3 GO dendrites, 4 GR->GO slots (streamed as the 16-bit table),
-// one zone, BC and SC blocks of at least 32 cells (the eyelid networks)
-template <> struct PassShape<1> {
-	static constexpr uint32_t mf = 4, go = 3, out = 4, z = 1;
-	static constexpr bool uniform = true, out16 = true;
-};
-
-template <int W, int RW, int S, int MINB, int MS, int SH>
-__global__ void __launch_bounds__(32 * (W + 1), MINB) grPassTmaKernel(const DevNet *const *nets,
-		const uint32_t *blockOffset, int numNets, uint32_t stepOffset, const DevNet *net0,
-		const __grid_constant__ MFParam mfp, uint32_t *exitCount)
-{
-	// the next step's small-cell kernel may launch (it waits for this pass)
-	pdlLaunchDependents();
-	using Sh = PassShape<SH>;
-	constexpr uint32_t R = W * RW;
-	// one network: its descriptor comes as a parameter (a round trip fewer)
-	uint32_t local = blockIdx.x;
-	const DevNet *__restrict__ N = net0 ? net0 : locateNet(nets, blockOffset, numNets, blockIdx.x, local);
-	const uint64_t t = stepsDone(N) + 1 + stepOffset;
-
-	const uint32_t P = N->P, bs = N->bs, K = N->K, Z = Sh::z ? Sh::z : N->numZones;
-	const uint32_t pc = local / N->tilesPerPC;
-	const uint32_t j0 = (local % N->tilesPerPC) * 32u;
-	const uint32_t rows = 2 * K, nStages = rows / R;
-	const uint32_t nMFSlots = Sh::mf ? Sh::mf : N->nMFSlots, nGOSlots = Sh::go ? Sh::go : N->nGOSlots,
-		nOutSlots = Sh::out ? Sh::out : N->nOutTma;
-	const PassLayout L = passLayout(R, nMFSlots, nGOSlots, nOutSlots, Z, Sh::out16 ? 2u : 4u);
-
-	extern __shared__ uint8_t passSmemRaw[];
-	uint8_t *stages = passSmemRaw + ((128u - (tma::smemAddr(passSmemRaw) & 127u)) & 127u);
-	uint64_t *full = reinterpret_cast<uint64_t *>(stages + (size_t)S * L.bytes);
-	uint64_t *empty = full + S;
-	// spikes of this step's MF and last step's GO as one byte per cell (the
-	// sentinel index numMF / numGO reads 0)
-	uint32_t *sBC = reinterpret_cast<uint32_t *>(empty + S);
-	uint32_t *sSC = sBC + N->bcLocal;
-	// 16-byte aligned: the spike tables after it take 16-byte stores
-	float *sX = reinterpret_cast<float *>(sSC + ((N->bcLocal + N->scLocal + 3u) & ~3u) - N->bcLocal);
-	uint8_t *sMF = reinterpret_cast<uint8_t *>(sX + (size_t)Z * rows * 32u);
-	uint8_t *sGO = sMF + 32u * N->mfWords;
-
-	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-	if (threadIdx.x == 0) {
-		for (int s = 0; s < S; s++) {
-			tma::mbarInit(&full[s], 1);
-			tma::mbarInit(&empty[s], W);
-		}
-		tma::fenceBarrierInit();
-	}
-	__syncthreads();
-
-	const bool plastStep = stepMod(t, N->tsPerHistBinGR) == 0;
-	const uint32_t rowBase = pc * rows;  // first row of the tile in the [numGR/bs][bs] view
-	const uint32_t bcBase = (pc * P) >> N->bcShift, scBase = (pc * P) >> N->scShift;
-
-	if (warp == W) {
-		// ---- producer: lane 0 issues the copies; the whole warp takes the
-		// running sums of the PF->PC reduction (sumInputsNew's per-thread
-		// tempSum += x[i] + x[i+bs], kernels.cu:326-362, lane = j) stage by
-		// stage in row order, as each stage is consumed
-		const CUtensorMap *maps = N->passMaps;
-		if (lane == 0)
-			for (int m = 0; m < PM_W0 + (int)Z; m++) tma::prefetchMap(&maps[m]);
-		const uint32_t tx = L.txBase + (plastStep ? L.txHist : 0u);
-		uint32_t issued = 0, slot = 0, phase = 0;
-		bool ok = true;
-		float run[kMaxZones], even[kMaxZones];
-#pragma unroll
-		for (uint32_t z = 0; z < kMaxZones; z++) run[z] = even[z] = 0.0f;
-		auto sumStage = [&](uint32_t sst) {
-			for (uint32_t rr = 0; rr < R; rr++) {
-				const uint32_t r = sst * R + rr;
-#pragma unroll
-				for (uint32_t z = 0; z < kMaxZones; z++) {
-					if (z >= Z) break;
-					const float x = sX[((size_t)z * rows + r) * 32u + lane];
-					if (r & 1u) run[z] += even[z] + x;
-					else even[z] = x;
-				}
-			}
-		};
-		{
-			for (uint32_t st = 0; st < nStages; st++) {
-				// refill number st/S of this slot waits until its previous
-				// contents are consumed (and summed)
-				if (st >= (uint32_t)S) {
-					const bool done = tma::waitBounded(&empty[slot], phase ^ 1u, kPassWaitLimitNs);
-					if (!__all_sync(0xffffffffu, done)) { ok = false; break; }
-					sumStage(st - S);
-				}
-				issued = st + 1;
-				if (lane != 0) { if (++slot == (uint32_t)S) { slot = 0; phase ^= 1u; } continue; }
-				uint8_t *b = stages + (size_t)slot * L.bytes;
-				uint64_t *bar = &full[slot];
-				tma::arriveExpectTx(bar, tx);
-				const int32_t x = (int32_t)j0, y = (int32_t)(rowBase + st * R);
-#pragma unroll
-				for (int m = PM_V; m <= PM_APBUF; m++) tma::load2d(b + (uint32_t)m * 128u * R, &maps[m], x, y, bar);
-				tma::load3d(b + L.mfIdx, &maps[PM_MFIDX], x, y, 0, bar);
-				tma::load3d(b + L.goIdx, &maps[PM_GOIDX], x, y, 0, bar);
-				tma::load3d(b + L.outCon, &maps[Sh::out16 ? PM_OUTCON16 : PM_OUTCON], x, y, 0, bar);
-				tma::load2d(b + L.pfDelay, &maps[PM_PFDELAY], x, y, bar);
-				for (uint32_t z = 0; z < Z; z++) tma::load2d(b + L.w + z * 128u * R, &maps[PM_W0 + z], x, y, bar);
-				if (plastStep) tma::load2d(b + L.hist, &maps[PM_HIST], x, y, bar);
-				if (++slot == (uint32_t)S) { slot = 0; phase ^= 1u; }
-			}
-			__syncwarp();
-			// the last stages, once consumed
-			for (uint32_t st = issued > (uint32_t)S ? issued - S : 0; ok && st < issued; st++) {
-				const bool done = tma::waitBounded(&empty[st % S], (st / S) & 1u, kPassWaitLimitNs);
-				if (!__all_sync(0xffffffffu, done)) { ok = false; break; }
-				sumStage(st);
-			}
-			if (ok) {
-				const uint32_t buf = (uint32_t)(t % 3);
-#pragma unroll
-				for (uint32_t z = 0; z < kMaxZones; z++) {
-					if (z >= Z) break;
-					N->zones[z].pcPartial[((size_t)buf * N->numPC + pc) * bs + j0 + lane] = run[z];
-				}
-			} else if (lane == 0) {
-				raiseError(N, kErrPassWait);
-				// let the copies in flight land before the CTA's shared memory is released
-				for (uint32_t st = issued > (uint32_t)S ? issued - S : 0; st < issued; st++)
-					tma::waitBounded(&full[st % S], (st / S) & 1u, kPassWaitLimitNs);
-			}
-		}
-	} else {
-		// ---- consumers: warp w updates rows w, w+W, ..., w+(RW-1)W of every
-		// stage.  They stage the spike tables while the first copies fly.
-		const uint32_t *mfSrc = N->mfBits + (size_t)stepMod(t - 1, N->mfRing) * N->mfWords;
-		const uint32_t *goSrc = N->goBits + (size_t)((t - 1) & 1) * N->goWords;
-		// one spike word per thread and round (the loads of a round in flight
-		// together), spread to a byte per cell: (nibble * 0x204081) & 0x01010101
-		// moves bit k of a nibble to bit 8k
-		const uint32_t mfWords = N->mfWords, nWords = mfWords + N->goWords;
-		for (uint32_t w0 = 0; w0 < nWords; w0 += 2u * 32u * W) {
-			uint32_t v[2];
-#pragma unroll
-			for (int u = 0; u < 2; u++) {
-				const uint32_t w = w0 + u * 32u * W + threadIdx.x;
-				// MF words from the launch when it carries them (mfp.n > 0)
-				v[u] = w >= nWords ? 0u : w >= mfWords ? __ldg(goSrc + (w - mfWords)) : mfp.n ? mfp.w[w] : __ldg(mfSrc + w);
-			}
-#pragma unroll
-			for (int u = 0; u < 2; u++) {
-				const uint32_t w = w0 + u * 32u * W + threadIdx.x;
-				if (w < nWords) {
-					uint4 *dst = reinterpret_cast<uint4 *>(w < mfWords ? sMF + 32u * w : sGO + 32u * (w - mfWords));
-					uint32_t q[8];
-#pragma unroll
-					for (int k = 0; k < 8; k++) q[k] = (((v[u] >> (4 * k)) & 0xFu) * 0x00204081u) & 0x01010101u;
-					dst[0] = make_uint4(q[0], q[1], q[2], q[3]);
-					dst[1] = make_uint4(q[4], q[5], q[6], q[7]);
-				}
-			}
-		}
-		for (uint32_t i = threadIdx.x; i < N->bcLocal + N->scLocal; i += 32u * W) sBC[i] = 0;
-		asm volatile("bar.sync 1, %0;" ::"r"(32u * W) : "memory");
-		float stepW[kMaxZones];
-#pragma unroll
-		for (uint32_t z = 0; z < kMaxZones; z++) {
-			stepW[z] = 0.0f;
-			if (z < Z && plastStep) {
-				const uint8_t sel = N->zones[z].plastSel[(t & 1) * N->numIO + N->zones[z].ioOfPC[pc]];
-				stepW[z] = plasticityStep(N, t, z, sel);
-			}
-		}
-		const float gLeak = N->gLeakGR, eLeak = N->eLeakGR, eGOIn = N->eGOGR;
-		const float threshBase = N->threshRestGR, threshMax = N->threshMaxGR, threshDecay = N->threshDecGR;
-		const float gDecMF = N->gDecMFtoGR, gIncMF = N->gIncMFtoGR, gDecGO = N->gDecGOtoGR, gIncGO = N->gIncGOtoGR;
-		uint32_t *goCount = N->goCount + (size_t)(t & 1) * N->numGO;
-		const bool bcWarpUniform = Sh::uniform || (1u << N->bcShift) >= 32u;
-		const bool scWarpUniform = Sh::uniform || (1u << N->scShift) >= 32u;
-		float *const vGR = N->vGR, *const gKCaGR = N->gKCaGR, *const threshGR = N->threshGR;
-		float *const gESum = N->gESum, *const gISum = N->gISum;
-		uint32_t *const apBufGR = N->apBufGR;
-		uint64_t *const historyGR = N->historyGR;
-		const uint32_t bcShift = N->bcShift, scShift = N->scShift;
-		const uint32_t gTile = pc * P + j0 + lane;  // this lane's cell in row 0 of the tile
-		uint32_t slot = 0, phase = 0;
-
-		for (uint32_t st = 0; st < nStages; st++) {
-			const bool ready = tma::waitBounded(&full[slot], phase, kPassWaitLimitNs);
-			if (!__all_sync(0xffffffffu, ready)) {
-				if (lane == 0) raiseError(N, kErrPassWait);
-				break;
-			}
-			const uint8_t *b = stages + (size_t)slot * L.bytes;
-			uint32_t pfs[RW];
-#pragma unroll
-			for (int q = 0; q < RW; q++) {
-				const uint32_t rr = warp + q * W;          // row within the stage
-				const uint32_t e = rr * 32u + lane;        // element within a region of R x 32
-				const uint32_t r = st * R + rr;            // row within the tile
-				const uint32_t g = gTile + r * bs;
-				const float *sF = reinterpret_cast<const float *>(b);
-				const float v = sF[0 * 32 * R + e];
-				const float gk = sF[1 * 32 * R + e];
-				const float th = sF[2 * 32 * R + e];
-				const float gE = sF[3 * 32 * R + e];
-				const float gI = sF[4 * 32 * R + e];
-				const uint32_t ab = reinterpret_cast<const uint32_t *>(b)[5 * 32 * R + e];
-				const uint16_t *mfI = reinterpret_cast<const uint16_t *>(b + L.mfIdx) + e;
-				const uint16_t *goI = reinterpret_cast<const uint16_t *>(b + L.goIdx) + e;
-				// the 32-bit slot table at element e (the 16-bit one is indexed from its base)
-				const uint32_t *outC = reinterpret_cast<const uint32_t *>(b + L.outCon) + (Sh::out16 ? 0u : e);
-				const uint32_t d = (b + L.pfDelay)[e];
-				const uint64_t h = plastStep ? reinterpret_cast<const uint64_t *>(b + L.hist)[e] : 0ull;
-				const int cntMF = countSpikes<MS>(sMF, mfI, nMFSlots, 32 * R);
-				const int cntGO = countSpikes<MS>(sGO, goI, nGOSlots, 32 * R);
-
-				// calcActivityGRGPU (kernels.cu:79-110)
-				const float tempV = v + (gLeak + gk * gk * gk * gk) * (eLeak - v) - (gE) * v + (gI) * (eGOIn - v);
-				const float tempThresh = th + (threshBase - th) * threshDecay;
-				const unsigned int tempAP = tempV > tempThresh;
-				const float thN = tempAP * threshMax + (!tempAP) * tempThresh;
-				const float gkd = gk * 0.9999f;
-				const float gkN = tempAP * (gkd + 0.003f) + (!tempAP) * gkd;
-				const uint32_t abN = (ab << 1) | tempAP;
-				// updateGRInOPGPU for MF (this step's spikes) and GO (last step's)
-				const float gEN = gE * gDecMF + gIncMF * (cntMF);
-				const float gIN = gI * gDecGO + gIncGO * (cntGO);
-				vGR[g] = tempV;
-				gKCaGR[g] = gkN;
-				threshGR[g] = thN;
-				gESum[g] = gEN;
-				gISum[g] = gIN;
-				apBufGR[g] = abN;
-				// plasticity (phase 1) before this step's PF->PC output (phase 2)
-				const uint32_t pf = d < 32u ? (abN >> d) & 1u : 0u;
-#pragma unroll
-				for (uint32_t z = 0; z < kMaxZones; z++) {
-					if (z >= Z) break;
-					float w = reinterpret_cast<const float *>(b + L.w)[z * 32 * R + e];
-					if (plastStep) {
-						w = w + ((h & 0x0000008000000000ull) > 0) * stepW[z];
-						w = (w > 0) * w;
-						w = (w > 1) + (w <= 1) * w;
-						N->zones[z].w[g] = w;
-					}
-					sX[((size_t)z * rows + r) * 32u + lane] = w * pf;
-				}
-				if (plastStep) historyGR[g] = (h << 1) | ((abN & 0x0000001Fu) > 0);
-				// GR->GO synapses whose delayed spike arrives now
-				if (abN) {
-					if constexpr (Sh::out16) {
-						const uint16_t *outC16 = reinterpret_cast<const uint16_t *>(outC) + e;
-#pragma unroll
-						for (uint32_t s = 0; s < Sh::out; s++) {
-							const uint32_t c = outC16[s * 32 * R];
-							if (c != kOut16None && ((abN >> (c & 31u)) & 1u)) atomicAdd(&goCount[c >> 5], 1u);
-						}
-					} else if constexpr (MS > 0) {
-#pragma unroll
-						for (uint32_t s = 0; s < (uint32_t)MS; s++) {
-							if (s >= nOutSlots) break;
-							const uint32_t c = outC[s * 32 * R];
-							const uint32_t dl = c & 0xFFu;
-							if (dl < 32u && ((abN >> dl) & 1u)) atomicAdd(&goCount[c >> 8], 1u);
-						}
-					} else {
-#pragma unroll 4
-						for (uint32_t s = 0; s < nOutSlots; s++) {
-							const uint32_t c = outC[s * 32 * R];
-							const uint32_t dl = c & 0xFFu;
-							if (dl < 32u && ((abN >> dl) & 1u)) atomicAdd(&goCount[c >> 8], 1u);
-						}
-					}
-				}
-				pfs[q] = pf;
-			}
-			__syncwarp();
-			if (lane == 0) tma::arrive(&empty[slot]);
-			if (++slot == (uint32_t)S) { slot = 0; phase ^= 1u; }
-#pragma unroll
-			for (int q = 0; q < RW; q++) {
-				const uint32_t pf = pfs[q];
-				const uint32_t g = gTile + (st * R + warp + q * W) * bs;
-				if (!bcWarpUniform) atomicAdd(&sBC[(g >> bcShift) - bcBase], pf);
-				if (!scWarpUniform) atomicAdd(&sSC[(g >> scShift) - scBase], pf);
-				const uint32_t cnt = __popc(__ballot_sync(0xffffffffu, pf != 0));
-				if (lane == 0 && cnt) {
-					const uint32_t base = g - lane;
-					if (bcWarpUniform) atomicAdd(&sBC[(base >> bcShift) - bcBase], cnt);
-					if (scWarpUniform) atomicAdd(&sSC[(base >> scShift) - scBase], cnt);
-				}
-			}
-		}
-	}
-	__syncthreads();
-
-	// GR->GO synapses past the streamed slot planes: their cells' new spike
-	// buffers were written by this CTA before the barrier
-	if (!Sh::out && N->ovStart) {
-		const uint32_t e1 = N->ovStart[local + 1];
-		uint32_t *goCountOv = N->goCount + (size_t)(t & 1) * N->numGO;
-		for (uint32_t e = N->ovStart[local] + threadIdx.x; e < e1; e += blockDim.x) {
-			const uint2 en = N->ovEntry[e];
-			const uint32_t cl = en.x & 0xFFFFFFu, dl = en.x >> 24;
-			const uint32_t g = pc * P + (cl >> 5) * bs + j0 + (cl & 31u);
-			if ((N->apBufGR[g] >> dl) & 1u) atomicAdd(&goCountOv[en.y], 1u);
-		}
-	}
-
-	// the BC and SC counts of the tile (the producer wrote the PF->PC partials)
-	const uint32_t buf = (uint32_t)(t % 3);
-	uint32_t *bcOut = N->bcCount + (size_t)buf * N->numBC;
-	uint32_t *scOut = N->scCount + (size_t)buf * N->numSC;
-	for (uint32_t i = threadIdx.x; i < N->bcLocal + N->scLocal; i += blockDim.x) {
-		const uint32_t c = sBC[i];
-		if (!c) continue;
-		if (i < N->bcLocal) atomicAdd(&bcOut[bcBase + i], c);
-		else atomicAdd(&scOut[scBase + i - N->bcLocal], c);
-	}
-	__syncthreads();
-	passExitWait(exitCount);
-}
-
-// Geometries the host can pick: (consumer warps, rows per warp, stages,
-// minimum resident CTAs per SM, slot bound MS); those with MS = 4 are also
-// compiled for shape 1 (instantiated where passTmaKernelFor takes them).
-#define CBM_PASS_TMA_CONFIGS(X) \
-	X(8, 1, 3, 2, 4) X(8, 1, 3, 3, 4) X(8, 1, 4, 2, 4) X(8, 1, 2, 3, 4) X(4, 1, 4, 4, 4) X(4, 2, 3, 3, 4) X(4, 2, 4, 2, 4) \
-	X(4, 2, 2, 4, 4) X(8, 1, 3, 2, 0) X(4, 1, 4, 1, 0) X(2, 1, 4, 1, 0) X(1, 1, 4, 1, 0)
-#define CBM_PASS_TMA_INST(W, RW, S, B, M) \
-	template __global__ void grPassTmaKernel<W, RW, S, B, M, 0>(const DevNet *const *, const uint32_t *, int, uint32_t, \
-		const DevNet *, const __grid_constant__ MFParam, uint32_t *);
-CBM_PASS_TMA_CONFIGS(CBM_PASS_TMA_INST)
-
-int passTmaConfigCount()
-{
-	int n = 0;
-#define CBM_PASS_TMA_COUNT(w, rw, s, b, m) n++;
-	CBM_PASS_TMA_CONFIGS(CBM_PASS_TMA_COUNT)
-#undef CBM_PASS_TMA_COUNT
-	return n;
-}
-
-void passTmaConfig(int i, int *W, int *RW, int *S, int *B, int *M)
-{
-	int k = 0;
-#define CBM_PASS_TMA_NTH(w, rw, s, b, m) if (k++ == i) { *W = w; *RW = rw; *S = s; *B = b; *M = m; return; }
-	CBM_PASS_TMA_CONFIGS(CBM_PASS_TMA_NTH)
-#undef CBM_PASS_TMA_NTH
-}
-
-const void *passTmaKernelFor(int W, int RW, int S, int B, int M, int shape)
-{
-#define CBM_PASS_TMA_PICK(w, rw, s, b, m) \
-	if (W == w && RW == rw && S == s && B == b && M == m) { \
-		if (shape == 0) return (const void *)&grPassTmaKernel<w, rw, s, b, m, 0>; \
-		if (shape == 1 && m == 4) return (const void *)&grPassTmaKernel<w, rw, s, b, m, (m == 4 ? 1 : 0)>; \
-		return nullptr; \
-	}
-	CBM_PASS_TMA_CONFIGS(CBM_PASS_TMA_PICK)
-#undef CBM_PASS_TMA_PICK
-	return nullptr;
-}
-
-int passShapeOf(const DevNet &h)
-{
-	using E = PassShape<1>;
-	if (h.numZones == E::z && h.nMFSlots == E::mf && h.nGOSlots == E::go && h.nOutSlots == E::out &&
-			(1u << h.bcShift) >= 32u && (1u << h.scShift) >= 32u && h.outCon16)
-		return 1;
-	return 0;
 }
 
 // ----------------------------------------------------- GR pass, persistent
@@ -920,7 +533,7 @@ __global__ void __launch_bounds__(32 * (W + 1), MINB) grPassPersistentKernel(con
 	const float gLeak = N->gLeakGR, eLeak = N->eLeakGR, eGOIn = N->eGOGR;
 	const float threshBase = N->threshRestGR, threshMax = N->threshMaxGR, threshDecay = N->threshDecGR;
 	const float gDecMF = N->gDecMFtoGR, gIncMF = N->gIncMFtoGR, gDecGO = N->gDecGOtoGR, gIncGO = N->gIncGOtoGR;
-	uint32_t *goCount = N->goCount + (size_t)(t & 1) * N->numGO;
+	uint32_t *goCount = N->goCount + (size_t)(t & (kGoRing - 1u)) * N->numGO;
 	const uint32_t buf = (uint32_t)(t % 3);
 	uint32_t *bcOut = N->bcCount + (size_t)buf * N->numBC;
 	uint32_t *scOut = N->scCount + (size_t)buf * N->numSC;
@@ -1128,7 +741,6 @@ __device__ void golgiRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm
 {
 	const uint32_t tid = threadIdx.x, nThr = blockDim.x, lane = tid & 31u;
 	const uint32_t numGO = N->numGO;
-	const uint32_t G = (uint32_t)((t - 1) & 1);
 	uint64_t *sExp2 = reinterpret_cast<uint64_t *>(sm);
 	uint32_t *sMF = sm + 64;
 	uint32_t *sMFGO = sMF + N->mfWords;  // MF->GO input counts of this step
@@ -1141,7 +753,7 @@ __device__ void golgiRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm
 	if (tid < 32) sExp2[tid] = kExp2Tab[tid];
 	__syncthreads();
 
-	uint32_t *goIn = N->goCount + (size_t)G * numGO;
+	uint32_t *goIn = N->goCount + (size_t)((t - 1) & (kGoRing - 1u)) * numGO;
 	uint32_t *goBitsOut = N->goBits + (size_t)(t & 1) * N->goWords;
 	const float gIncGRtoGO = N->ctl->gIncGRtoGO;
 	for (uint32_t base = 0; base < numGO; base += nThr) {

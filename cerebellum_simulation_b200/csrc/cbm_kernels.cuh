@@ -12,10 +12,13 @@ constexpr int kPassThreads = 256;
 constexpr int kTailThreads = 768;
 
 // Programmatic dependent launch between the two kernels of consecutive
-// steps.  Steps launched one at a time run as small-cell(t) -> pass(t) ->
+// steps.  With the per-tile pass, steps run as small-cell(t) -> pass(t) ->
 // small-cell(t+1) -> ..., each launched as the programmatic dependent of the
-// kernel before it, so that the next kernel is resident before its
-// predecessor ends.  Two rules keep that equal to full stream order:
+// kernel before it (one at a time, and in the graphs of chunked runs), so that
+// the next kernel is resident before its predecessor ends.  In graphs whose
+// steps joined both kernels before the next one, a step took 0.6-1.3 us longer
+// (14.2 against 13.6 us on 1M GR, 14.3 against 13.0 on 256K).  Two rules keep
+// that equal to full stream order:
 //  - the small-cell kernel waits for its predecessor (the previous step's
 //    GR pass) before it reads anything, and only then lets its own
 //    dependent (this step's GR pass) launch;
@@ -23,11 +26,11 @@ constexpr int kTailThreads = 768;
 //    (this step's small-cell kernel) before it exits, so that a finished
 //    GR pass means a finished step (passExitWait).
 // A pass lets the next small-cell kernel launch from its start.  Launched
-// without the attribute (CUDA graphs), each wait returns at once.
+// without the attribute (the other passes), each wait returns at once.
 __device__ __forceinline__ void pdlWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdlLaunchDependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // At the end of a GR-pass CTA, after a barrier of the whole CTA: with a
-// counter (chained single steps), the launch's last CTA to get here resets
+// counter (chained steps), the launch's last CTA to get here resets
 // it and waits for the step's small-cell kernel; the others exit, so that
 // the slots of early CTAs go to later waves.
 __device__ __forceinline__ void passExitWait(uint32_t *exitCount)
@@ -40,18 +43,34 @@ __device__ __forceinline__ void passExitWait(uint32_t *exitCount)
 
 __global__ void grPassKernel(const DevNet *const *nets, const uint32_t *blockOffset, int numNets,
 		uint32_t stepOffset);
-// TMA GR pass with W consumer warps of RW rows each per stage, S stages
-// deep, at least B resident CTAs per SM, synapse-slot loops bounded by M
-// (0: any count), compiled for network shape `shape` (0: any network; see
-// passShapeOf); launched with 32 * (W + 1) threads, the grPassKernel
-// arguments and the descriptor of a single network (null for a batch).
-// Returns null for a geometry that is not compiled in.
-const void *passTmaKernelFor(int W, int RW, int S, int B, int M, int shape);
-// The most specific pass shape a network matches (0 when none).
-int passShapeOf(const DevNet &h);
+// Each CTA of a batch's per-tile pass: the network, and its tile or (events)
+// the block of cells whose events it takes.
+struct PassBlock {
+	const DevNet *net;
+	uint32_t tile, events;
+};
+// Per-tile GR pass (cbm_pass_event.cu) with W consumer warps and S stages;
+// launched with 32 * (W + 1) threads and (blocks, event CTAs, stepOffset,
+// descriptor of a single network or null, MF words, exit counter); oneZone:
+// every network has one zone.  Returns null for a geometry that is not
+// compiled in.
+const void *passTmaKernelFor(int W, int S, bool oneZone);
 // The compiled per-tile geometries, in table order.
 int passTmaConfigCount();
-void passTmaConfig(int i, int *W, int *RW, int *S, int *B, int *M);
+void passTmaConfig(int i, int *W, int *S, int *B);
+// GR arrays between the reference's order and the per-tile pass's.
+__global__ void evOrderKernel(const DevNet *N, const void *src, void *dst, uint32_t size, uint32_t rows, bool toTile);
+// Building a network's event tables (numMF + numGO sources): cells per
+// (block, source), their prefix sums per block, per-block bases, the lists, and
+// the cell-major GR->GO table; and the ring's arrivals after step T.
+__global__ void evCountKernel(const DevNet *N, uint32_t *cnt);
+__global__ void evScanKernel(uint32_t *cnt, uint32_t nSrc);
+__global__ void evBaseKernel(uint32_t *start, uint32_t *next, const uint32_t *base, uint32_t nSrc);
+__global__ void evFillKernel(const DevNet *N, uint32_t *next, uint16_t *entry);
+__global__ void evUnusedKernel(uint32_t *p, size_t n, uint32_t x);
+__global__ void evOutKernel(const DevNet *N, uint4 *outCell, uint4 *outMore, uint32_t *more);
+__global__ void goRingFillKernel(const DevNet *N, uint64_t T);
+__global__ void conductancesKernel(const DevNet *N, uint64_t T, float *outE, float *outI);
 // Persistent single-network TMA GR pass: W consumer warps (2W rows per
 // unit), S stages, B resident CTAs per SM, slot bound M; grid of any size,
 // 32 * (W + 1) threads, the grPassKernel arguments with one network.

@@ -113,7 +113,7 @@ __device__ __forceinline__ VecNet vecNet(const DevNet *N, uint64_t t)
 	c.gDecMF = N->gDecMFtoGR; c.gIncMF = N->gIncMFtoGR; c.gDecGO = N->gDecGOtoGR; c.gIncGO = N->gIncGOtoGR;
 	c.numGR = N->numGR; c.P = N->P; c.bs = N->bs; c.K = N->K;
 	c.bcShift = N->bcShift; c.scShift = N->scShift; c.jGroups = N->bs / 64u;
-	c.goCount = N->goCount + (size_t)(t & 1) * N->numGO;
+	c.goCount = N->goCount + (size_t)(t & (kGoRing - 1u)) * N->numGO;
 	c.vGR = N->vGR; c.gKCaGR = N->gKCaGR; c.threshGR = N->threshGR; c.gESum = N->gESum; c.gISum = N->gISum;
 	c.wGR = N->zones[0].w;
 	c.pairOut = N->zones[0].pairSum + (size_t)(t & 1) * N->numPC * N->K * N->bs;
@@ -537,8 +537,8 @@ const void *passVecBatchKernel() { return (const void *)&grPassVecBatchKernel; }
 
 bool passVecCapable(const DevNet &h)
 {
-	return passShapeOf(h) == 1 && h.numZones == 1 && h.bs >= 64 && h.bs % 64 == 0 && h.numGR % 128 == 0 &&
-		(1u << h.bcShift) >= 64u && (1u << h.scShift) >= 64u && !h.ovStart && h.outCon16 &&
+	return h.nMFSlots == 4 && h.nGOSlots == 3 && h.nOutSlots == 4 && h.numZones == 1 && h.bs >= 64 && h.bs % 64 == 0 && h.numGR % 128 == 0 &&
+		(1u << h.bcShift) >= 64u && (1u << h.scShift) >= 64u && h.outCon16 &&
 		h.P % (2 * h.bs) == 0;
 }
 

@@ -81,11 +81,35 @@ size_t Network::passSmemBytes() const
 		sizeof(float) * (size_t)h_.numZones * 2 * h_.K * h_.J;
 }
 
-size_t Network::passTmaSmemBytes(uint32_t R, uint32_t S, uint32_t outBytes) const
+bool Network::eventTiling(uint32_t target, uint32_t SC, DevNet *o) const
 {
-	const PassLayout L = passLayout(R, h_.nMFSlots, h_.nGOSlots, h_.nOutTma, h_.numZones, outBytes);
-	return 128 + (size_t)S * L.bytes + 16ull * S + sizeof(uint32_t) * (((size_t)h_.bcLocal + h_.scLocal + 3) & ~(size_t)3) +
-		sizeof(float) * (size_t)h_.numZones * 2 * h_.K * 32 + 32ull * (h_.mfWords + h_.goWords);
+	// Sources are numbered in 16 bits, arriving spikes counted in 4 a cell and kind.
+	if (h_.J != 32 || h_.numMF + h_.numGO > 65535u || h_.nMFSlots > 15u || h_.nGOSlots > 15u) return false;
+	// One PC's rows of 32 cells are the narrowest tile; smaller ones widen up
+	// to 128 cells, then take several PCs (all powers of two).  A round of SC
+	// cells has an even number of rows, so no pair of the reduction straddles two.
+	const uint32_t rowsPC = 2u * h_.K;
+	uint32_t wd = 32, pcs = 1;
+	while (wd < 128 && wd < h_.bs && 4u * wd <= SC && 2u * rowsPC * wd <= target) wd *= 2;
+	while (h_.numPC % (2u * pcs) == 0 && 2u * rowsPC * wd * pcs <= target) pcs *= 2;
+	const uint32_t TC = rowsPC * wd * pcs;
+	if (TC < SC || TC > kEvMaxTile) return false;
+	o->evWdShift = (uint32_t)__builtin_ctz(wd);
+	o->evRows = rowsPC * pcs;
+	o->evTilesX = h_.bs / wd;
+	o->evTiles = h_.numGR / TC;
+	o->evPCs = pcs;
+	// BC and SC blocks of a tile's rows (aligned powers of two of cells)
+	o->evBC = std::max<uint32_t>(1, (o->evRows * h_.bs) >> h_.bcShift);
+	o->evSC = std::max<uint32_t>(1, (o->evRows * h_.bs) >> h_.scShift);
+	return true;
+}
+
+size_t Network::eventSmemBytes(const DevNet &h, uint32_t SC, uint32_t S)
+{
+	const uint32_t TC = h.evRows << h.evWdShift;
+	return std::max<size_t>(kEvRoleBytes, 128 + eventSmem(std::min(S, TC / SC), eventLayout(SC, h.numZones).bytes, TC,
+			h.numZones, h.evPCs, h.evBC + h.evSC).bytes);
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link
@@ -144,12 +168,9 @@ std::string Network::buildPassMaps(uint32_t R)
 	CKS(enc2(PM_GISUM, h_.gISum, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4));
 	CKS(enc2(PM_APBUF, h_.apBufGR, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4));
 	const uint32_t mfS = std::max(1u, h_.nMFSlots), goS = std::max(1u, h_.nGOSlots), outS = std::max(1u, h_.nOutSlots);
-	const uint32_t outT = std::max(1u, h_.nOutTma);
 	CKS(enc3(PM_MFIDX, h_.mfIdx, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, mfS, mfS));
 	CKS(enc3(PM_GOIDX, h_.goIdx, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, goS, goS));
-	CKS(enc3(PM_OUTCON, h_.outCon, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, outS, outT));
-	if (h_.outCon16)
-		CKS(enc3(PM_OUTCON16, h_.outCon16, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, outS, outT));
+	CKS(enc3(PM_OUTCON, h_.outCon, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, outS, outS));
 	CKS(enc2(PM_PFDELAY, h_.pfDelay, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1));
 	CKS(enc2(PM_HIST, h_.historyGR, CU_TENSOR_MAP_DATA_TYPE_UINT64, 8));
 	for (uint32_t z = 0; z < h_.numZones; z++) CKS(enc2(PM_W0 + z, h_.zones[z].w, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4));
@@ -157,6 +178,138 @@ std::string Network::buildPassMaps(uint32_t R)
 	if (!d) return "device allocation failed";
 	CK(cudaMemcpy(d, maps.data(), PM_COUNT * sizeof(CUtensorMap), cudaMemcpyHostToDevice), "uploading TMA descriptors");
 	h_.passMaps = d;
+	return uploadDesc();
+}
+
+std::string Network::buildEventPass(uint32_t target, uint32_t SC, cudaStream_t s)
+{
+	// a new tiling drops the spikes the last step left for the next: the ring
+	// is refilled from the spike buffers (setEventMode) whenever it is entered
+	CKS(setEventMode(false, s));
+	const uint32_t rows0 = h_.evRows, wd0 = h_.evWdShift;
+	if (!eventTiling(target, SC, &h_)) return "no tiling of the per-tile GR pass covers the cells";
+	if (!h_.evCnt) {
+		h_.evCnt = alloc<uint8_t>(2ull * h_.numGR);
+		if (!h_.evCnt) return "device allocation failed";
+	}
+	const uint32_t N = h_.numGR, nSrc = h_.numMF + h_.numGO;
+	if (h_.evStart && h_.evRows == rows0 && h_.evWdShift == wd0) return uploadDesc();
+
+	// event tables in the tiling's order, built on the device from the slot tables
+	for (void *q : {(void *)h_.evStart, (void *)h_.evEntry, (void *)h_.outCell, (void *)h_.outMore, (void *)h_.evPfDelay,
+			(void *)h_.spkBits})
+		if (q) release(q);
+	h_.evStart = nullptr; h_.evEntry = nullptr; h_.outCell = h_.outMore = nullptr; h_.evPfDelay = nullptr; h_.spkBits = nullptr;
+	const uint32_t blocks = eventBlocks(), grid = (N + 255) / 256;
+	const size_t nStart = (size_t)blocks * (nSrc + 1);
+	h_.spkBits = alloc<uint32_t>(2ull * (N / 32));
+	uint32_t *start = alloc<uint32_t>(nStart), *next = alloc<uint32_t>(nStart), *base = alloc<uint32_t>(blocks);
+	if (!h_.spkBits || !start || !next || !base) return "device allocation failed";
+	CKS(uploadDesc());
+	evCountKernel<<<grid, 256, 0, s>>>(devPtr(), start);
+	evScanKernel<<<blocks, 256, 0, s>>>(start, nSrc);
+	std::vector<uint32_t> hb(blocks);
+	CK(cudaMemcpy2DAsync(hb.data(), 4, start + nSrc, 4ull * (nSrc + 1), 4, blocks, cudaMemcpyDeviceToHost, s), "event tables");
+	CK(cudaStreamSynchronize(s), "event tables");
+	uint64_t total = 0;
+	for (uint32_t &x : hb) { const uint32_t n = x; x = (uint32_t)total; total += n; }
+	if (total > 0x1FFFFFFFull) return "too many GR synapses for the event tables";
+	uint16_t *entry = alloc<uint16_t>(8 * total);
+	if (!entry) return "device allocation failed";
+	evUnusedKernel<<<1184, 256, 0, s>>>((uint32_t *)entry, 4 * total, kEvUnused | (kEvUnused << 16));
+	CK(cudaMemcpyAsync(base, hb.data(), 4ull * blocks, cudaMemcpyHostToDevice, s), "event tables");
+	evBaseKernel<<<blocks, 256, 0, s>>>(start, next, base, nSrc);
+	evFillKernel<<<grid, 256, 0, s>>>(devPtr(), next, entry);
+	// items of 64 cells for a usual list (its mean and two deviations)
+	auto items = [&](uint32_t slots, uint32_t sources) {
+		const double mean = (double)std::min(N, kEvCells) * slots / sources;
+		return std::min(16u, std::max(1u, (uint32_t)std::ceil((mean + 2 * std::sqrt(mean)) / 64)));
+	};
+	h_.evPerMF = items(h_.nMFSlots, h_.numMF);
+	h_.evPerGO = items(h_.nGOSlots, h_.numGO);
+	uint4 *oc = alloc<uint4>(N);
+	uint8_t *pd = alloc<uint8_t>(N);
+	uint32_t *rows = alloc<uint32_t>(2), nRows = 0;  // zeroed
+	if (!oc || !pd || !rows) return "device allocation failed";
+	evOutKernel<<<grid, 256, 0, s>>>(devPtr(), nullptr, nullptr, rows);
+	CK(cudaMemcpyAsync(&nRows, rows, 4, cudaMemcpyDeviceToHost, s), "event tables");
+	CK(cudaStreamSynchronize(s), "event tables");
+	if (nRows > 0xFFFFFFu) return "too many GR->GO synapses for the event tables";
+	uint4 *om = alloc<uint4>(std::max(1u, nRows));
+	if (!om) return "device allocation failed";
+	evOutKernel<<<grid, 256, 0, s>>>(devPtr(), oc, om, rows + 1);
+	evOrderKernel<<<grid, 256, 0, s>>>(devPtr(), h_.pfDelay, pd, 1, 1, true);
+	h_.outCell = oc;
+	h_.outMore = om;
+	h_.evPfDelay = pd;
+	CK(cudaGetLastError(), "event tables");
+	CK(cudaStreamSynchronize(s), "event tables");
+	release(next);
+	release(base);
+	release(rows);
+	h_.evStart = start;
+	h_.evEntry = (const uint4 *)entry;
+	return uploadDesc();
+}
+
+// Device scratch of 8 bytes a GR, kept for the network's life (reordering and
+// exports, one at a time in the stream's order).
+std::string Network::scratch(void **p)
+{
+	if (!scratch_) scratch_ = alloc<uint64_t>(h_.numGR);
+	if (!scratch_) return "device allocation failed";
+	*p = scratch_;
+	return "";
+}
+
+// An array of `rows` x numGR elements into the per-tile pass's order (toTile) or
+// back, in place.
+std::string Network::reorder(void *a, uint32_t size, uint32_t rows, bool toTile, cudaStream_t s)
+{
+	if (h_.evTilesX == 1) return "";  // tiles of whole rows: the orders agree
+	void *tmp = nullptr;
+	CKS(scratch(&tmp));
+	const uint32_t most = 8u / size;  // rows the scratch holds
+	for (uint32_t r = 0; r < rows; r += most) {
+		const uint32_t k = std::min(most, rows - r);
+		const uint64_t n = (uint64_t)h_.numGR * k;
+		uint8_t *const q = (uint8_t *)a + (uint64_t)h_.numGR * r * size;
+		CK(cudaMemcpyAsync(tmp, q, n * size, cudaMemcpyDeviceToDevice, s), "reordering GR arrays");
+		evOrderKernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(devPtr(), tmp, q, size, k, toTile);
+		CK(cudaGetLastError(), "reordering GR arrays");
+	}
+	return "";
+}
+
+std::string Network::setEventMode(bool on, cudaStream_t s)
+{
+	if (evMode_ == on) return "";
+	CK(cudaStreamSynchronize(s), "pass switch");
+	const unsigned grid = (h_.numGR + 255) / 256;
+	if (on) {
+		// every arrival still to come, the last step's spikes included; the
+		// conductances are final
+		CK(cudaMemsetAsync(h_.spkBits, 0, 8ull * (h_.numGR / 32), s), "pass switch");
+		CK(cudaMemsetAsync(h_.evCnt, 0, 2ull * h_.numGR, s), "pass switch");
+		goRingFillKernel<<<grid, 256, 0, s>>>(devPtr(), hostT_);
+		h_.evFirst = hostT_ + 1;
+	} else {
+		// slot T is complete and still to be read by the next small-cell
+		// update; what the last step's pass left to deliver is not delivered
+		for (uint64_t k = 1; k < kGoRing; k++)
+			CK(cudaMemsetAsync(h_.goCount + (size_t)((hostT_ + k) & (kGoRing - 1)) * h_.numGO, 0, 4ull * h_.numGO, s),
+					"pass switch");
+		if (conductancesPending()) conductancesKernel<<<grid, 256, 0, s>>>(devPtr(), hostT_, h_.gESum, h_.gISum);
+	}
+	CK(cudaGetLastError(), "pass switch");
+	for (void *a : {(void *)h_.vGR, (void *)h_.gKCaGR, (void *)h_.threshGR, (void *)h_.gESum, (void *)h_.gISum,
+			(void *)h_.apBufGR})
+		CKS(reorder(a, 4, 1, on, s));
+	for (uint32_t z = 0; z < h_.numZones; z++) CKS(reorder(h_.zones[z].w, 4, 1, on, s));
+	CKS(reorder(h_.historyGR, 8, 1, on, s));
+	if (hProto_.grPSH) CKS(reorder(hProto_.grPSH, 2, hProto_.nBins, on, s));
+	CK(cudaStreamSynchronize(s), "pass switch");
+	evMode_ = on;
 	return uploadDesc();
 }
 
@@ -320,12 +473,12 @@ double Network::bytesPerStepAlgorithmic() const
 
 double Network::bytesPerStepLayout() const
 {
-	// GR state read and written (6 x 4 B each way), synapse slots (u16 MF and
-	// GO indices, u32 GR->GO targets), the PF delay byte, the PF->PC weight
-	// of every zone; history read + write and weight writes on plasticity steps
-	const double perGR = 48.0 + 2.0 * h_.nMFSlots + 2.0 * h_.nGOSlots + (double)outBytes_ * outPlanes_ +
-		12.0 * ovUsed_ / h_.numGR + 1.0 + 4.0 * h_.numZones +
-		(16.0 + 4.0 * h_.numZones) / h_.tsPerHistBinGR;
+	// GR state read and written (6 x 4 B each way), the PF delay byte, the
+	// PF->PC weight of every zone; history read + write and weight writes on
+	// plasticity steps; the synapse tables (u16 MF and GO indices, u32 GR->GO
+	// slots) where the pass streams them, else the counts of arrived spikes
+	const double slots = streamsSlots_ ? 2.0 * h_.nMFSlots + 2.0 * h_.nGOSlots + 4.0 * h_.nOutSlots : 2.0;
+	const double perGR = 48.0 + slots + 1.0 + 4.0 * h_.numZones + (16.0 + 4.0 * h_.numZones) / h_.tsPerHistBinGR;
 	return perGR * h_.numGR;
 }
 
@@ -500,12 +653,14 @@ std::string Network::build(State *st, const std::vector<int> &seeds, uint32_t mf
 	std::vector<uint16_t> goIdx((size_t)std::max(1u, nGO) * N, (uint16_t)c.numGO);
 	std::vector<uint32_t> outCon((size_t)std::max(1u, nOut) * N, kNoDelay);
 	std::vector<uint8_t> pfDelay(N);
+	h.outNow = 0;
 	for (uint32_t g = 0; g < N; g++) {
 		for (int k = 0; k < numMFin[g]; k++) mfIdx[(size_t)k * N + g] = (uint16_t)pMF[(size_t)g * strideGO + k];
 		for (int k = 0; k < numGOin[g]; k++) goIdx[(size_t)k * N + g] = (uint16_t)pGO[(size_t)g * strideGO + k];
 		uint32_t bit = 0;
 		for (int k = 0; k < numOut[g]; k++) {
 			singleBitOrZero(pOutMask[(size_t)g * strideOut + k], bit);
+			if (bit == 0) h.outNow = 1;
 			outCon[(size_t)k * N + g] = (pOut[(size_t)g * strideOut + k] << 8) | bit;
 		}
 		singleBitOrZero(pfMask[g], bit);
@@ -514,39 +669,9 @@ std::string Network::build(State *st, const std::vector<int> &seeds, uint32_t mf
 	h.mfIdx = upload(mfIdx.data(), mfIdx.size());
 	h.goIdx = upload(goIdx.data(), goIdx.size());
 	h.outCon = upload(outCon.data(), outCon.size());
-	// Networks with more than 4 GR->GO synapses on some GR (a fan-out padded
-	// to its maximum): the per-tile TMA pass streams the first 4 slot planes
-	// and takes the rest from per-tile lists after its rows
-	h.nOutTma = nOut;
-	h.ovStart = nullptr;
-	h.ovEntry = nullptr;
-	if (nOut > kOutInline && h.J == 32) {
-		const uint32_t tiles = c.numPC * h.tilesPerPC;
-		std::vector<std::vector<uint2>> per(tiles);
-		for (uint32_t g = 0; g < N; g++)
-			for (int k = (int)kOutInline; k < numOut[g]; k++) {
-				const uint32_t cv = outCon[(size_t)k * N + g];
-				if ((cv & 0xFFu) >= 32u) continue;  // a synapse without a delay bit never fires
-				const uint32_t off = g % P, r = off / h.bs, jf = off % h.bs;
-				const uint32_t tile = (g / P) * h.tilesPerPC + jf / 32;
-				per[tile].push_back(make_uint2((r * 32 + jf % 32) | ((cv & 0xFFu) << 24), cv >> 8));
-			}
-		std::vector<uint32_t> start(tiles + 1, 0);
-		std::vector<uint2> ent;
-		for (uint32_t b = 0; b < tiles; b++) {
-			start[b] = (uint32_t)ent.size();
-			ent.insert(ent.end(), per[b].begin(), per[b].end());
-		}
-		start[tiles] = (uint32_t)ent.size();
-		if (ent.empty()) ent.push_back(make_uint2(0, 0));  // never read: every range is empty
-		h.nOutTma = kOutInline;
-		h.ovStart = upload(start.data(), start.size());
-		h.ovEntry = upload(ent.data(), ent.size());
-		ovEntries_ = start[tiles];
-	}
 	h.outCon16 = nullptr;
 	if (c.numGO <= kOut16MaxGO) {
-		// the 16-bit copy the shape-specialised GR pass streams
+		// the 16-bit copy the vector pass reads
 		std::vector<uint16_t> out16(outCon.size(), kOut16None);
 		for (size_t i = 0; i < outCon.size(); i++)
 			if ((outCon[i] & 0xFFu) < 32u) out16[i] = (uint16_t)(((outCon[i] >> 8) << 5) | (outCon[i] & 0x1Fu));
@@ -699,7 +824,7 @@ std::string Network::build(State *st, const std::vector<int> &seeds, uint32_t mf
 	h.pairStep = alloc<uint64_t>(2);
 	h.passClaim = alloc<uint32_t>(4);
 	h.pcDone = alloc<uint32_t>(c.numPC);
-	h.goCount = alloc<uint32_t>((size_t)2 * c.numGO);
+	h.goCount = alloc<uint32_t>((size_t)kGoRing * c.numGO);
 	h.bcCount = alloc<uint32_t>((size_t)3 * c.numBC);
 	h.scCount = alloc<uint32_t>((size_t)3 * c.numSC);
 	h.goBits = alloc<uint32_t>((size_t)2 * h.goWords);
@@ -983,6 +1108,21 @@ std::string Network::readRecord(int kind, void *dst, size_t bytes, cudaStream_t 
 		: !trialDataRecord(kind, &off, &n) ? nullptr
 		: kind <= CBM_REC_PSH_IO ? (const void *)(hProto_.tdPSH + off) : (const void *)(hProto_.tdRaster + off);
 	if (!src) return "unknown record kind";
+	if (kind == CBM_REC_GR_PSH && evMode_ && h_.evTilesX > 1) {
+		// recorded in the pass's order
+		void *tmp = nullptr;
+		CKS(scratch(&tmp));
+		const size_t row = 2ull * h_.numGR, rows = bytes / row;
+		for (size_t r = 0; r < rows; r += 4) {
+			const size_t n = std::min<size_t>(4, rows - r);
+			evOrderKernel<<<(unsigned)((n * h_.numGR + 255) / 256), 256, 0, s>>>(devPtr(), (const uint8_t *)src + r * row, tmp,
+					2, (uint32_t)n, false);
+			CK(cudaGetLastError(), "reading a record");
+			CK(cudaMemcpyAsync((uint8_t *)dst + r * row, tmp, n * row, cudaMemcpyDeviceToHost, s), "reading a record");
+		}
+		CK(cudaStreamSynchronize(s), "reading a record");
+		return "";
+	}
 	CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s), "reading a record");
 	CK(cudaStreamSynchronize(s), "reading a record");
 	return "";
@@ -1033,15 +1173,22 @@ std::string Network::exportField(Field f, uint32_t zone, void *dst, size_t bytes
 	switch (f) {
 	case F_AP_GR: {
 		uint8_t *tmp = nullptr;
-		CK(cudaMallocAsync((void **)&tmp, h.numGR, s), "export scratch");
+		CKS(scratch((void **)&tmp));
 		extractSpikesKernel<<<(h.numGR + 255) / 256, 256, 0, s>>>(h.apBufGR, tmp, h.numGR);
-		CK(cudaMemcpyAsync(dst, tmp, h.numGR, cudaMemcpyDeviceToHost, s), "export");
-		CK(cudaFreeAsync(tmp, s), "export scratch");
+		CKS(exportGR(tmp, 1, tmp + h.numGR, dst, s));
 		return "";
 	}
 	case F_VM_GR: src = h.vGR; break;
-	case F_GESUM_GR: src = h.gESum; break;
-	case F_GISUM_GR: src = h.gISum; break;
+	case F_GESUM_GR: case F_GISUM_GR: {
+		src = f == F_GESUM_GR ? h.gESum : h.gISum;
+		if (!conductancesPending()) break;
+		float *tmp = nullptr;
+		CKS(scratch((void **)&tmp));
+		conductancesKernel<<<(h.numGR + 255) / 256, 256, 0, s>>>(devPtr(), hostT_, f == F_GESUM_GR ? tmp : nullptr,
+				f == F_GISUM_GR ? tmp : nullptr);
+		CKS(exportGR(tmp, 4, tmp + h.numGR, dst, s));
+		return "";
+	}
 	case F_APBUF_GR: src = h.apBufGR; break;
 	case F_HIST_GR: src = h.historyGR; break;
 	case F_THRESH_GR: src = h.threshGR; break;
@@ -1073,7 +1220,27 @@ std::string Network::exportField(Field f, uint32_t zone, void *dst, size_t bytes
 	case F_MFNC_WEIGHT: src = Q.mfSynWeightNC; break;
 	default: return "unknown field";
 	}
+	if (f <= F_GKCA_GR || f == F_PFPC_WEIGHT) {
+		// a GR array: in the reference's order
+		void *tmp = nullptr;
+		if (evMode_ && h.evTilesX > 1) CKS(scratch(&tmp));
+		CKS(exportGR(src, (uint32_t)(bytes / h.numGR), tmp, dst, s));
+		return "";
+	}
 	CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s), "export");
+	return "";
+}
+
+// A GR array (numGR elements of `size` bytes, as the pass in use holds it) to
+// host memory in the reference's order; tmp: device scratch of its size.
+std::string Network::exportGR(const void *src, uint32_t size, void *tmp, void *dst, cudaStream_t s)
+{
+	if (evMode_ && h_.evTilesX > 1) {
+		evOrderKernel<<<(h_.numGR + 255) / 256, 256, 0, s>>>(devPtr(), src, tmp, size, 1, false);
+		CK(cudaGetLastError(), "export");
+		src = tmp;
+	}
+	CK(cudaMemcpyAsync(dst, src, (size_t)size * h_.numGR, cudaMemcpyDeviceToHost, s), "export");
 	return "";
 }
 
@@ -1096,15 +1263,19 @@ std::string Network::writeToState(cudaStream_t s)
 	};
 	// InNet::writeToState (innet.cpp:608-667)
 	{
-		std::vector<uint32_t> ab(h.numGR);
-		CK(cudaMemcpy(ab.data(), h.apBufGR, 4ull * h.numGR, cudaMemcpyDeviceToHost), "apBufGR");
+		const struct { const char *name; Field f; } gr[] = {{"apBufGR", F_APBUF_GR}, {"gMFSumGR", F_GESUM_GR},
+			{"gGOSumGR", F_GISUM_GR}, {"threshGR", F_THRESH_GR}, {"vGR", F_VM_GR}, {"gKCaGR", F_GKCA_GR},
+			{"historyGR", F_HIST_GR}};
+		for (const auto &a : gr) {
+			NamedArray *x = st_->find(a.name, -1);
+			CKS(exportField(a.f, 0, x->bytes.data(), x->bytes.size(), s));
+		}
+		CK(cudaStreamSynchronize(s), "GR state");
+		const uint32_t *ab = st_->find("apBufGR")->as<uint32_t>();
 		uint8_t *apGR = st_->find("apGR")->as<uint8_t>();
 		// outputGRGPU holds zeros until the first step (innet.cpp:477)
 		for (uint32_t i = 0; i < h.numGR; i++) apGR[i] = hostT_ ? (uint8_t)(ab[i] & 1u) : 0;
-		memcpy(st_->find("apBufGR")->bytes.data(), ab.data(), 4ull * h.numGR);
 	}
-	CKS(D("gMFSumGR", -1, h.gESum)); CKS(D("gGOSumGR", -1, h.gISum)); CKS(D("threshGR", -1, h.threshGR));
-	CKS(D("vGR", -1, h.vGR)); CKS(D("gKCaGR", -1, h.gKCaGR)); CKS(D("historyGR", -1, h.historyGR));
 	{
 		const uint32_t buf = (uint32_t)((hostT_ + 2) % 3);
 		CKS(D("inputSumPFSC", -1, h.scCount + (size_t)buf * h.numSC));
@@ -1124,7 +1295,11 @@ std::string Network::writeToState(cudaStream_t s)
 		const DevZone &Q = h.zones[z];
 		int zi = (int)z;
 		// MZone::writeToState (mzone.cpp:139-147)
-		CKS(D("pfSynWeightPC", zi, Q.w));
+		{
+			NamedArray *x = st_->find("pfSynWeightPC", zi);
+			CKS(exportField(F_PFPC_WEIGHT, z, x->bytes.data(), x->bytes.size(), s));
+			CK(cudaStreamSynchronize(s), "pfSynWeightPC");
+		}
 		{
 			const uint32_t buf = (uint32_t)((hostT_ + 2) % 3);
 			std::vector<float> part((size_t)h.numPC * h.bs);
@@ -1180,7 +1355,7 @@ Simulator::~Simulator()
 	for (cudaEvent_t e : stepEv_) if (e) cudaEventDestroy(e);
 	for (Network *n : nets_) delete n;
 	for (DeviceBuf *b : {&dNetPtrs_, &dBlockOffset_, &dTBasePtrs_, &dStageBytes_, &dCellOffset_, &dVecUnitOffset_,
-			&dVecPcOffset_, &dVecClaim_, &dExitCount_})
+			&dVecPcOffset_, &dVecClaim_, &dExitCount_, &dPassBlocks_})
 		if (b->ptr) cudaFree(b->ptr);
 	if (s0_) cudaStreamDestroy(s0_);
 	if (s1_) cudaStreamDestroy(s1_);
@@ -1265,17 +1440,43 @@ std::string Simulator::create(const std::vector<State *> &states, const std::vec
 	return usePassGeometry(cands.front());
 }
 
+// Cells a tile of the per-tile pass should hold, a multiple of rounds of SC:
+// 2048 (64 rows of 32 cells of the 1M-GR network: one wave of four CTAs an SM),
+// down to 512 where that leaves fewer than two tiles an SM (a single small
+// network).
+static uint32_t tileTarget(const std::vector<Network *> &nets, uint32_t SC)
+{
+	uint64_t total = 0;
+	for (Network *n : nets) total += n->dev().numGR;
+	uint32_t target = 2048;
+	while (target > 512 && target > SC && total / target < 296) target /= 2;
+	return std::max(target, SC);
+}
+
+// Stages of the per-tile pass in a geometry: its rows per warp times its
+// stages, in the compiled range.
+static uint32_t stagesOf(const PassGeometry &g) { return (uint32_t)std::min(4, g.RW * g.S); }
+
+// Whether every network has a tiling for the geometry and its CTA's shared
+// memory fits; *smem receives that.
+bool Simulator::passTmaFits(const PassGeometry &g, size_t *smem) const
+{
+	const uint32_t SC = 128u * g.W, target = tileTarget(nets_, SC);
+	*smem = 0;
+	for (Network *n : nets_) {
+		DevNet h = n->dev();
+		if (!n->eventTiling(target, SC, &h)) return false;
+		*smem = std::max(*smem, Network::eventSmemBytes(h, SC, stagesOf(g)));
+	}
+	return !nets_.empty() && *smem <= 227 * 1024;
+}
+
 std::vector<PassGeometry> Simulator::passCandidates() const
 {
-	// the default first: 4 consumer warps of 1 row, 4 stages, 4 CTAs/SM,
-	// slot loops for at most 4 slots (8,1,3,2 with open slot loops past 4)
 	std::vector<PassGeometry> out;
 	// the vector pass where it applies (networks of the compiled shape),
-	// after the per-tile default: on the 1M eyelid network it measured
-	// 31 us flushed against 24 us for the per-tile pass, its units being two
-	// dependent round trips each where the per-tile pass keeps four stages
-	// of loads in flight.  CBM_PASS_VEC=0 leaves it out, CBM_PASS_VEC=1 puts
-	// it first.
+	// after the per-tile default.  CBM_PASS_VEC=0 leaves it out,
+	// CBM_PASS_VEC=1 puts it first.
 	const char *vecEnv = getenv("CBM_PASS_VEC");
 	bool vec = !nets_.empty() && !(vecEnv && !strcmp(vecEnv, "0"));
 	for (Network *n : nets_) vec = vec && passVecCapable(n->dev());
@@ -1283,50 +1484,21 @@ std::vector<PassGeometry> Simulator::passCandidates() const
 	v.kind = 3;
 	const bool vecFirst = vec && vecEnv && !strcmp(vecEnv, "1");
 	if (vecFirst) out.push_back(v);
-	bool tma = !nets_.empty();
-	uint32_t minRows = UINT32_MAX, maxSlots = 0;
-	for (Network *n : nets_) {
-		tma = tma && n->passTmaCapable();
-		minRows = std::min(minRows, n->passRows());
-		maxSlots = std::max({maxSlots, n->dev().nMFSlots, n->dev().nGOSlots, n->dev().nOutTma});
-	}
-	if (tma) {
-		PassGeometry d;
-		d.kind = 1;
-		if (maxSlots <= 4) { d.W = 4; d.RW = 1; d.S = 4; d.B = 4; d.M = 4; }
-		else { d.W = 8; d.RW = 1; d.S = 3; d.B = 2; d.M = 0; }
-		// Networks whose per-step working set stays in L2 (GR state read and
-		// written, synapse slots, delays, weights: about 75 B a GR) are bound
-		// by issue and latency: two rows per consumer warp.  On the 1M-GR
-		// network 4,2,2,4 ran 9.6 % faster back to back than 4,1,4,4 (1.9 %
-		// slower after an L2 flush); where the state streams from HBM (the
-		// dense 4M network) single rows and a deeper ring are faster.
-		int l2 = 0;
-		cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device_);
-		double set = 0;
-		for (Network *n : nets_) {
-			const DevNet &h = n->dev();
-			set += (48.0 + 2.0 * (h.nMFSlots + h.nGOSlots + h.nOutTma) + 1.0 + 4.0 * h.numZones) * h.numGR;
-		}
-		if (maxSlots <= 4 && set <= 0.75 * l2 && 8u <= minRows) {
-			PassGeometry r = d;
-			r.RW = 2;
-			r.S = 2;
-			out.push_back(r);
-		}
-		if ((uint32_t)(d.W * d.RW) <= minRows) out.push_back(d);
-		if (vec && !vecFirst) out.push_back(v);
-		for (int i = 0; i < passTmaConfigCount(); i++) {
-			PassGeometry c;
-			c.kind = 1;
-			passTmaConfig(i, &c.W, &c.RW, &c.S, &c.B, &c.M);
-			if ((uint32_t)(c.W * c.RW) > minRows || (c.M > 0 && maxSlots > (uint32_t)c.M)) continue;
-			bool listed = false;
-			for (const PassGeometry &o : out)
-				listed = listed || (o.kind == 1 && c.W == o.W && c.RW == o.RW && c.S == o.S && c.B == o.B && c.M == o.M);
-			if (listed) continue;
-			out.push_back(c);
-		}
+	uint32_t maxSlots = 0;
+	for (Network *n : nets_)
+		maxSlots = std::max({maxSlots, n->dev().nMFSlots, n->dev().nGOSlots, n->dev().nOutSlots});
+	// the first compiled per-tile geometry that fits is the default
+	bool tma = false;
+	for (int i = 0; i < passTmaConfigCount(); i++) {
+		PassGeometry c;
+		c.kind = 1;
+		passTmaConfig(i, &c.W, &c.S, &c.B);
+		c.M = maxSlots <= 4 ? 4 : 0;
+		size_t smem = 0;
+		if (!passTmaFits(c, &smem)) continue;
+		out.push_back(c);
+		if (!tma && vec && !vecFirst) out.push_back(v);
+		tma = true;
 	}
 	if (vec && !vecFirst && !tma) out.push_back(v);
 	PassGeometry plain;
@@ -1340,18 +1512,23 @@ std::string Simulator::usePassGeometry(const PassGeometry &g)
 	CK(cudaSetDevice(device_), "selecting the device");
 	uint32_t minRows = UINT32_MAX, maxSlots = 0;
 	bool capable = !nets_.empty();
-	uint32_t maxSlotsTile = 0;  // the per-tile pass streams nOutTma GR->GO planes
 	for (Network *n : nets_) {
 		capable = capable && n->passTmaCapable();
 		minRows = std::min(minRows, n->passRows());
 		maxSlots = std::max({maxSlots, n->dev().nMFSlots, n->dev().nGOSlots, n->dev().nOutSlots});
-		maxSlotsTile = std::max({maxSlotsTile, n->dev().nMFSlots, n->dev().nGOSlots, n->dev().nOutTma});
 	}
-	for (Network *n : nets_) { n->outBytes_ = 4; n->outPlanes_ = n->dev().nOutSlots; n->ovUsed_ = 0; }
 	// leaving the vector pass: the last step's PF->PC reduction is still pair
 	// sums, and the small-cell update goes back to partial sums
 	if (passVec_ && g.kind != 3)
 		for (Network *n : nets_) CKS(n->setPcSumMode(false, s0_));
+	// everything but the per-tile pass counts GR->GO spikes when they arrive
+	auto arriveMode = [&]() -> std::string {
+		for (Network *n : nets_) {
+			CKS(n->setEventMode(false, s0_));
+			n->streamsSlots_ = true;
+		}
+		return "";
+	};
 	if (g.kind == 3 && nets_.size() > 1) {
 		for (Network *n : nets_)
 			if (!passVecCapable(n->dev())) return "the vector GR pass runs networks of its compiled shape";
@@ -1382,10 +1559,12 @@ std::string Simulator::usePassGeometry(const PassGeometry &g)
 				(uint32_t)std::max(1, perSM) * (uint32_t)numSMs));
 		CK(cudaMemset(dVecClaim_.ptr, 0, dVecClaim_.bytes), "pass claim counters");
 		for (Network *n : nets_) CKS(n->setPcSumMode(true, s0_));
+		CKS(arriveMode());
 		passTmaFn_ = fn;
 		passVec_ = true;
 		passPersistent_ = false;
 		passTmaW_ = kVecWarps - 1;
+		passTmaThreads_ = 32u * kVecWarps;
 		passTmaR_ = passTmaS_ = 0;
 		passTmaSmem_ = 0;
 		passGeom_ = g;
@@ -1418,10 +1597,12 @@ std::string Simulator::usePassGeometry(const PassGeometry &g)
 		// claim counters from zero (another pass kind may have run meanwhile)
 		CK(cudaMemset(n.dev().passClaim, 0, 4 * sizeof(uint32_t)), "pass claim counters");
 		CKS(n.setPcSumMode(true, s0_));
+		CKS(arriveMode());
 		passTmaFn_ = fn;
 		passVec_ = true;
 		passPersistent_ = false;
-		passTmaW_ = kVecWarps - 1;  // launchPass's block is 32 * (W + 1) threads
+		passTmaW_ = kVecWarps - 1;
+		passTmaThreads_ = 32u * kVecWarps;
 		passTmaR_ = passTmaS_ = 0;
 		passTmaSmem_ = smem;
 		passGeom_ = g;
@@ -1430,6 +1611,7 @@ std::string Simulator::usePassGeometry(const PassGeometry &g)
 	}
 	passVec_ = false;
 	if (g.kind == 0) {
+		CKS(arriveMode());
 		passTmaFn_ = nullptr;
 		passPersistent_ = false;
 		passTmaW_ = passTmaR_ = passTmaS_ = 0;
@@ -1438,32 +1620,47 @@ std::string Simulator::usePassGeometry(const PassGeometry &g)
 		return "";
 	}
 	if (!capable) return "the TMA GR pass needs tiles of 32-cell rows in every network";
-	if (g.M > 0 && (g.kind == 1 ? maxSlotsTile : maxSlots) > (uint32_t)g.M)
+	// (the per-tile pass has no slot loops: M is accepted and has no effect)
+	if (g.kind != 1 && g.M > 0 && maxSlots > (uint32_t)g.M)
 		return "a network has more synapse slots than the geometry's slot bound";
 	const void *fn = nullptr;
 	uint32_t R = 0, threads = 0, grid = passBlocks_;
 	size_t smem = 0;
 	if (g.kind == 1) {
-		// the shape-specialised instance when every network has that shape
-		// (CBM_PASS_SHAPE=0 keeps the run-time-shape kernel: testing)
-		int shape = g.M == 4 ? 1 : 0;
-		for (Network *n : nets_) if (passShapeOf(n->dev()) != 1) shape = 0;
-		if (const char *env = getenv("CBM_PASS_SHAPE"))
-			if (!strcmp(env, "0")) shape = 0;
-		fn = passTmaKernelFor(g.W, g.RW, g.S, g.B, g.M, shape);
+		bool oneZone = true;
+		for (Network *n : nets_) oneZone = oneZone && n->dev().numZones == 1;
+		fn = g.RW > 0 && g.S > 0 ? passTmaKernelFor(g.W, (int)stagesOf(g), oneZone) : nullptr;
 		if (!fn) return "per-tile GR-pass geometry not compiled in";
-		R = (uint32_t)(g.W * g.RW);
-		if (R > minRows) return "more rows per stage than a tile has";
-		for (Network *n : nets_) smem = std::max(smem, n->passTmaSmemBytes(R, (uint32_t)g.S, shape == 1 ? 2u : 4u));
-		for (Network *n : nets_) {
-			n->outBytes_ = shape == 1 ? 2u : 4u;
-			n->outPlanes_ = n->dev().nOutTma;
-			n->ovUsed_ = n->ovEntries_;
-		}
+		if (!passTmaFits(g, &smem)) return "the per-tile GR-pass geometry does not fit every network";
+		const uint32_t SC = 128u * g.W, target = tileTarget(nets_, SC);
+		R = SC / 32u;
 		threads = 32u * (g.W + 1);
+		std::vector<PassBlock> blocks;
+		for (Network *n : nets_) {
+			CKS(n->buildEventPass(target, SC, s0_));
+			CKS(n->setEventMode(true, s0_));
+			n->streamsSlots_ = false;
+		}
+		// the event CTAs first: theirs is the longer chain of latencies
+		passEvents_ = nets_.size() > 1 ? 0u : nets_[0]->eventBlocks();
+		grid = passEvents_ + nets_[0]->dev().evTiles;
+		if (nets_.size() > 1) {
+			for (Network *n : nets_)
+				for (uint32_t b = 0; b < n->eventBlocks(); b++) blocks.push_back({n->devPtr(), b, 1});
+			for (Network *n : nets_)
+				for (uint32_t b = 0; b < n->dev().evTiles; b++) blocks.push_back({n->devPtr(), b, 0});
+			grid = (uint32_t)blocks.size();
+		}
+		if (dPassBlocks_.ptr) cudaFree(dPassBlocks_.ptr);
+		dPassBlocks_ = DeviceBuf();
+		if (!blocks.empty()) {
+			CK(cudaMalloc(&dPassBlocks_.ptr, blocks.size() * sizeof(PassBlock)), "allocating launch tables");
+			dPassBlocks_.bytes = blocks.size() * sizeof(PassBlock);
+			CK(cudaMemcpy(dPassBlocks_.ptr, blocks.data(), dPassBlocks_.bytes, cudaMemcpyHostToDevice), "uploading launch tables");
+		}
 	} else {
 		if (nets_.size() != 1) return "the persistent GR pass runs one network";
-		if (nets_[0]->dev().ovStart) return "the persistent GR pass streams every GR->GO slot; this network has per-tile lists";
+		if (nets_[0]->dev().nOutSlots > kOutInline) return "the persistent GR pass streams at most 4 GR->GO slots";
 		fn = passPersistentKernelFor(g.W, g.S, g.B, g.M);
 		if (!fn) return "persistent GR-pass geometry not compiled in";
 		R = (uint32_t)(2 * g.W);
@@ -1475,7 +1672,10 @@ std::string Simulator::usePassGeometry(const PassGeometry &g)
 		threads = 32u * (g.W + 1);
 	}
 	if (smem > 227 * 1024) return "GR-pass geometry needs more shared memory than a CTA has";
-	for (Network *n : nets_) CKS(n->buildPassMaps(R));
+	if (g.kind == 2) {
+		CKS(nets_[0]->buildPassMaps(R));
+		CKS(arriveMode());
+	}
 	CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "pass smem");
 	if (g.kind == 2) {
 		int perSM = 0, numSMs = 0;
@@ -1488,6 +1688,7 @@ std::string Simulator::usePassGeometry(const PassGeometry &g)
 	passTmaFn_ = fn;
 	passPersistent_ = g.kind == 2;
 	passTmaW_ = (uint32_t)g.W;
+	passTmaThreads_ = threads;
 	passTmaR_ = R;
 	passTmaS_ = (uint32_t)g.S;
 	passTmaSmem_ = smem;
@@ -1525,19 +1726,21 @@ std::string Simulator::enqueueStep(uint32_t k, bool instrument, bool chained)
 		if (passTmaFn_) {
 			// the per-tile pass takes the single network's descriptor too; the
 			// vector pass takes it alone
-			// chained single steps: the pass's last CTA waits for the step's
+			// chained steps: the pass's last CTA waits for the step's
 			// small-cell kernel (passExitWait) on this simulator's counter
 			uint32_t *exitArg = chained ? (uint32_t *)dExitCount_.ptr : nullptr;
-			void *argsTma[] = {&netsArg, &offsArg, &numNetsArg, &stepArg, &net0Arg, &stepMF_, &exitArg};
+			const PassBlock *blocksArg = (const PassBlock *)dPassBlocks_.ptr;
+			void *argsTma[] = {&blocksArg, &passEvents_, &stepArg, &net0Arg, &stepMF_, &exitArg};
+			void *argsPersist[] = {&netsArg, &offsArg, &numNetsArg, &stepArg};
 			void *argsVec[] = {&net0Arg, &stepArg, &vecClaimArg};
 			const uint32_t *unitOffArg = (const uint32_t *)dVecUnitOffset_.ptr;
 			const uint32_t *pcOffArg = (const uint32_t *)dVecPcOffset_.ptr;
 			uint32_t *claimArg = (uint32_t *)dVecClaim_.ptr;
 			void *argsVecBatch[] = {&netsArg, &unitOffArg, &pcOffArg, &numNetsArg, &stepArg, &claimArg};
-			void **args = !passVec_ ? argsTma : nets_.size() == 1 ? argsVec : argsVecBatch;
+			void **args = passPersistent_ ? argsPersist : !passVec_ ? argsTma : nets_.size() == 1 ? argsVec : argsVecBatch;
 			cudaLaunchConfig_t cfg = {};
 			cfg.gridDim = dim3(passGrid_);
-			cfg.blockDim = dim3(32 * (passTmaW_ + 1));
+			cfg.blockDim = dim3(passTmaThreads_);
 			cfg.dynamicSmemBytes = passTmaSmem_;
 			cfg.stream = st;
 			cudaLaunchAttribute attr;
@@ -1578,7 +1781,7 @@ std::string Simulator::enqueueStep(uint32_t k, bool instrument, bool chained)
 		return recordStep(k);
 	}
 	if (chained) {
-		// steps launched one at a time: the small-cell kernel is the
+		// with the per-tile pass: the small-cell kernel is the
 		// programmatic dependent of the previous step's GR pass and waits for
 		// it on the device (pdlWait, cbm_kernels.cuh), so that it is resident
 		// when that pass ends; the GR pass follows as before, and its exit
@@ -1670,7 +1873,7 @@ std::string Simulator::launchSteps(uint32_t nsteps)
 		mailboxArg_ = nets_.size() == 1 ? nets_[0]->dMailbox_ : nullptr;
 		// the chain needs the per-tile pass's exit wait; other pass kinds
 		// are launched in plain stream order
-		std::string e = enqueueStep(directPending_, false, passTmaFn_ && !passVec_ && !passPersistent_);
+		std::string e = enqueueStep(directPending_, false, chains());
 		mailboxArg_ = nullptr;
 		stepMF_.n = 0;
 		if (!e.empty()) return e;
@@ -1900,7 +2103,7 @@ std::string Simulator::runGraph(uint64_t nsteps, uint32_t chunk, bool instrument
 		cudaGraph_t g;
 		CK(cudaStreamBeginCapture(s0_, cudaStreamCaptureModeThreadLocal), "graph capture");
 		for (uint32_t k = 0; k < chunk; k++) {
-			std::string e = enqueueStep(k, instrument);
+			std::string e = enqueueStep(k, instrument, chains());
 			if (!e.empty()) { cudaStreamEndCapture(s0_, &g); return e; }
 		}
 		advanceStepKernel<<<1, 64, 0, s0_>>>((uint64_t *const *)dTBasePtrs_.ptr, (int)nets_.size(), chunk);

@@ -105,6 +105,7 @@ public:
 	std::vector<PassGeometry> passCandidates() const;
 	const PassGeometry &passGeometryInUse() const { return passGeom_; }
 	std::string usePassGeometry(const PassGeometry &g);
+	bool passTmaFits(const PassGeometry &g, size_t *smem) const;
 	// Device error word of every network (kErr* bits): non-empty on error.
 	std::string checkDeviceErrors();
 	void passGeometry(unsigned *kind, unsigned *warps, unsigned *rows, unsigned *stages) const
@@ -147,6 +148,7 @@ private:
 	cudaStream_t s0_ = nullptr, s1_ = nullptr;
 	cudaEvent_t fork_ = nullptr, join_ = nullptr, ev0_ = nullptr, ev1_ = nullptr, tev0_ = nullptr, tev1_ = nullptr;
 	DeviceBuf dNetPtrs_, dBlockOffset_, dTBasePtrs_, dStageBytes_;
+	DeviceBuf dPassBlocks_;   // the per-tile pass's CTAs (batches)
 	DeviceBuf dExitCount_;    // the per-tile pass's CTAs that finished a chained single step (passExitWait)
 	DeviceBuf dCellOffset_;   // trialDataBatchKernel's instance map (batches recording trial data)
 	// the batched vector pass: first 128-cell unit and first PC of each
@@ -157,7 +159,10 @@ private:
 	size_t passSmem_ = 0, tailSmem_ = 0;
 	// TMA GR pass geometry (passTmaFn_ null: the plain pass kernel runs)
 	const void *passTmaFn_ = nullptr;
-	uint32_t passTmaW_ = 0, passTmaR_ = 0, passTmaS_ = 0, passGrid_ = 0;
+	// the per-tile pass: a step's kernels chain to the next step's (enqueueStep)
+	bool chains() const { return passTmaFn_ && !passVec_ && !passPersistent_; }
+	uint32_t passTmaW_ = 0, passTmaR_ = 0, passTmaS_ = 0, passTmaThreads_ = 0, passGrid_ = 0;
+	uint32_t passEvents_ = 0;  // the per-tile pass's event CTAs (one network)
 	bool passPersistent_ = false;
 	bool passVec_ = false;  // the vector pass (kind 3) runs
 	// the small-cell kernel argument of the step being enqueued: the NC
@@ -229,9 +234,26 @@ public:
 	std::string setPcSumMode(bool on, cudaStream_t s);
 	bool passTmaCapable() const { return h_.J == 32; }
 	uint32_t passRows() const { return 2 * h_.K; }
+	uint32_t eventBlocks() const { return (h_.numGR + kEvCells - 1) / kEvCells; }
 	// Encode the TMA descriptors for boxes of R rows and upload them.
 	std::string buildPassMaps(uint32_t R);
-	size_t passTmaSmemBytes(uint32_t R, uint32_t S, uint32_t outBytes = 4) const;
+	// The per-tile pass's tiling for about `target` cells a tile and stages of
+	// SC cells (false: no tiling fits), and its shared memory in that tiling
+	// with S stages.
+	bool eventTiling(uint32_t target, uint32_t SC, DevNet *h) const;
+	static size_t eventSmemBytes(const DevNet &h, uint32_t SC, uint32_t S);
+	// Tile the cells and build the event tables unless they are there.
+	std::string buildEventPass(uint32_t target, uint32_t SC, cudaStream_t s);
+	// Enter or leave the per-tile pass's form of the state: GR->GO counts
+	// delivered when cells spike instead of when the spikes arrive, the
+	// conductances one step behind with the arrived spikes beside them, and the
+	// GR arrays in tile order.
+	std::string setEventMode(bool on, cudaStream_t s);
+	std::string reorder(void *a, uint32_t size, uint32_t rows, bool toTile, cudaStream_t s);
+	std::string exportGR(const void *src, uint32_t size, void *tmp, void *dst, cudaStream_t s);
+	std::string scratch(void **p);
+	uint64_t *scratch_ = nullptr;
+	bool conductancesPending() const { return evMode_ && hostT_ >= h_.evFirst; }
 	size_t zoneScratchBytes() const;
 	// shared memory a small-cell CTA may use (the staged arrays included)
 	static constexpr size_t kTailSmemBudget = 200 * 1024;
@@ -260,10 +282,8 @@ private:
 	std::vector<void *> allocs_;
 	std::map<const void *, size_t> allocBytes_;
 	double avgMF_ = 0, avgGO_ = 0, avgOut_ = 0;
-	uint32_t outBytes_ = 4;  // bytes per GR->GO slot the GR pass in use streams
-	uint32_t outPlanes_ = 0; // GR->GO slot planes it streams
-	size_t ovEntries_ = 0;   // GR->GO synapses in the per-tile lists
-	size_t ovUsed_ = 0;      // those the GR pass in use reads (0 unless the per-tile pass)
+	bool streamsSlots_ = true;  // the GR pass in use streams the synapse tables (not the per-tile pass)
+	bool evMode_ = false;       // the state is in the per-tile pass's form (setEventMode)
 	// pinned staging of host MF input: kMFStage slots, each reused once the
 	// copy that last read it has run (mfStageEv_)
 	uint32_t *hErr_ = nullptr;  // the error word (mapped pinned host memory; h_.errFlag maps it)

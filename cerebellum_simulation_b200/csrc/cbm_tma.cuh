@@ -87,5 +87,14 @@ __device__ __forceinline__ void load3d(void *dst, const void *map, int32_t x, in
 		: "memory");
 }
 
+// Untiled load of `bytes` (a multiple of 16) from 16-byte aligned global memory.
+__device__ __forceinline__ void loadBulk(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
+{
+	asm volatile(
+		"cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+		::"r"(smemAddr(dst)), "l"(src), "r"(bytes), "r"(smemAddr(bar))
+		: "memory");
+}
+
 }  // namespace tma
 }  // namespace cbm
