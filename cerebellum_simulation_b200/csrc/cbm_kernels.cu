@@ -56,7 +56,11 @@ __device__ uint64_t kExp2Tab[32] = {
 // exp of a float: x = (k + r) ln2/32, 2^(k/32) from the table (kExp2Tab or
 // a shared-memory copy), 2^(r/32) from a cubic in r (coefficients of the
 // published algorithm).
-__device__ float cbmExpf(float x, const uint64_t *__restrict__ tab)
+// Not inlined: the small-cell kernel runs each piece of its code once a step and
+// spends much of its time on fetching it; with one copy for the eight calls a
+// 256K step took 12.8 instead of 13.0 us, a 1M one after an L2 flush 25.1
+// instead of 26.7.
+__device__ __noinline__ float cbmExpf(float x, const uint64_t *__restrict__ tab)
 {
 	const uint32_t ux = __float_as_uint(x);
 	const uint32_t abstop = (ux >> 20) & 0x7ffu;
@@ -1129,18 +1133,40 @@ __device__ void zoneRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm,
 	// ---- microzone outputs (mzone.cpp:409-524) and the MF->NC population
 	// bookkeeping (mzone.cpp:536-580): independent gathers, run as one flat
 	// task space so that their loads are in flight together
-	const bool popStep = stepMod(t, N->tsPerPopHistBinPC) == 0;
+	const bool popStep = stepMod(t, N->tsPerPopHistBinPC) == 0, nextPlast = stepMod(t + 1, N->tsPerHistBinGR) == 0;
 	// the device protocol's record of step t (its NC and PC spikes are final
 	// now) on the last warp, beside the outputs: neither reads what the
 	// other writes
 	const bool recWarp = N->proto != nullptr && warp == nWarps - 1;
 	const uint32_t oThr = N->proto != nullptr ? nThr - 32u : nThr;
 	if (recWarp) protocolRecordWarp(N, t, lane);
-	{
+	// the longest chains on warps of their own, beside the others' gathers: the
+	// first takes the NC->IO release probabilities (mzone.cpp:492-504), the second
+	// the release draws' random numbers; the plasticity selector is made where its
+	// timer is.  (The draws and the selector as a phase of their own, behind
+	// one more barrier, took 2.7 us of a 16K network's 12.7 us step; so 11.8.)
+	if (warp == 0) {
+		for (uint32_t r = lane; r < Z * numNC; r += 32u) {
+			const uint32_t z = Z == 1 ? 0u : r / numNC, i = Z == 1 ? r : r % numNC;
+			const DevZone &Q = N->zones[z];
+			const uint8_t apNC = Q.apNC[i];
+			float p = Q.synIOPReleaseNC[i];
+			p = p * cbmExpf(-N->msPerTimeStep / (N->relPDecTSofNCtoIO * cbmExpf(-p / N->relPDecTTofNCtoIO, exp2) + N->relPDecT0ofNCtoIO), exp2);
+			p = p + apNC * N->relPIncNCtoIO * cbmExpf(-p / N->relPIncTauNCtoIO, exp2);
+			Q.synIOPReleaseNC[i] = p;
+		}
+	} else if (warp == 1) {
+		// (the IO updates have read ioScratch)
+		for (uint32_t r = lane; r < Z * numIO * nIONC; r += 32u) {
+			const uint32_t per = numIO * nIONC;
+			const uint32_t z = Z == 1 ? 0u : r / per, k = Z == 1 ? r : r % per;
+			ioScratch[r] = rng::uniform24Keyed(N->zones[z].ncioKey, rng::ncioCounter(t, k / nIONC, k % nIONC, nIONC));
+		}
+	} else if (!recWarp) {
 		const uint32_t nMFIn = Z * numNC * nMFNC, nBCPC = Z * numPC, nSCPC = Z * numPC * N->numpPCfromSCtoPC,
-			nPCBC = Z * numBC, nPCNC = Z * numNC * N->numpNCfromPCtoNC, nIO = Z * numIO, nNC = Z * numNC;
-		const uint32_t total = nMFIn + nBCPC + nSCPC + nPCBC + nPCNC + nIO + nNC + Z;
-		for (uint32_t task = recWarp ? total : tid; task < total; task += oThr) {
+			nPCBC = Z * numBC, nPCNC = Z * numNC * N->numpNCfromPCtoNC, nIO = Z * numIO;
+		const uint32_t total = nMFIn + nBCPC + nSCPC + nPCBC + nPCNC + nIO + Z;
+		for (uint32_t task = tid - 64u; task < total; task += oThr - 64u) {
 			uint32_t r = task;
 			if (r < nMFIn) {
 				const uint32_t z = Z == 1 ? 0u : r / (numNC * nMFNC), k = Z == 1 ? r : r % (numNC * nMFNC);
@@ -1194,22 +1220,15 @@ __device__ void zoneRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm,
 				float vc = 0;
 				for (uint32_t j = 0; j < N->numpIOInIOIO; j++)
 					vc = vc + N->coupleRiRjRatioIO * (Q.vIO[Q.pIOInIOIO[(size_t)i * N->numpIOInIOIO + j]] - vOwn);
-				Q.pfPCPlastTimerIO[i] = (!ap) * (timer + 1) + ap * N->tsLTDStartAPIO;
+				const int32_t tm = (!ap) * (timer + 1) + ap * N->tsLTDStartAPIO;
+				Q.pfPCPlastTimerIO[i] = tm;
 				Q.vCoupleIO[i] = vc;
+				// plasticity selector of the next step
+				Q.plastSel[((t + 1) & 1) * numIO + i] =
+					!nextPlast ? 0 : tm < N->tsLTDEndIO ? 1 : (tm > N->tsLTPStartAPIO ? 2 : 0);
 				continue;
 			}
 			r -= nIO;
-			if (r < nNC) {
-				const uint32_t z = Z == 1 ? 0u : r / numNC, i = Z == 1 ? r : r % numNC;
-				const DevZone &Q = N->zones[z];
-				const uint8_t apNC = Q.apNC[i];
-				float p = Q.synIOPReleaseNC[i];
-				p = p * cbmExpf(-N->msPerTimeStep / (N->relPDecTSofNCtoIO * cbmExpf(-p / N->relPDecTTofNCtoIO, exp2) + N->relPDecT0ofNCtoIO), exp2);
-				p = p + apNC * N->relPIncNCtoIO * cbmExpf(-p / N->relPIncTauNCtoIO, exp2);
-				Q.synIOPReleaseNC[i] = p;
-				continue;
-			}
-			r -= nNC;
 			{
 				// updateMFNCSyn's population-activity bookkeeping for zone r
 				const DevZone &Q = N->zones[r];
@@ -1237,52 +1256,36 @@ __device__ void zoneRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm,
 	__syncthreads();
 
 	// NC->IO release draws (mzone.cpp:505-511), MF->NC plasticity
-	// (mzone.cpp:586-600), plasticity selector of the next step
+	// (mzone.cpp:586-600)
 	{
-		const uint32_t nDraw = Z * numIO * nIONC, nW = popStep ? Z * numNC * nMFNC : 0, nSel = Z * numIO;
-		const bool nextPlast = stepMod(t + 1, N->tsPerHistBinGR) == 0;
-		for (uint32_t task = tid; task < nDraw + nW + nSel; task += nThr) {
+		const uint32_t nDraw = Z * numIO * nIONC, nW = popStep ? Z * numNC * nMFNC : 0;
+		for (uint32_t task = tid; task < nDraw + nW; task += nThr) {
 			uint32_t r = task;
 			if (r < nDraw) {
 				const uint32_t per = numIO * nIONC;
 				const uint32_t z = Z == 1 ? 0u : r / per, k = Z == 1 ? r : r % per;
-				const uint32_t i = k / nIONC, j = k % nIONC;
 				const DevZone &Q = N->zones[z];
-				const double u = (double)rng::uniform24Keyed(Q.ncioKey, rng::ncioCounter(t, i, j, nIONC));
-				Q.inputNCIO[k] = (u < Q.synIOPReleaseNC[Q.pIOfromNCtoIO[k]]);
+				Q.inputNCIO[k] = ((double)ioScratch[r] < Q.synIOPReleaseNC[Q.pIOfromNCtoIO[k]]);
 				continue;
 			}
 			r -= nDraw;
-			if (r < nW) {
-				const uint32_t z = Z == 1 ? 0u : r / (numNC * nMFNC), k = Z == 1 ? r : r % (numNC * nMFNC);
-				const DevZone &Q = N->zones[z];
-				const int doLTD = sFlags[2 * z], doLTP = sFlags[2 * z + 1];
-				const float wOld = Q.mfSynWeightNC[k];
-				const float synWDelta = N->histMF[Q.pNCfromMFtoNC[k]] *
-					(doLTD * N->synLTDStepSizeMFtoNC + doLTP * N->synLTPStepSizeMFtoNC);
-				float w = wOld;
-				w = w + synWDelta;
-				w = (w > 0) * w;
-				w = (w <= 1) * w + (w > 1);
-				Q.mfSynWeightNC[k] = w;
-				continue;
-			}
-			r -= nW;
-			{
-				const uint32_t z = Z == 1 ? 0u : r / numIO, i = Z == 1 ? r : r % numIO;
-				const DevZone &Q = N->zones[z];
-				uint8_t sel = 0;
-				if (nextPlast) {
-					const int32_t tm = Q.pfPCPlastTimerIO[i];
-					sel = tm < N->tsLTDEndIO ? 1 : (tm > N->tsLTPStartAPIO ? 2 : 0);
-				}
-				Q.plastSel[((t + 1) & 1) * numIO + i] = sel;
-			}
+			const uint32_t z = Z == 1 ? 0u : r / (numNC * nMFNC), k = Z == 1 ? r : r % (numNC * nMFNC);
+			const DevZone &Q = N->zones[z];
+			const int doLTD = sFlags[2 * z], doLTP = sFlags[2 * z + 1];
+			const float wOld = Q.mfSynWeightNC[k];
+			const float synWDelta = N->histMF[Q.pNCfromMFtoNC[k]] *
+				(doLTD * N->synLTDStepSizeMFtoNC + doLTP * N->synLTPStepSizeMFtoNC);
+			float w = wOld;
+			w = w + synWDelta;
+			w = (w > 0) * w;
+			w = (w <= 1) * w + (w > 1);
+			Q.mfSynWeightNC[k] = w;
 		}
 	}
-	__syncthreads();
-	if (stepMod(t, N->numTSinMFHist) == 0)
+	if (stepMod(t, N->numTSinMFHist) == 0) {
+		__syncthreads();
 		for (uint32_t i = tid; i < numMF; i += nThr) N->histMF[i] = 0;
+	}
 	// the error drive is consumed once (mzone.cpp:334)
 	if (tid < Z) ctl->errDrive[tid] = 0;
 }
