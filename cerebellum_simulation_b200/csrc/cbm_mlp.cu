@@ -3,8 +3,10 @@
 // kernel, gemmKernel, on the 5th-generation tensor cores: BF16 operands staged
 // in shared memory in the canonical K-major layout, tcgen05.mma issued by one
 // thread, the FP32 accumulator in tensor memory read back with tcgen05.ld for
-// the epilogue (bias, ReLU, FP32 and/or BF16 store).  Weights are kept in
-// FP32 (Adam) and rounded to BF16 for the products.
+// the epilogue (bias, ReLU, ReLU derivative or loss gradient, FP32 and/or BF16
+// store).  Weights are kept in FP32 (Adam) and rounded to BF16 for the products.
+// A minibatch is a chain of eight small launches, each waiting for the last on
+// the device (programmatic dependent launch).
 //
 // No counterpart in the reference (its parameter sweeps simulate every
 // candidate).
@@ -21,6 +23,8 @@
 #include <cuda_runtime.h>
 
 #include "../../include/cbm_surrogate.h"
+#include "cbm_device.cuh"
+#include "cbm_kernels.cuh"
 #include "cbm_tma.cuh"
 
 extern thread_local std::string g_cbmLastError;
@@ -29,7 +33,14 @@ namespace cbm {
 namespace mlp {
 
 constexpr uint64_t kMmaWaitLimitNs = 2000000000ull;
-constexpr int kKChunk = 64;  // K elements staged per round
+constexpr int kTileM = 128, kTileN = 32;  // one CTA's output
+constexpr int kThreads = 256;
+constexpr int kKChunk = 256;              // K elements staged per round
+// A staged operand: row r, 16-byte K piece c at (r / 8) kSBO + c kLBO + (r % 8) 16.
+// The 16 bytes beyond a core matrix, and beyond a row group, keep neighbouring
+// pieces and neighbouring row groups on different banks.
+constexpr uint32_t kLBO = 128 + 16, kSBO = (kKChunk / 8) * kLBO + 16;
+constexpr uint32_t kGemmSmem = 128 + (kTileM + kTileN) / 8 * kSBO;
 
 __device__ __forceinline__ uint32_t smemU32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -58,26 +69,129 @@ __host__ __device__ constexpr uint32_t instrDesc(uint32_t n)
 		| ((128u >> 4) << 24);  // M / 16
 }
 
-// out[m][n] = act(sum_k A[m][k] * B[n][k] + bias[n]) for m < M, n < N.
-// A is M x K, B is N x K, both BF16 row-major (K contiguous, lda = ldb = K);
-// K is a multiple of 64; N <= NT.  One CTA of 128 threads per 128-row tile.
-// outF (FP32, leading dimension ldo) and outH (BF16, ldo) may each be null.
-template <int NT>
-__global__ void __launch_bounds__(128) gemmKernel(const __nv_bfloat16 *__restrict__ A, const __nv_bfloat16 *__restrict__ B,
-		int M, int N, int K, const float *__restrict__ bias, int relu, float *outF, __nv_bfloat16 *outH, int ldo,
-		uint32_t *err)
+// One product, out[m][n] = f(sum_k A(m,k) B(n,k)) for m < M, n < N, or the
+// column sums of a matrix (colSum != null).
+// A(m,k) is A[m lda + k], or A[k lda + m] with tA (a product over the batch, or
+// with a transposed weight matrix, reads its operand as it lies); B alike.  N, lda
+// and ldb are multiples of 64, and K, but for an operand pair that is transposed.
+struct GemmJob {
+	const __nv_bfloat16 *A = nullptr, *B = nullptr;
+	int M = 0, N = 0, K = 0, lda = 0, ldb = 0;
+	bool tA = false, tB = false, relu = false;
+	const float *bias = nullptr;          // [N], added
+	const __nv_bfloat16 *mask = nullptr;  // [M][N]: 0 where it is not positive (the ReLU derivative)
+	// mean squared error against target [M][nOut]: the outputs are 2 (v - target) / (M nOut),
+	// 0 for n >= nOut, and the squares are added to *loss
+	const float *target = nullptr;
+	float *loss = nullptr;
+	float *outF = nullptr;                // FP32 [M][ldo], columns < nOut
+	__nv_bfloat16 *outH = nullptr;        // BF16 [M][N]
+	int ldo = 0, nOut = 0;
+	const float *colSum = nullptr;        // [M][N]: outF[n] = sum over m
+};
+struct GemmJobs {
+	GemmJob j[4];
+};
+
+// Rows [r0, r0 + ROWS) of an operand (R valid), K elements [k0, k0 + kPad) of
+// K, into its staged layout; zeros outside.
+template <int ROWS>
+__device__ __forceinline__ void stageOperand(uint8_t *s, const __nv_bfloat16 *X, int ld, bool trans, int r0, int R,
+		int k0, int K, int kPad)
 {
+	const int tid = threadIdx.x;
+	if (!trans) {
+		// 16-byte pieces along K, all in flight (no registers)
+		const int pieces = kPad / 8;
+		for (int q = tid; q < ROWS * pieces; q += kThreads) {
+			const int r = q / pieces, c = q % pieces;
+			uint8_t *d = s + (r / 8) * kSBO + c * kLBO + (r % 8) * 16;
+			if (r0 + r < R)
+				asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smemU32(d)),
+						"l"(X + (size_t)(r0 + r) * ld + k0 + c * 8) : "memory");
+			else
+				*reinterpret_cast<uint4 *>(d) = make_uint4(0, 0, 0, 0);
+		}
+		return;
+	}
+	// two consecutive K rows of eight elements at a time, transposed in registers
+	constexpr int G = ROWS / 8, U = ROWS >= 128 ? 8 : 2;
+	const int pairs = kPad / 2 * G;
+	for (int q0 = tid; q0 < pairs; q0 += U * kThreads) {
+		uint4 v[U][2];
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			const int q = q0 + u * kThreads, g = q % G, k = k0 + 2 * (q / G);
+			v[u][0] = v[u][1] = make_uint4(0, 0, 0, 0);
+			if (q < pairs && r0 + 8 * g < R) {
+				if (k < K) v[u][0] = *reinterpret_cast<const uint4 *>(X + (size_t)k * ld + r0 + 8 * g);
+				if (k + 1 < K) v[u][1] = *reinterpret_cast<const uint4 *>(X + (size_t)(k + 1) * ld + r0 + 8 * g);
+			}
+		}
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			const int q = q0 + u * kThreads, g = q % G, k = 2 * (q / G);
+			if (q >= pairs) break;
+			uint8_t *d = s + g * kSBO + (k / 8) * kLBO + (k % 8) * 2;
+			const uint32_t a[4] = {v[u][0].x, v[u][0].y, v[u][0].z, v[u][0].w};
+			const uint32_t b[4] = {v[u][1].x, v[u][1].y, v[u][1].z, v[u][1].w};
+#pragma unroll
+			for (int i = 0; i < 4; i++) {
+				*reinterpret_cast<uint32_t *>(d + 32 * i) = __byte_perm(a[i], b[i], 0x5410);
+				*reinterpret_cast<uint32_t *>(d + 32 * i + 16) = __byte_perm(a[i], b[i], 0x7632);
+			}
+		}
+	}
+}
+
+// Column sums of columns [32 blockIdx.y, + 32): eight row groups, then a tree.
+__device__ void colSums(const GemmJob &J, float *s)
+{
+	const int c = threadIdx.x % 32, g = threadIdx.x / 32, n = 32 * blockIdx.y + c;
+	float x = 0.0f;
+#pragma unroll 8
+	for (int r = g; r < J.M; r += kThreads / 32) x += J.colSum[(size_t)r * J.N + n];
+	s[threadIdx.x] = x;
+	__syncthreads();
+	if (g == 0) {
+		float y[8];
+#pragma unroll
+		for (int i = 0; i < 8; i++) y[i] = s[32 * i + c];
+		J.outF[n] = ((y[0] + y[4]) + (y[2] + y[6])) + ((y[1] + y[5]) + (y[3] + y[7]));
+	}
+}
+
+// The products of these layers (at most 256 wide) are tiny: what bounds them is
+// latency, one round trip for the operands, the MMAs, one store.  So a CTA takes
+// 128 x 32 outputs and stages its operands' whole depth (up to 256) with every
+// load in flight before one wait; two independent products of the backward pass
+// share a launch (blockIdx.z).  A 128 x 256 tile in rounds of 64 K elements, each
+// waiting for its loads and its MMAs, on one or two CTAs took 30-62 us a product;
+// transposed copies of the operands, the ReLU derivative and the loss were
+// launches of their own.  A 64-256-256-50 network's gradients over 200 rows took
+// 518 us and take 139, a training minibatch of 256 took 482 and takes 92, a
+// forward pass over 256 rows 228 and 58 (copies to and from the host included).
+__global__ void __launch_bounds__(kThreads) gemmKernel(const __grid_constant__ GemmJobs jobs, uint32_t *err)
+{
+	pdlLaunchDependents();
 	extern __shared__ uint8_t gemmSmemRaw[];
-	uint8_t *sA = gemmSmemRaw + ((1024u - (smemU32(gemmSmemRaw) & 1023u)) & 1023u);
-	uint8_t *sB = sA + 128 * kKChunk * 2;
+	const GemmJob &J = jobs.j[blockIdx.z];
+	const int m0 = blockIdx.x * kTileM, n0 = blockIdx.y * kTileN;
+	uint8_t *sA = gemmSmemRaw + ((128u - (smemU32(gemmSmemRaw) & 127u)) & 127u);
+	if (n0 >= J.N || (J.colSum ? blockIdx.x > 0 : m0 >= J.M)) return;
+	if (J.colSum) {
+		pdlWait();
+		colSums(J, reinterpret_cast<float *>(sA));
+		return;
+	}
+	uint8_t *sB = sA + kTileM / 8 * kSBO;
 	__shared__ __align__(8) uint64_t bar;
 	__shared__ uint32_t tmemBase;
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-	const int m0 = blockIdx.x * 128;
 
 	if (warp == 0) {
 		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemU32(&tmemBase)),
-				"r"((uint32_t)NT) : "memory");
+				"r"((uint32_t)kTileN) : "memory");
 		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 	}
 	if (tid == 0) {
@@ -88,32 +202,21 @@ __global__ void __launch_bounds__(128) gemmKernel(const __nv_bfloat16 *__restric
 	__syncthreads();
 	asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 	const uint32_t tmem = tmemBase;
+	pdlWait();
 
-	// canonical layout of a staged chunk: row r, 16-byte K piece c at
-	// (r / 8) * SBO + c * 128 + (r % 8) * 16, SBO = (kKChunk / 8) * 128
-	constexpr uint32_t kLBO = 128, kSBO = (kKChunk / 8) * 128;
-	constexpr uint32_t idesc = instrDesc(NT);
+	constexpr uint32_t idesc = instrDesc(kTileN);
 	bool ok = true;
-	for (int k0 = 0; k0 < K; k0 += kKChunk) {
-		// stage A rows [m0, m0+128) and B rows [0, NT) of columns [k0, k0+64)
-		for (int q = tid; q < 128 * (kKChunk / 8); q += blockDim.x) {
-			const int r = q / (kKChunk / 8), c = q % (kKChunk / 8);
-			uint4 v = make_uint4(0, 0, 0, 0);
-			if (m0 + r < M) v = *reinterpret_cast<const uint4 *>(A + (size_t)(m0 + r) * K + k0 + c * 8);
-			*reinterpret_cast<uint4 *>(sA + (r / 8) * kSBO + c * kLBO + (r % 8) * 16) = v;
-		}
-		for (int q = tid; q < NT * (kKChunk / 8); q += blockDim.x) {
-			const int r = q / (kKChunk / 8), c = q % (kKChunk / 8);
-			uint4 v = make_uint4(0, 0, 0, 0);
-			if (r < N) v = *reinterpret_cast<const uint4 *>(B + (size_t)r * K + k0 + c * 8);
-			*reinterpret_cast<uint4 *>(sB + (r / 8) * kSBO + c * kLBO + (r % 8) * 16) = v;
-		}
+	for (int k0 = 0, round = 0; k0 < J.K; k0 += kKChunk, round++) {
+		const int kPad = (min(kKChunk, J.K - k0) + 15) & ~15;
+		stageOperand<kTileM>(sA, J.A, J.lda, J.tA, m0, J.M, k0, J.K, kPad);
+		stageOperand<kTileN>(sB, J.B, J.ldb, J.tB, n0, J.N, k0, J.K, kPad);
+		asm volatile("cp.async.wait_all;" ::: "memory");
 		// make the generic-proxy stores visible to the tensor cores
 		asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 		__syncthreads();
 		if (tid == 0) {
 			asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-			for (int ks = 0; ks < kKChunk; ks += 16) {
+			for (int ks = 0; ks < kPad; ks += 16) {
 				const uint64_t da = smemDesc(smemU32(sA) + (ks / 8) * kLBO, kLBO, kSBO);
 				const uint64_t db = smemDesc(smemU32(sB) + (ks / 8) * kLBO, kLBO, kSBO);
 				const uint32_t accumulate = (k0 > 0 || ks > 0) ? 1u : 0u;
@@ -128,128 +231,119 @@ __global__ void __launch_bounds__(128) gemmKernel(const __nv_bfloat16 *__restric
 					::"r"(smemU32(&bar)) : "memory");
 		}
 		// the chunk's MMAs have read shared memory once the barrier flips
-		const bool done = tma::waitBounded(&bar, (uint32_t)((k0 / kKChunk) & 1), kMmaWaitLimitNs);
+		const bool done = tma::waitBounded(&bar, (uint32_t)(round & 1), kMmaWaitLimitNs);
 		if (!__syncthreads_and(done)) {
 			ok = false;
 			break;
 		}
 		asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 	}
+	float e2 = 0.0f;
 	if (!ok) {
 		if (tid == 0) atomicOr(err, 1u);
 	} else {
-		// epilogue: warp w owns TMEM lanes (rows) 32w..32w+31
-		const int m = m0 + warp * 32 + lane;
-		for (int c0 = 0; c0 < NT; c0 += 16) {
-			uint32_t r[16];
-			const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
-			asm volatile(
-				"tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-				: "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-				  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-				: "r"(taddr));
-			asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-			if (m < M) {
+		// epilogue: warp w owns TMEM lanes (rows) 32 (w mod 4).. and columns 16 (w / 4)..
+		const int m = m0 + (warp % 4) * 32 + lane, c0 = warp / 4 * 16, n1 = n0 + c0;
+		uint32_t r[16];
+		const uint32_t taddr = tmem + ((uint32_t)(warp % 4 * 32) << 16) + (uint32_t)c0;
+		asm volatile(
+			"tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+			: "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+			  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+			: "r"(taddr));
+		asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+		if (m < J.M) {
+			float v[16];
+#pragma unroll
+			for (int j = 0; j < 16; j++) v[j] = __uint_as_float(r[j]);
+			if (J.bias)
+#pragma unroll
+				for (int j = 0; j < 16; j++) v[j] += __ldg(J.bias + n1 + j);
+			if (J.relu)
+#pragma unroll
+				for (int j = 0; j < 16; j++) v[j] = v[j] > 0.0f ? v[j] : 0.0f;
+			if (J.mask) {
+				__align__(16) __nv_bfloat16 h[16];
+				*reinterpret_cast<uint4 *>(h) = *reinterpret_cast<const uint4 *>(J.mask + (size_t)m * J.N + n1);
+				*reinterpret_cast<uint4 *>(h + 8) = *reinterpret_cast<const uint4 *>(J.mask + (size_t)m * J.N + n1 + 8);
+#pragma unroll
+				for (int j = 0; j < 16; j++) v[j] = __bfloat162float(h[j]) > 0.0f ? v[j] : 0.0f;
+			}
+			if (J.target)
 #pragma unroll
 				for (int j = 0; j < 16; j++) {
-					const int n = c0 + j;
-					if (n >= N) break;
-					float v = __uint_as_float(r[j]);
-					if (bias) v += bias[n];
-					if (relu) v = v > 0.0f ? v : 0.0f;
-					if (outF) outF[(size_t)m * ldo + n] = v;
-					if (outH) outH[(size_t)m * ldo + n] = __float2bfloat16_rn(v);
+					float g = 0.0f;
+					if (n1 + j < J.nOut) {
+						const float d = v[j] - J.target[(size_t)m * J.nOut + n1 + j];
+						e2 += d * d;
+						g = 2.0f * d / ((float)J.M * (float)J.nOut);
+					}
+					v[j] = g;
 				}
+			if (J.outF) {
+				float *o = J.outF + (size_t)m * J.ldo + n1;
+				if (J.ldo == J.N)
+#pragma unroll
+					for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4 *>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+				else
+#pragma unroll
+					for (int j = 0; j < 16; j++)
+						if (n1 + j < J.nOut) o[j] = v[j];
 			}
+			if (J.outH) {
+				__align__(16) __nv_bfloat16 h[16];
+#pragma unroll
+				for (int j = 0; j < 16; j++) h[j] = __float2bfloat16_rn(v[j]);
+				uint4 *o = reinterpret_cast<uint4 *>(J.outH + (size_t)m * J.N + n1);
+				o[0] = *reinterpret_cast<const uint4 *>(h);
+				o[1] = *reinterpret_cast<const uint4 *>(h + 8);
+			}
+		}
+		if (J.target) {
+			for (int o = 16; o > 0; o >>= 1) e2 += __shfl_down_sync(0xffffffffu, e2, o);
+			if (lane == 0 && e2 != 0.0f) atomicAdd(J.loss, e2);
 		}
 	}
 	asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 	__syncthreads();
 	if (warp == 0)
-		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)NT) : "memory");
+		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)kTileN) : "memory");
 }
 
 // ------------------------------------------------------------ elementwise
-__global__ void toBf16Kernel(const float *in, __nv_bfloat16 *out, size_t n)
+// The rows x nIn input as BF16 rows of I (zeros beyond nIn), the parameters as
+// BF16 (nP of them, or 0 to leave the copy), and the loss to 0.
+__global__ void prepareKernel(const float *x, uint32_t rows, uint32_t nIn, uint32_t I, __nv_bfloat16 *X, const float *P,
+		size_t nP, __nv_bfloat16 *Wh, float *loss)
 {
-	const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (i < n) out[i] = __float2bfloat16_rn(in[i]);
-}
-
-// out[c][r] = in[r][c] for r < R, 0 for R <= r < Rp; in is R x C (ld C),
-// out C x Rp (ld Rp).
-__global__ void transposeKernel(const __nv_bfloat16 *in, int R, int C, int Rp, __nv_bfloat16 *out)
-{
-	__shared__ __nv_bfloat16 tile[32][33];
-	const int c = blockIdx.x * 32 + threadIdx.x, r0 = blockIdx.y * 32;
-	for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-		const int r = r0 + j;
-		tile[j][threadIdx.x] = (r < R && c < C) ? in[(size_t)r * C + c] : __float2bfloat16_rn(0.0f);
-	}
-	__syncthreads();
-	const int oc = r0 + threadIdx.x, or0 = blockIdx.x * 32;
-	for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-		const int orow = or0 + j;
-		if (orow < C && oc < Rp) out[(size_t)orow * Rp + oc] = tile[threadIdx.x][j];
-	}
-}
-
-// Mean squared error over rows < rows and columns < cols of Y - T (both
-// rows x ld); dY = 2 (Y - T) / (rows * cols) as BF16 (zero outside), the
-// loss sum accumulated into *loss.
-__global__ void mseGradKernel(const float *Y, const float *T, int rows, int cols, int ld, float *dYf,
-		__nv_bfloat16 *dYh, float *loss)
-{
-	const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-	const size_t total = (size_t)rows * ld;
-	float e2 = 0.0f;
-	if (i < total) {
-		const int c = (int)(i % ld);
-		float g = 0.0f;
-		if (c < cols) {
-			const float d = Y[i] - T[i];
-			e2 = d * d;
-			g = 2.0f * d / ((float)rows * (float)cols);
-		}
-		dYf[i] = g;
-		dYh[i] = __float2bfloat16_rn(g);
-	}
-	for (int o = 16; o > 0; o >>= 1) e2 += __shfl_down_sync(0xffffffffu, e2, o);
-	if ((threadIdx.x & 31) == 0 && e2 != 0.0f) atomicAdd(loss, e2);
-}
-
-// g = g * (h > 0): the ReLU derivative applied to an upstream gradient; BF16 copy.
-__global__ void reluBackKernel(float *g, const __nv_bfloat16 *h, size_t n, __nv_bfloat16 *gh)
-{
-	const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+	pdlLaunchDependents();
+	pdlWait();
+	const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, n = (size_t)rows * I;
+	if (i == 0) *loss = 0.0f;
 	if (i < n) {
-		const float v = __bfloat162float(h[i]) > 0.0f ? g[i] : 0.0f;
-		g[i] = v;
-		gh[i] = __float2bfloat16_rn(v);
+		const uint32_t r = (uint32_t)(i / I), c = (uint32_t)(i % I);
+		X[i] = __float2bfloat16_rn(c < nIn ? x[(size_t)r * nIn + c] : 0.0f);
+	} else if (i - n < nP) {
+		Wh[i - n] = __float2bfloat16_rn(P[i - n]);
 	}
 }
 
-// db[c] = sum over rows of g[r][c] (rows x cols, ld cols).
-__global__ void colSumKernel(const float *g, int rows, int cols, float *db)
-{
-	const int c = blockIdx.x * blockDim.x + threadIdx.x;
-	if (c >= cols) return;
-	float s = 0.0f;
-	for (int r = 0; r < rows; r++) s += g[(size_t)r * cols + c];
-	db[c] = s;
-}
-
-// Adam (Kingma and Ba, 2015) on n parameters, bias-corrected step t.
+// Adam (Kingma and Ba, 2015) on n parameters, bias-corrected step t, and the
+// parameters' BF16 copy.
 __global__ void adamKernel(float *p, const float *g, float *m, float *v, size_t n, float lr, float b1, float b2,
-		float eps, float c1, float c2)
+		float eps, float c1, float c2, __nv_bfloat16 *h)
 {
+	pdlLaunchDependents();
+	pdlWait();
 	const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
 	const float gi = g[i];
 	const float mi = b1 * m[i] + (1 - b1) * gi, vi = b2 * v[i] + (1 - b2) * gi * gi;
 	m[i] = mi;
 	v[i] = vi;
-	p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+	const float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+	p[i] = pi;
+	h[i] = __float2bfloat16_rn(pi);
 }
 
 }  // namespace mlp
@@ -269,9 +363,9 @@ struct cbm_mlp {
 	size_t nP = 0;
 	size_t oW1 = 0, ob1 = 0, oW2 = 0, ob2 = 0, oW3 = 0, ob3 = 0;
 	// BF16 copies and activations
-	__nv_bfloat16 *Wh = nullptr, *W2t = nullptr, *W3t = nullptr;
-	__nv_bfloat16 *X = nullptr, *Xt = nullptr, *H1h = nullptr, *H1t = nullptr, *H2h = nullptr, *H2t = nullptr;
-	__nv_bfloat16 *dYh = nullptr, *dYt = nullptr, *dH2h = nullptr, *dH2t = nullptr, *dH1h = nullptr, *dH1t = nullptr;
+	__nv_bfloat16 *Wh = nullptr;
+	__nv_bfloat16 *X = nullptr, *H1h = nullptr, *H2h = nullptr, *dYh = nullptr, *dH2h = nullptr, *dH1h = nullptr;
+	// inputs, outputs and targets as the caller has them; FP32 gradients of the layers' outputs
 	float *Xf = nullptr, *Yf = nullptr, *Tf = nullptr, *dYf = nullptr, *dH2f = nullptr, *dH1f = nullptr;
 	float *loss = nullptr;
 	uint32_t *err = nullptr;
@@ -298,33 +392,56 @@ template <typename T> static T *dalloc(cbm_mlp *n, size_t count)
 	return (T *)p;
 }
 
-// C = act(A B^T + bias), A M x K, B N x K (BF16), N <= 256, K % 64 == 0.
-template <int NT> static size_t gemmSmem() { return 1024 + (size_t)(128 + NT) * kKChunk * 2; }
-
-static int gemm(cbm_mlp *n, const __nv_bfloat16 *A, const __nv_bfloat16 *B, int M, int N, int K, const float *bias,
-		bool relu, float *outF, __nv_bfloat16 *outH, int ldo)
+// One launch that may start while the one before it ends (each kernel waits for
+// it on the device, pdlWait).
+template <typename... P, typename... A>
+static int launch(cbm_mlp *n, void (*k)(P...), dim3 grid, size_t smem, const char *what, A... args)
 {
-	const dim3 grid((M + 127) / 128);
-	if (K % kKChunk) return mfail(CBM_ERR_ARG, "product depth must be a multiple of 64");
-	if (N <= 64) gemmKernel<64><<<grid, 128, gemmSmem<64>(), n->s>>>(A, B, M, N, K, bias, relu, outF, outH, ldo, n->err);
-	else if (N <= 256) gemmKernel<256><<<grid, 128, gemmSmem<256>(), n->s>>>(A, B, M, N, K, bias, relu, outF, outH, ldo, n->err);
-	else return mfail(CBM_ERR_ARG, "layer wider than 256");
-	MCK(cudaGetLastError(), "launching a tensor-core product");
+	cudaLaunchConfig_t c = {};
+	c.gridDim = grid;
+	c.blockDim = dim3(kThreads);
+	c.dynamicSmemBytes = smem;
+	c.stream = n->s;
+	cudaLaunchAttribute at = {};
+	at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	at.val.programmaticStreamSerializationAllowed = 1;
+	c.attrs = &at;
+	c.numAttrs = 1;
+	MCK(cudaLaunchKernelEx(&c, k, args...), what);
 	return CBM_OK;
 }
 
-static int transpose(cbm_mlp *n, const __nv_bfloat16 *in, int R, int C, int Rp, __nv_bfloat16 *out)
+// Independent products (and column sums), one launch.
+static int gemm(cbm_mlp *n, const std::vector<GemmJob> &jobs)
 {
-	transposeKernel<<<dim3((C + 31) / 32, (Rp + 31) / 32), dim3(32, 8), 0, n->s>>>(in, R, C, Rp, out);
-	MCK(cudaGetLastError(), "transpose");
-	return CBM_OK;
+	GemmJobs J;
+	dim3 grid(1, 1, (unsigned)jobs.size());
+	for (size_t i = 0; i < jobs.size(); i++) {
+		J.j[i] = jobs[i];
+		if (!jobs[i].colSum) grid.x = std::max(grid.x, (unsigned)((jobs[i].M + kTileM - 1) / kTileM));
+		grid.y = std::max(grid.y, (unsigned)(jobs[i].N / kTileN));
+	}
+	return launch(n, gemmKernel, grid, kGemmSmem, "launching a tensor-core product", J, n->err);
 }
 
-static int toBf16(cbm_mlp *n, const float *in, __nv_bfloat16 *out, size_t count)
+static GemmJob product(const __nv_bfloat16 *A, int lda, bool tA, const __nv_bfloat16 *B, int ldb, bool tB, int M, int N,
+		int K)
 {
-	toBf16Kernel<<<(unsigned)((count + 255) / 256), 256, 0, n->s>>>(in, out, count);
-	MCK(cudaGetLastError(), "cast");
-	return CBM_OK;
+	GemmJob j;
+	j.A = A; j.lda = lda; j.tA = tA;
+	j.B = B; j.ldb = ldb; j.tB = tB;
+	j.M = M; j.N = N; j.K = K;
+	j.ldo = j.nOut = N;
+	return j;
+}
+
+static GemmJob columnSums(const float *g, int M, int N, float *out)
+{
+	GemmJob j;
+	j.colSum = g;
+	j.M = M; j.N = N;
+	j.outF = out;
+	return j;
 }
 
 static int checkErr(cbm_mlp *n)
@@ -338,62 +455,63 @@ static int checkErr(cbm_mlp *n)
 
 #define MTRY(x) do { int r_ = (x); if (r_ != CBM_OK) return r_; } while (0)
 
-// Upload rows [0, b) of x (b x nIn, FP32) into the padded input, BF16 copy.
-static int loadInput(cbm_mlp *n, const float *x, uint32_t b)
+// The BF16 input from b uploaded rows (x on the device, b x nIn), and the
+// weights' copy when it may be old.
+static int prepare(cbm_mlp *n, const float *x, uint32_t b, bool weights, float *loss)
 {
-	std::vector<float> buf((size_t)n->Bp * n->I, 0.0f);
-	for (uint32_t r = 0; r < b; r++) memcpy(&buf[(size_t)r * n->I], x + (size_t)r * n->nIn, 4ull * n->nIn);
-	MCK(cudaMemcpyAsync(n->Xf, buf.data(), buf.size() * 4, cudaMemcpyHostToDevice, n->s), "input");
-	MTRY(toBf16(n, n->Xf, n->X, buf.size()));
-	return CBM_OK;
+	const size_t count = (size_t)b * n->I + (weights ? n->nP : 0);
+	return launch(n, prepareKernel, dim3((unsigned)((count + kThreads - 1) / kThreads)), 0, "cast", x, b, n->nIn, n->I,
+			n->X, (const float *)n->P, weights ? n->nP : (size_t)0, n->Wh, loss);
 }
 
-static int forward(cbm_mlp *n, uint32_t b)
+// Forward over b rows: the outputs to Yf (b x nOut), or, with a target (b x nOut,
+// on the device), the mean squared error's gradient to dYf and dYh and its sum to
+// *loss.
+static int forward(cbm_mlp *n, uint32_t b, const float *target, float *loss)
 {
-	const int Bp = (int)pad(b, 128);
-	MTRY(toBf16(n, n->P, n->Wh, n->nP));
 	const __nv_bfloat16 *W1 = n->Wh + n->oW1, *W2 = n->Wh + n->oW2, *W3 = n->Wh + n->oW3;
-	MTRY(gemm(n, n->X, W1, Bp, n->H1, n->I, n->P + n->ob1, true, nullptr, n->H1h, n->H1));
-	MTRY(gemm(n, n->H1h, W2, Bp, n->H2, n->H1, n->P + n->ob2, true, nullptr, n->H2h, n->H2));
-	MTRY(gemm(n, n->H2h, W3, Bp, n->O, n->H2, n->P + n->ob3, false, n->Yf, nullptr, n->O));
-	return CBM_OK;
+	const int B = (int)b;
+	GemmJob l1 = product(n->X, n->I, false, W1, n->I, false, B, n->H1, n->I);
+	l1.bias = n->P + n->ob1; l1.relu = true; l1.outH = n->H1h;
+	GemmJob l2 = product(n->H1h, n->H1, false, W2, n->H1, false, B, n->H2, n->H1);
+	l2.bias = n->P + n->ob2; l2.relu = true; l2.outH = n->H2h;
+	GemmJob l3 = product(n->H2h, n->H2, false, W3, n->H2, false, B, n->O, n->H2);
+	l3.bias = n->P + n->ob3; l3.nOut = n->nOut;
+	if (target) {
+		l3.target = target; l3.loss = loss;
+		l3.outF = n->dYf; l3.outH = n->dYh;
+	} else {
+		l3.outF = n->Yf; l3.ldo = n->nOut;
+	}
+	MTRY(gemm(n, {l1}));
+	MTRY(gemm(n, {l2}));
+	return gemm(n, {l3});
 }
 
-// Gradients of the mean squared error over the b valid rows into G.
+// Gradients of the mean squared error over the b rows of the last forward into G.
 static int backward(cbm_mlp *n, uint32_t b)
 {
-	const int B = (int)b;
-	const size_t yN = (size_t)b * n->O;
-	MCK(cudaMemsetAsync(n->loss, 0, 4, n->s), "loss");
-	mseGradKernel<<<(unsigned)((yN + 255) / 256), 256, 0, n->s>>>(n->Yf, n->Tf, B, n->nOut, n->O, n->dYf, n->dYh, n->loss);
-	MCK(cudaGetLastError(), "loss");
 	const __nv_bfloat16 *W2 = n->Wh + n->oW2, *W3 = n->Wh + n->oW3;
-	// transposed operands of the weight-gradient products, whose depth is
-	// the batch (zero-padded to a multiple of 64)
-	const int Kb = (int)pad(b, 64);
-	MTRY(transpose(n, n->dYh, B, n->O, Kb, n->dYt));      // O x Kb
-	MTRY(transpose(n, n->H2h, B, n->H2, Kb, n->H2t));     // H2 x Kb
-	MTRY(transpose(n, n->H1h, B, n->H1, Kb, n->H1t));     // H1 x Kb
-	MTRY(transpose(n, n->X, B, n->I, Kb, n->Xt));         // I x Kb
-	MTRY(transpose(n, W3, n->O, n->H2, n->O, n->W3t));    // H2 x O
-	MTRY(transpose(n, W2, n->H2, n->H1, n->H2, n->W2t));  // H1 x H2
-	// layer 3
-	MTRY(gemm(n, n->dYt, n->H2t, n->O, n->H2, Kb, nullptr, false, n->G + n->oW3, nullptr, n->H2));
-	colSumKernel<<<(n->O + 127) / 128, 128, 0, n->s>>>(n->dYf, B, n->O, n->G + n->ob3);
-	MTRY(gemm(n, n->dYh, n->W3t, B, n->H2, n->O, nullptr, false, n->dH2f, nullptr, n->H2));
-	reluBackKernel<<<(unsigned)(((size_t)B * n->H2 + 255) / 256), 256, 0, n->s>>>(n->dH2f, n->H2h, (size_t)B * n->H2, n->dH2h);
-	// layer 2
-	MTRY(transpose(n, n->dH2h, B, n->H2, Kb, n->dH2t));   // H2 x Kb
-	MTRY(gemm(n, n->dH2t, n->H1t, n->H2, n->H1, Kb, nullptr, false, n->G + n->oW2, nullptr, n->H1));
-	colSumKernel<<<(n->H2 + 127) / 128, 128, 0, n->s>>>(n->dH2f, B, n->H2, n->G + n->ob2);
-	MTRY(gemm(n, n->dH2h, n->W2t, B, n->H1, n->H2, nullptr, false, n->dH1f, nullptr, n->H1));
-	reluBackKernel<<<(unsigned)(((size_t)B * n->H1 + 255) / 256), 256, 0, n->s>>>(n->dH1f, n->H1h, (size_t)B * n->H1, n->dH1h);
-	// layer 1
-	MTRY(transpose(n, n->dH1h, B, n->H1, Kb, n->dH1t));   // H1 x Kb
-	MTRY(gemm(n, n->dH1t, n->Xt, n->H1, n->I, Kb, nullptr, false, n->G + n->oW1, nullptr, n->I));
-	colSumKernel<<<(n->H1 + 127) / 128, 128, 0, n->s>>>(n->dH1f, B, n->H1, n->G + n->ob1);
-	MCK(cudaGetLastError(), "backward");
-	return CBM_OK;
+	const int B = (int)b;
+	// weight gradients: dY^T H, products over the batch
+	auto weights = [&](const __nv_bfloat16 *d, uint32_t out, const __nv_bfloat16 *h, uint32_t in, float *g) {
+		GemmJob j = product(d, out, true, h, in, true, out, in, B);
+		j.outF = g;
+		return j;
+	};
+	// a layer's upstream gradient through the ReLU: dY W
+	auto upstream = [&](const __nv_bfloat16 *d, uint32_t out, const __nv_bfloat16 *W, uint32_t in,
+			const __nv_bfloat16 *h, float *f, __nv_bfloat16 *o) {
+		GemmJob j = product(d, out, false, W, in, true, B, in, out);
+		j.mask = h; j.outF = f; j.outH = o;
+		return j;
+	};
+	MTRY(gemm(n, {weights(n->dYh, n->O, n->H2h, n->H2, n->G + n->oW3),
+			upstream(n->dYh, n->O, W3, n->H2, n->H2h, n->dH2f, n->dH2h)}));
+	MTRY(gemm(n, {weights(n->dH2h, n->H2, n->H1h, n->H1, n->G + n->oW2),
+			upstream(n->dH2h, n->H2, W2, n->H1, n->H1h, n->dH1f, n->dH1h)}));
+	return gemm(n, {weights(n->dH1h, n->H1, n->X, n->I, n->G + n->oW1), columnSums(n->dYf, B, n->O, n->G + n->ob3),
+			columnSums(n->dH2f, B, n->H2, n->G + n->ob2), columnSums(n->dH1f, B, n->H1, n->G + n->ob1)});
 }
 
 extern "C" {
@@ -415,8 +533,7 @@ int cbm_mlp_create(unsigned nIn, unsigned h1, unsigned h2, unsigned nOut, unsign
 		delete n;
 		return mfail(CBM_ERR_CUDA, "stream");
 	}
-	if (cudaFuncSetAttribute(gemmKernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemmSmem<64>()) != cudaSuccess ||
-			cudaFuncSetAttribute(gemmKernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemmSmem<256>()) != cudaSuccess) {
+	if (cudaFuncSetAttribute(gemmKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem) != cudaSuccess) {
 		cudaStreamDestroy(n->s);
 		delete n;
 		return mfail(CBM_ERR_CUDA, "tensor-core product shared memory");
@@ -429,19 +546,13 @@ int cbm_mlp_create(unsigned nIn, unsigned h1, unsigned h2, unsigned nOut, unsign
 	n->P = dalloc<float>(n, n->nP); n->G = dalloc<float>(n, n->nP);
 	n->Mo = dalloc<float>(n, n->nP); n->Ve = dalloc<float>(n, n->nP);
 	n->Wh = dalloc<__nv_bfloat16>(n, n->nP);
-	n->W2t = dalloc<__nv_bfloat16>(n, (size_t)n->H1 * n->H2);
-	n->W3t = dalloc<__nv_bfloat16>(n, (size_t)n->H2 * n->O);
-	n->X = dalloc<__nv_bfloat16>(n, B * n->I); n->Xt = dalloc<__nv_bfloat16>(n, B * n->I);
-	n->Xf = dalloc<float>(n, B * n->I);
-	n->H1h = dalloc<__nv_bfloat16>(n, B * n->H1); n->H1t = dalloc<__nv_bfloat16>(n, B * n->H1);
-	n->H2h = dalloc<__nv_bfloat16>(n, B * n->H2); n->H2t = dalloc<__nv_bfloat16>(n, B * n->H2);
-	n->Yf = dalloc<float>(n, B * n->O); n->Tf = dalloc<float>(n, B * n->O);
-	n->dYf = dalloc<float>(n, B * n->O);
-	n->dYh = dalloc<__nv_bfloat16>(n, B * n->O); n->dYt = dalloc<__nv_bfloat16>(n, B * n->O);
-	n->dH2f = dalloc<float>(n, B * n->H2);
-	n->dH2h = dalloc<__nv_bfloat16>(n, B * n->H2); n->dH2t = dalloc<__nv_bfloat16>(n, B * n->H2);
-	n->dH1f = dalloc<float>(n, B * n->H1);
-	n->dH1h = dalloc<__nv_bfloat16>(n, B * n->H1); n->dH1t = dalloc<__nv_bfloat16>(n, B * n->H1);
+	n->X = dalloc<__nv_bfloat16>(n, B * n->I);
+	n->H1h = dalloc<__nv_bfloat16>(n, B * n->H1); n->H2h = dalloc<__nv_bfloat16>(n, B * n->H2);
+	n->Xf = dalloc<float>(n, B * n->nIn);
+	n->Yf = dalloc<float>(n, B * n->nOut); n->Tf = dalloc<float>(n, B * n->nOut);
+	n->dYf = dalloc<float>(n, B * n->O); n->dYh = dalloc<__nv_bfloat16>(n, B * n->O);
+	n->dH2f = dalloc<float>(n, B * n->H2); n->dH2h = dalloc<__nv_bfloat16>(n, B * n->H2);
+	n->dH1f = dalloc<float>(n, B * n->H1); n->dH1h = dalloc<__nv_bfloat16>(n, B * n->H1);
 	n->loss = dalloc<float>(n, 1);
 	n->err = dalloc<uint32_t>(n, 1);
 	for (void *p : n->allocs) if (!p) { cbm_mlp_destroy(n); return mfail(CBM_ERR_CUDA, "device allocation failed"); }
@@ -509,21 +620,12 @@ int cbm_mlp_forward(cbm_mlp *n, const float *x, unsigned batch, float *y)
 	cudaSetDevice(n->device);
 	for (unsigned b0 = 0; b0 < batch; b0 += n->maxBatch) {
 		const unsigned b = std::min(n->maxBatch, batch - b0);
-		MTRY(loadInput(n, x + (size_t)b0 * n->nIn, b));
-		MTRY(forward(n, b));
-		std::vector<float> out((size_t)b * n->O);
-		MCK(cudaMemcpyAsync(out.data(), n->Yf, out.size() * 4, cudaMemcpyDeviceToHost, n->s), "output");
+		MCK(cudaMemcpyAsync(n->Xf, x + (size_t)b0 * n->nIn, 4ull * b * n->nIn, cudaMemcpyHostToDevice, n->s), "input");
+		MTRY(prepare(n, n->Xf, b, b0 == 0, n->loss));
+		MTRY(forward(n, b, nullptr, nullptr));
+		MCK(cudaMemcpyAsync(y + (size_t)b0 * n->nOut, n->Yf, 4ull * b * n->nOut, cudaMemcpyDeviceToHost, n->s), "output");
 		MTRY(checkErr(n));
-		for (unsigned r = 0; r < b; r++) memcpy(y + (size_t)(b0 + r) * n->nOut, &out[(size_t)r * n->O], 4ull * n->nOut);
 	}
-	return CBM_OK;
-}
-
-static int loadTarget(cbm_mlp *n, const float *t, uint32_t b)
-{
-	std::vector<float> buf((size_t)b * n->O, 0.0f);
-	for (uint32_t r = 0; r < b; r++) memcpy(&buf[(size_t)r * n->O], t + (size_t)r * n->nOut, 4ull * n->nOut);
-	MCK(cudaMemcpyAsync(n->Tf, buf.data(), buf.size() * 4, cudaMemcpyHostToDevice, n->s), "target");
 	return CBM_OK;
 }
 
@@ -532,9 +634,10 @@ int cbm_mlp_gradients(cbm_mlp *n, const float *x, const float *target, unsigned 
 	if (!n || !x || !target || !grads) return mfail(CBM_ERR_ARG, "null argument");
 	if (batch == 0 || batch > n->maxBatch) return mfail(CBM_ERR_ARG, "batch must be 1..maxBatch");
 	cudaSetDevice(n->device);
-	MTRY(loadInput(n, x, batch));
-	MTRY(loadTarget(n, target, batch));
-	MTRY(forward(n, batch));
+	MCK(cudaMemcpyAsync(n->Xf, x, 4ull * batch * n->nIn, cudaMemcpyHostToDevice, n->s), "input");
+	MCK(cudaMemcpyAsync(n->Tf, target, 4ull * batch * n->nOut, cudaMemcpyHostToDevice, n->s), "target");
+	MTRY(prepare(n, n->Xf, batch, true, n->loss));
+	MTRY(forward(n, batch, n->Tf, n->loss));
 	MTRY(backward(n, batch));
 	MCK(cudaMemcpyAsync(grads, n->G, n->nP * 4, cudaMemcpyDeviceToHost, n->s), "gradients");
 	float l = 0;
@@ -565,16 +668,17 @@ int cbm_mlp_train(cbm_mlp *n, const float *x, const float *target, unsigned coun
 				memcpy(&xb[(size_t)r * n->nIn], x + (size_t)order[b0 + r] * n->nIn, 4ull * n->nIn);
 				memcpy(&tb[(size_t)r * n->nOut], target + (size_t)order[b0 + r] * n->nOut, 4ull * n->nOut);
 			}
-			MTRY(loadInput(n, xb.data(), batch));
-			MTRY(loadTarget(n, tb.data(), batch));
-			MTRY(forward(n, batch));
+			MCK(cudaMemcpyAsync(n->Xf, xb.data(), 4 * xb.size(), cudaMemcpyHostToDevice, n->s), "input");
+			MCK(cudaMemcpyAsync(n->Tf, tb.data(), 4 * tb.size(), cudaMemcpyHostToDevice, n->s), "target");
+			// Adam keeps the weights' copy from then on
+			MTRY(prepare(n, n->Xf, batch, e == 0 && b0 == 0, n->loss));
+			MTRY(forward(n, batch, n->Tf, n->loss));
 			MTRY(backward(n, batch));
 			n->adamStep++;
 			const float b1 = 0.9f, b2 = 0.999f;
 			const float c1 = 1.0f - (float)std::pow(b1, (double)n->adamStep), c2 = 1.0f - (float)std::pow(b2, (double)n->adamStep);
-			adamKernel<<<(unsigned)((n->nP + 255) / 256), 256, 0, n->s>>>(n->P, n->G, n->Mo, n->Ve, n->nP, lr, b1, b2,
-					1e-8f, c1, c2);
-			MCK(cudaGetLastError(), "Adam");
+			MTRY(launch(n, adamKernel, dim3((unsigned)((n->nP + kThreads - 1) / kThreads)), 0, "Adam", n->P,
+					(const float *)n->G, n->Mo, n->Ve, n->nP, lr, b1, b2, 1e-8f, c1, c2, n->Wh));
 			MCK(cudaMemcpyAsync(&l, n->loss, 4, cudaMemcpyDeviceToHost, n->s), "loss");
 			MTRY(checkErr(n));
 			epochLoss += l / ((double)batch * n->nOut);
