@@ -144,21 +144,31 @@ __device__ __forceinline__ void stageOperand(uint8_t *s, const __nv_bfloat16 *X,
 	}
 }
 
-// Column sums of columns [32 blockIdx.y, + 32): eight row groups, then a tree.
+// Column sums of columns [32 blockIdx.y, + 32), row after row: a sum's sign can
+// decide an Adam step, so the order stays that of one thread walking its column.
+// The rows come to shared memory 256 at a time, all their loads in flight (a
+// thread a column loading as it adds took 16 us over 256 rows).
 __device__ void colSums(const GemmJob &J, float *s)
 {
-	const int c = threadIdx.x % 32, g = threadIdx.x / 32, n = 32 * blockIdx.y + c;
+	const int tid = threadIdx.x, c4 = tid % 8, r0 = tid / 8, n0 = 32 * blockIdx.y;
 	float x = 0.0f;
-#pragma unroll 8
-	for (int r = g; r < J.M; r += kThreads / 32) x += J.colSum[(size_t)r * J.N + n];
-	s[threadIdx.x] = x;
-	__syncthreads();
-	if (g == 0) {
-		float y[8];
+	for (int m0 = 0; m0 < J.M; m0 += 256) {
+		const int rows = min(256, J.M - m0);
+		float4 v[8];
 #pragma unroll
-		for (int i = 0; i < 8; i++) y[i] = s[32 * i + c];
-		J.outF[n] = ((y[0] + y[4]) + (y[2] + y[6])) + ((y[1] + y[5]) + (y[3] + y[7]));
+		for (int u = 0; u < 8; u++)
+			if (r0 + 32 * u < rows)
+				v[u] = *reinterpret_cast<const float4 *>(J.colSum + (size_t)(m0 + r0 + 32 * u) * J.N + n0 + 4 * c4);
+#pragma unroll
+		for (int u = 0; u < 8; u++)
+			if (r0 + 32 * u < rows) *reinterpret_cast<float4 *>(s + 32 * (r0 + 32 * u) + 4 * c4) = v[u];
+		__syncthreads();
+		if (tid < 32)
+#pragma unroll 16
+			for (int r = 0; r < rows; r++) x += s[32 * r + tid];
+		__syncthreads();
 	}
+	if (tid < 32) J.outF[n0 + tid] = x;
 }
 
 // The products of these layers (at most 256 wide) are tiny: what bounds them is
