@@ -450,17 +450,11 @@ void cbm_sim_destroy(cbm_sim *sim);
  * weights[i] * ((apBuf[i] & pfDelayMask[i]) != 0) in the reference's
  * order (updatePFPCOutGPU then sumInputsNew) into sums[numPC], on `stream`
  * (a cudaStream_t, NULL for the default stream).
- * Scratch is one file-scope device array of CBM_NOALLOC_MAX_PARTIALS floats
- * that every device loading the library keeps until exit: numPC times the
- * reduction width (512 for rows of 2048 fibres or more) must fit in it, or
- * the call fails with CBM_ERR_ARG.  All calls on a device share the array;
- * each call rewrites the part it reads, so no clearing is needed, but calls
- * that overlap on the GPU race.  The first call on a device looks up the
- * array's address; make it before any stream capture.  The address is kept;
- * after a reset of the device's context it is looked up again, and the
- * first call after the reset must again precede any capture.  A CUDA error
- * already pending in the calling thread fails the call (CBM_ERR_CUDA) and is
- * left pending. */
+ * One launch, which may overlap others and, after the device's first call (which
+ * loads the code), be captured; nothing is kept between calls.  numPC times the reduction width (512 for rows of 2048 fibres
+ * or more) is at most CBM_NOALLOC_MAX_PARTIALS, or the call fails with
+ * CBM_ERR_ARG.  A CUDA error already pending in the calling thread fails the
+ * call (CBM_ERR_CUDA) and is left pending. */
 #define CBM_NOALLOC_MAX_PARTIALS 65536
 int cbm_pfpc_sums_noalloc(const uint32_t *apBuf, const uint32_t *pfDelayMask, const float *weights,
 		uint32_t numGR, uint32_t numPC, float *sums, void *stream);
