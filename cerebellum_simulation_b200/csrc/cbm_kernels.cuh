@@ -108,10 +108,11 @@ const void *pcTreeKernelFn();
 __global__ void tailKernel(const DevNet *const *nets, const uint32_t *stageBytes, uint32_t stepOffset,
 		const DevNet *net0, uint32_t stage0, uint8_t *ncMailbox, const __grid_constant__ MFParam mfp);
 __global__ void protocolPrimeKernel(const DevNet *N);
-// GR peri-stimulus histogram of step t = stepsDone(N) + 1 + stepOffset, after
-// the GR pass of that step: 8 GR per thread.
-__global__ void grPSHKernel(const DevNet *N, uint32_t stepOffset);
-__global__ void trialDataKernel(const DevNet *N, uint32_t stepOffset);
+// The records of step t = stepsDone(N) + 1 + stepOffset, after both kernels of
+// that step: ECTrialsData on the first trialBlocks blocks, a cell a thread, then
+// the GR peri-stimulus histogram, 8 GR a thread.  May be launched as the
+// programmatic dependent of the step's GR pass.
+__global__ void recordKernel(const DevNet *N, uint32_t stepOffset, uint32_t trialBlocks);
 // All networks of a batch: cellOffset[n] is the first grid thread of network
 // n's small cells (cellOffset[numNets] the total).
 __global__ void trialDataBatchKernel(const DevNet *const *nets, const uint32_t *cellOffset, int numNets,

@@ -1778,7 +1778,7 @@ std::string Simulator::enqueueStep(uint32_t k, bool instrument, bool chained)
 		CK(cudaEventRecordWithFlags(tailEv_[2 * k + 1], s1_, cudaEventRecordExternal), "tail timing");
 		CK(cudaEventRecord(join_, s1_), "join");
 		CK(cudaStreamWaitEvent(s0_, join_, 0), "join");
-		return recordStep(k);
+		return recordStep(k, false);
 	}
 	if (chained) {
 		// with the per-tile pass: the small-cell kernel is the
@@ -1799,7 +1799,7 @@ std::string Simulator::enqueueStep(uint32_t k, bool instrument, bool chained)
 		CK(cudaLaunchKernelEx(&cfg, tailKernel, netsArg, stageArg, k, net0Arg, stage0Arg, mailboxArg_, stepMF_),
 				"launching the small-cell update");
 		CKS(launchPass(s0_, true));
-		return recordStep(k);
+		return recordStep(k, true);
 	}
 	// One stream: the small-cell CTAs launch first and let the GR pass start
 	// as soon as they are resident (programmatic dependent launch; the two
@@ -1811,10 +1811,10 @@ std::string Simulator::enqueueStep(uint32_t k, bool instrument, bool chained)
 	CK(cudaEventRecord(join_, s0_), "join");
 	CKS(launchPass(s0_, true));
 	CK(cudaStreamWaitEvent(s0_, join_, 0), "join");
-	return recordStep(k);
+	return recordStep(k, false);
 }
 
-std::string Simulator::recordStep(uint32_t k)
+std::string Simulator::recordStep(uint32_t k, bool chained)
 {
 	// after both kernels of the step: its GR spikes into the histogram, and
 	// its small-cell state into the trial data
@@ -1826,15 +1826,20 @@ std::string Simulator::recordStep(uint32_t k)
 		return "";
 	}
 	const DevNet &h = nets_[0]->dev();
-	if (nets_[0]->recordsGR()) {
-		const uint32_t threads = (h.numGR + 7) / 8;
-		grPSHKernel<<<(threads + 255) / 256, 256, 0, s0_>>>(nets_[0]->devPtr(), k);
-		CK(cudaGetLastError(), "launching the GR histogram");
-	}
-	if (nets_[0]->recordsTrialData()) {
-		const uint32_t cells = h.numGO + h.numMF + h.numSC + h.numBC + h.numPC + h.numIO + h.numNC;
-		trialDataKernel<<<(cells + 255) / 256, 256, 0, s0_>>>(nets_[0]->devPtr(), k);
-		CK(cudaGetLastError(), "launching the trial-data record");
+	const uint32_t cells = h.numGO + h.numMF + h.numSC + h.numBC + h.numPC + h.numIO + h.numNC;
+	const uint32_t trialBlocks = nets_[0]->recordsTrialData() ? (cells + 255) / 256 : 0;
+	const uint32_t grBlocks = nets_[0]->recordsGR() ? ((h.numGR + 7) / 8 + 255) / 256 : 0;
+	if (trialBlocks + grBlocks) {
+		cudaLaunchConfig_t cfg = {};
+		cfg.gridDim = dim3(trialBlocks + grBlocks);
+		cfg.blockDim = dim3(256);
+		cfg.stream = s0_;
+		cudaLaunchAttribute attr;
+		attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+		attr.val.programmaticStreamSerializationAllowed = 1;
+		cfg.attrs = &attr;
+		cfg.numAttrs = chained ? 1 : 0;
+		CK(cudaLaunchKernelEx(&cfg, recordKernel, nets_[0]->devPtr(), k, trialBlocks), "launching the step's records");
 	}
 	return "";
 }

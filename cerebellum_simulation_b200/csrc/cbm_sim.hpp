@@ -124,7 +124,7 @@ private:
 	// chained: launched one at a time, the small-cell kernel as the
 	// programmatic dependent of the previous step (see launchSteps)
 	std::string enqueueStep(uint32_t stepOffset, bool instrument, bool chained = false);
-	std::string recordStep(uint32_t stepOffset);
+	std::string recordStep(uint32_t stepOffset, bool chained);
 	void dropGraphs();
 	void markInputSlotsFree();  // after a full synchronisation
 	// Issue the copy of MF input that a single-step graph would have carried.
