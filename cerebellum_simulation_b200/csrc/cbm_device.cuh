@@ -84,7 +84,7 @@ struct StageSeg {
 	uint32_t writeBack;  // copied back to global memory after the step
 };
 
-// Shared-memory layout of one pipeline stage of the GR pass (R rows of 32
+// Shared-memory layout of one pipeline stage of the persistent GR pass (R rows of 32
 // cells); every region starts on a 128-byte boundary.
 struct PassLayout {
 	uint32_t mfIdx, goIdx, outCon, pfDelay, w, hist;  // region offsets (the six state arrays start at 0)
@@ -95,9 +95,7 @@ struct PassLayout {
 
 CBM_LAYOUT_FN uint32_t align128(uint32_t x) { return (x + 127u) & ~127u; }
 
-// outBytes: 4 for the 32-bit GR->GO slot table, 2 for the 16-bit one.
-CBM_LAYOUT_FN PassLayout passLayout(uint32_t R, uint32_t nMF, uint32_t nGO, uint32_t nOut, uint32_t Z,
-		uint32_t outBytes = 4)
+CBM_LAYOUT_FN PassLayout passLayout(uint32_t R, uint32_t nMF, uint32_t nGO, uint32_t nOut, uint32_t Z)
 {
 	const uint32_t mfS = nMF ? nMF : 1, goS = nGO ? nGO : 1, outS = nOut ? nOut : 1;
 	const uint32_t row4 = 128u * R;  // one 4-byte array: R rows x 32 cells
@@ -105,12 +103,12 @@ CBM_LAYOUT_FN PassLayout passLayout(uint32_t R, uint32_t nMF, uint32_t nGO, uint
 	uint32_t o = 6 * row4;
 	L.mfIdx = o; o = align128(o + 64u * R * mfS);
 	L.goIdx = o; o = align128(o + 64u * R * goS);
-	L.outCon = o; o = align128(o + 32u * outBytes * R * outS);
+	L.outCon = o; o = align128(o + 128u * R * outS);
 	L.pfDelay = o; o = align128(o + 32u * R);
 	L.w = o; o = align128(o + row4 * Z);
 	L.hist = o; o = align128(o + 256u * R);
 	L.bytes = o;
-	L.txBase = 6 * row4 + 64u * R * mfS + 64u * R * goS + 32u * outBytes * R * outS + 32u * R + row4 * Z;
+	L.txBase = 6 * row4 + 64u * R * mfS + 64u * R * goS + 128u * R * outS + 32u * R + row4 * Z;
 	L.txHist = 256u * R;
 	return L;
 }
