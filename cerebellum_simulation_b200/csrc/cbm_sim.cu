@@ -26,13 +26,20 @@ std::string cudaErr(cudaError_t e, const char *what)
 #define CKS(expr) do { std::string s_ = (expr); if (!s_.empty()) return s_; } while (0)
 
 // ------------------------------------------------------------------ Network
-template <typename T> T *Network::alloc(size_t n)
+// Device arrays are filled on the simulator's step stream, the one that every
+// kernel and copy using them is ordered by.  (A cudaMemset or cudaMemcpy would run
+// on the default stream, which a non-blocking stream does not wait for: behind
+// another library's work there, it could land after the kernels' own writes.)
+template <typename T> T *Network::alloc(size_t n, bool zero)
 {
 	void *p = nullptr;
 	// whole 16-byte units, so that arrays can be copied with 16-byte accesses
 	size_t bytes = (std::max<size_t>(n * sizeof(T), 16) + 15) & ~(size_t)15;
-	if (cudaMalloc(&p, bytes) != cudaSuccess) return nullptr;
-	if (cudaMemset(p, 0, bytes) != cudaSuccess) { cudaFree(p); return nullptr; }
+	if (cudaMalloc(&p, bytes) != cudaSuccess) {
+		cudaGetLastError();  // reported here, not by the next launch's check
+		return nullptr;
+	}
+	if (zero && cudaMemsetAsync(p, 0, bytes, stream_) != cudaSuccess) { cudaFree(p); return nullptr; }
 	allocs_.push_back(p);
 	allocBytes_[p] = bytes;
 	return (T *)p;
@@ -40,8 +47,12 @@ template <typename T> T *Network::alloc(size_t n)
 
 template <typename T> T *Network::upload(const T *src, size_t n)
 {
-	T *d = alloc<T>(n);
-	if (d && n) cudaMemcpy(d, src, n * sizeof(T), cudaMemcpyHostToDevice);
+	// the bytes that pad the array are zeroed too
+	T *d = alloc<T>(n, n * sizeof(T) % 16 != 0 || n == 0);
+	if (d && n && cudaMemcpyAsync(d, src, n * sizeof(T), cudaMemcpyHostToDevice, stream_) != cudaSuccess) {
+		release(d);
+		return nullptr;
+	}
 	return d;
 }
 
@@ -176,7 +187,8 @@ std::string Network::buildPassMaps(uint32_t R)
 	for (uint32_t z = 0; z < h_.numZones; z++) CKS(enc2(PM_W0 + z, h_.zones[z].w, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4));
 	CUtensorMap *d = alloc<CUtensorMap>(PM_COUNT);
 	if (!d) return "device allocation failed";
-	CK(cudaMemcpy(d, maps.data(), PM_COUNT * sizeof(CUtensorMap), cudaMemcpyHostToDevice), "uploading TMA descriptors");
+	CK(cudaMemcpyAsync(d, maps.data(), PM_COUNT * sizeof(CUtensorMap), cudaMemcpyHostToDevice, stream_),
+			"uploading TMA descriptors");
 	h_.passMaps = d;
 	return uploadDesc();
 }
@@ -214,7 +226,7 @@ std::string Network::buildEventPass(uint32_t target, uint32_t SC, cudaStream_t s
 	uint64_t total = 0;
 	for (uint32_t &x : hb) { const uint32_t n = x; x = (uint32_t)total; total += n; }
 	if (total > 0x1FFFFFFFull) return "too many GR synapses for the event tables";
-	uint16_t *entry = alloc<uint16_t>(8 * total);
+	uint16_t *entry = alloc<uint16_t>(8 * total, false);
 	if (!entry) return "device allocation failed";
 	evUnusedKernel<<<1184, 256, 0, s>>>((uint32_t *)entry, 4 * total, kEvUnused | (kEvUnused << 16));
 	CK(cudaMemcpyAsync(base, hb.data(), 4ull * blocks, cudaMemcpyHostToDevice, s), "event tables");
@@ -227,15 +239,15 @@ std::string Network::buildEventPass(uint32_t target, uint32_t SC, cudaStream_t s
 	};
 	h_.evPerMF = items(h_.nMFSlots, h_.numMF);
 	h_.evPerGO = items(h_.nGOSlots, h_.numGO);
-	uint4 *oc = alloc<uint4>(N);
-	uint8_t *pd = alloc<uint8_t>(N);
+	uint4 *oc = alloc<uint4>(N, false);
+	uint8_t *pd = alloc<uint8_t>(N, false);
 	uint32_t *rows = alloc<uint32_t>(2), nRows = 0;  // zeroed
 	if (!oc || !pd || !rows) return "device allocation failed";
 	evOutKernel<<<grid, 256, 0, s>>>(devPtr(), nullptr, nullptr, rows);
 	CK(cudaMemcpyAsync(&nRows, rows, 4, cudaMemcpyDeviceToHost, s), "event tables");
 	CK(cudaStreamSynchronize(s), "event tables");
 	if (nRows > 0xFFFFFFu) return "too many GR->GO synapses for the event tables";
-	uint4 *om = alloc<uint4>(std::max(1u, nRows));
+	uint4 *om = alloc<uint4>(std::max(1u, nRows), false);
 	if (!om) return "device allocation failed";
 	evOutKernel<<<grid, 256, 0, s>>>(devPtr(), oc, om, rows + 1);
 	evOrderKernel<<<grid, 256, 0, s>>>(devPtr(), h_.pfDelay, pd, 1, 1, true);
@@ -256,7 +268,7 @@ std::string Network::buildEventPass(uint32_t target, uint32_t SC, cudaStream_t s
 // exports, one at a time in the stream's order).
 std::string Network::scratch(void **p)
 {
-	if (!scratch_) scratch_ = alloc<uint64_t>(h_.numGR);
+	if (!scratch_) scratch_ = alloc<uint64_t>(h_.numGR, false);
 	if (!scratch_) return "device allocation failed";
 	*p = scratch_;
 	return "";
@@ -315,7 +327,7 @@ std::string Network::setEventMode(bool on, cudaStream_t s)
 
 std::string Network::uploadDesc()
 {
-	CK(cudaMemcpy(dNet_.ptr, &h_, sizeof(DevNet), cudaMemcpyHostToDevice), "uploading the network descriptor");
+	CK(cudaMemcpyAsync(dNet_.ptr, &h_, sizeof(DevNet), cudaMemcpyHostToDevice, stream_), "uploading the network descriptor");
 	return "";
 }
 
@@ -413,21 +425,24 @@ std::string Network::buildZoneStaging()
 	CK(cudaMalloc((void **)&blk, block), "allocating the staging block");
 	zoneBlock_ = blk;
 	dNet_.ptr = blk;  // the descriptor heads the block (freed with it)
-	CK(cudaMemset(blk, 0, block), "clearing the staging block");
+	CK(cudaMemsetAsync(blk, 0, block, stream_), "clearing the staging block");
+	std::vector<void *> moved;
 	for (const StageSeg &sg : segs) {
 		void **field = (void **)((char *)&h_ + sg.fieldOff);
 		uint8_t *dst = blk + kStageArenaOff + sg.smemOff;
-		CK(cudaMemcpy(dst, *field, sg.bytes, cudaMemcpyDeviceToDevice), "filling the staging block");
-		release(*field);
+		CK(cudaMemcpyAsync(dst, *field, sg.bytes, cudaMemcpyDeviceToDevice, stream_), "filling the staging block");
+		moved.push_back(*field);
 		*field = dst;
 	}
 	// the step counter lives in the block, so that the copy brings it along
 	uint64_t *tb = (uint64_t *)(blk + kStageNetBytes);
-	CK(cudaMemcpy(tb, h_.tBase, sizeof(uint64_t), cudaMemcpyDeviceToDevice), "moving the step counter");
-	release(h_.tBase);
+	CK(cudaMemcpyAsync(tb, h_.tBase, sizeof(uint64_t), cudaMemcpyDeviceToDevice, stream_), "moving the step counter");
+	moved.push_back(h_.tBase);
 	h_.tBase = tb;
 	StageSeg *dSegs = (StageSeg *)(blk + kStageArenaOff + arena);
-	CK(cudaMemcpy(dSegs, segs.data(), segs.size() * sizeof(StageSeg), cudaMemcpyHostToDevice), "staging table");
+	CK(cudaMemcpyAsync(dSegs, segs.data(), segs.size() * sizeof(StageSeg), cudaMemcpyHostToDevice, stream_), "staging table");
+	CK(cudaStreamSynchronize(stream_), "filling the staging block");
+	for (void *p : moved) release(p);
 	h_.zoneSegs = dSegs;
 	h_.numZoneSegs = (uint32_t)segs.size();
 	h_.zoneArenaBytes = arena;
@@ -561,10 +576,11 @@ std::string checkNetwork(const State &st)
 	return "";
 }
 
-std::string Network::build(State *st, const std::vector<int> &seeds, uint32_t mfRing, uint32_t mfSeed)
+std::string Network::build(State *st, const std::vector<int> &seeds, uint32_t mfRing, uint32_t mfSeed, cudaStream_t s)
 {
 	(void)mfSeed;
 	st_ = st;
+	stream_ = s;
 	const ConParams &c = st->cp;
 	const ActParams &a = st->ap;
 	// checkNetwork(*st) has passed: every count and index below is in range
@@ -812,7 +828,8 @@ std::string Network::build(State *st, const std::vector<int> &seeds, uint32_t mf
 				sel[c.numIO + i] = tm[i] < h.tsLTDEndIO ? 1 : (tm[i] > h.tsLTPStartAPIO ? 2 : 0);
 		}
 		if (!Q.plastSel) return "device allocation failed";
-		CK(cudaMemcpy(Q.plastSel, sel.data(), sel.size(), cudaMemcpyHostToDevice), "uploading the plasticity selector");
+		CK(cudaMemcpyAsync(Q.plastSel, sel.data(), sel.size(), cudaMemcpyHostToDevice, stream_),
+				"uploading the plasticity selector");
 		ctl.ltdStep[z] = a.synLTDStepSizeGRtoPC;
 		ctl.ltpStep[z] = a.synLTPStepSizeGRtoPC;
 		ctl.errDrive[z] = zs.errDrive;
@@ -859,15 +876,16 @@ std::string Network::build(State *st, const std::vector<int> &seeds, uint32_t mf
 		dNet_.ptr = zoneBlock_;
 	} else {
 		CK(cudaMalloc(&dNet_.ptr, kStageArenaOff), "allocating the network descriptor");
-		CK(cudaMemset(dNet_.ptr, 0, kStageArenaOff), "clearing the network descriptor");
+		CK(cudaMemsetAsync(dNet_.ptr, 0, kStageArenaOff, stream_), "clearing the network descriptor");
 		uint64_t *tb = (uint64_t *)((char *)dNet_.ptr + kStageNetBytes);
-		CK(cudaMemcpy(tb, h.tBase, sizeof(uint64_t), cudaMemcpyDeviceToDevice), "moving the step counter");
+		CK(cudaMemcpyAsync(tb, h.tBase, sizeof(uint64_t), cudaMemcpyDeviceToDevice, stream_), "moving the step counter");
+		CK(cudaStreamSynchronize(stream_), "moving the step counter");
 		release(h.tBase);
 		h.tBase = tb;
 	}
 	dNet_.bytes = sizeof(DevNet);
-	CK(cudaMemcpy(dNet_.ptr, &h, sizeof(DevNet), cudaMemcpyHostToDevice), "uploading the network descriptor");
-	CK(cudaDeviceSynchronize(), "network build");
+	CKS(uploadDesc());
+	CK(cudaStreamSynchronize(stream_), "network build");
 	hostT_ = 0;
 	return "";
 }
@@ -1392,7 +1410,7 @@ std::string Simulator::create(const std::vector<State *> &states, const std::vec
 		Network *n = new Network();
 		nets_.push_back(n);
 		std::vector<int> sd = i < seeds.size() ? seeds[i] : std::vector<int>();
-		CKS(n->build(states[i], sd, mfRing, mfSeeds && i < mfSeeds->size() ? (*mfSeeds)[i] : 0));
+		CKS(n->build(states[i], sd, mfRing, mfSeeds && i < mfSeeds->size() ? (*mfSeeds)[i] : 0, s0_));
 		offs.push_back(passBlocks_);
 		passBlocks_ += n->passBlocks();
 		ptrs.push_back(n->devPtr());
@@ -1404,7 +1422,7 @@ std::string Simulator::create(const std::vector<State *> &states, const std::vec
 	auto up = [&](DeviceBuf &b, const void *src, size_t bytes) -> std::string {
 		CK(cudaMalloc(&b.ptr, bytes), "allocating launch tables");
 		b.bytes = bytes;
-		CK(cudaMemcpy(b.ptr, src, bytes, cudaMemcpyHostToDevice), "uploading launch tables");
+		CK(cudaMemcpyAsync(b.ptr, src, bytes, cudaMemcpyHostToDevice, s0_), "uploading launch tables");
 		return "";
 	};
 	CKS(up(dNetPtrs_, ptrs.data(), ptrs.size() * sizeof(DevNet *)));
@@ -1542,7 +1560,7 @@ std::string Simulator::usePassGeometry(const PassGeometry &g)
 			auto up = [&](DeviceBuf &b, const std::vector<uint32_t> &v) -> std::string {
 				CK(cudaMalloc(&b.ptr, v.size() * sizeof(uint32_t)), "allocating vector-pass tables");
 				b.bytes = v.size() * sizeof(uint32_t);
-				CK(cudaMemcpy(b.ptr, v.data(), b.bytes, cudaMemcpyHostToDevice), "uploading vector-pass tables");
+				CK(cudaMemcpyAsync(b.ptr, v.data(), b.bytes, cudaMemcpyHostToDevice, s0_), "uploading vector-pass tables");
 				return "";
 			};
 			CKS(up(dVecUnitOffset_, units));
@@ -1557,7 +1575,7 @@ std::string Simulator::usePassGeometry(const PassGeometry &g)
 		const uint32_t claims = (units + kVecBatchClaim - 1) / kVecBatchClaim;
 		passGrid_ = std::max<uint32_t>(1, std::min<uint32_t>((claims + kVecWarps - 1) / kVecWarps,
 				(uint32_t)std::max(1, perSM) * (uint32_t)numSMs));
-		CK(cudaMemset(dVecClaim_.ptr, 0, dVecClaim_.bytes), "pass claim counters");
+		CK(cudaMemsetAsync(dVecClaim_.ptr, 0, dVecClaim_.bytes, s0_), "pass claim counters");
 		for (Network *n : nets_) CKS(n->setPcSumMode(true, s0_));
 		CKS(arriveMode());
 		passTmaFn_ = fn;
@@ -1595,7 +1613,7 @@ std::string Simulator::usePassGeometry(const PassGeometry &g)
 		passGrid_ = std::max<uint32_t>(1, std::min<uint32_t>((claims + kVecWarps - 1) / kVecWarps,
 				(uint32_t)std::max(1, perSM) * sms)) + passVecReduceCTAs(n.dev());
 		// claim counters from zero (another pass kind may have run meanwhile)
-		CK(cudaMemset(n.dev().passClaim, 0, 4 * sizeof(uint32_t)), "pass claim counters");
+		CK(cudaMemsetAsync(n.dev().passClaim, 0, 4 * sizeof(uint32_t), s0_), "pass claim counters");
 		CKS(n.setPcSumMode(true, s0_));
 		CKS(arriveMode());
 		passTmaFn_ = fn;
@@ -1656,7 +1674,8 @@ std::string Simulator::usePassGeometry(const PassGeometry &g)
 		if (!blocks.empty()) {
 			CK(cudaMalloc(&dPassBlocks_.ptr, blocks.size() * sizeof(PassBlock)), "allocating launch tables");
 			dPassBlocks_.bytes = blocks.size() * sizeof(PassBlock);
-			CK(cudaMemcpy(dPassBlocks_.ptr, blocks.data(), dPassBlocks_.bytes, cudaMemcpyHostToDevice), "uploading launch tables");
+			CK(cudaMemcpyAsync(dPassBlocks_.ptr, blocks.data(), dPassBlocks_.bytes, cudaMemcpyHostToDevice, s0_),
+					"uploading launch tables");
 		}
 	} else {
 		if (nets_.size() != 1) return "the persistent GR pass runs one network";
@@ -1976,7 +1995,7 @@ std::string Simulator::recordTrialData(size_t i)
 		}
 		CK(cudaMalloc(&dCellOffset_.ptr, off.size() * sizeof(uint32_t)), "cell offsets");
 		dCellOffset_.bytes = off.size() * sizeof(uint32_t);
-		CK(cudaMemcpy(dCellOffset_.ptr, off.data(), dCellOffset_.bytes, cudaMemcpyHostToDevice), "cell offsets");
+		CK(cudaMemcpyAsync(dCellOffset_.ptr, off.data(), dCellOffset_.bytes, cudaMemcpyHostToDevice, s0_), "cell offsets");
 		cellTotal_ = off.back();
 	}
 	if (!was) dropGraphs();  // the step graphs gain the trial-data kernel

@@ -185,7 +185,8 @@ private:
 class Network {
 public:
 	~Network();
-	std::string build(State *st, const std::vector<int> &seeds, uint32_t mfRing, uint32_t mfSeed);
+	// s: the simulator's step stream, which orders all work on the network
+	std::string build(State *st, const std::vector<int> &seeds, uint32_t mfRing, uint32_t mfSeed, cudaStream_t s);
 	// host setters of the reference's API
 	void setPlastSteps(uint32_t zone, float ltd, float ltp);
 	void resetPlastSteps(uint32_t zone);
@@ -270,9 +271,10 @@ public:
 
 private:
 	friend class Simulator;
-	template <typename T> T *alloc(size_t n);
+	template <typename T> T *alloc(size_t n, bool zero = true);
 	template <typename T> T *upload(const T *src, size_t n);
 	State *st_ = nullptr;
+	cudaStream_t stream_ = nullptr;
 	DevNet h_{};
 	DeviceBuf dNet_;
 	std::string buildZoneStaging();
