@@ -77,6 +77,9 @@ __global__ void __launch_bounds__(kThreads) pfpcSumsKernel(const uint32_t *apBuf
 	__shared__ __align__(16) float sTerm[kThreads * V];
 	__shared__ float sPart[512];  // the PC's partials (in the cluster's first CTA)
 	cg::cluster_group cluster = cg::this_cluster();
+	// a CTA's shared memory may be written from another one once it has started:
+	// every CTA says so here, and the others wait for that behind their loads
+	cluster.barrier_arrive();
 	const uint32_t part = cluster.block_rank(), pc = blockIdx.x / cluster.num_blocks();
 	const uint32_t tid = threadIdx.x, lanes = cols / V, rows = blockDim.x / lanes;
 	const uint32_t j = part * cols + tid % lanes * V, r = tid / lanes, K = P / (2 * bs);
@@ -103,6 +106,7 @@ __global__ void __launch_bounds__(kThreads) pfpcSumsKernel(const uint32_t *apBuf
 		__syncthreads();
 	}
 	// the partials to the cluster's first CTA
+	cluster.barrier_wait();
 	if (tid < cols) cluster.map_shared_rank(sPart, 0)[part * cols + tid] = s;
 	cluster.sync();
 	if (part || tid >= 32) return;
