@@ -584,7 +584,9 @@ int cbm_mlp_create(unsigned nIn, unsigned h1, unsigned h2, unsigned nOut, unsign
 		return o;
 	};
 	const size_t bytes = layout(nullptr);
-	if (cudaMalloc(&n->arena, bytes) != cudaSuccess || cudaMemset(n->arena, 0, bytes) != cudaSuccess) {
+	// on the handle's stream, like everything after it (the default stream would not
+	// be waited for)
+	if (cudaMalloc(&n->arena, bytes) != cudaSuccess || cudaMemsetAsync(n->arena, 0, bytes, n->s) != cudaSuccess) {
 		cbm_mlp_destroy(n);
 		return mfail(CBM_ERR_CUDA, "device allocation failed");
 	}
@@ -601,7 +603,8 @@ int cbm_mlp_create(unsigned nIn, unsigned h1, unsigned h2, unsigned nOut, unsign
 	init(n->oW1, h1, nIn, n->I, nIn);
 	init(n->oW2, h2, h1, n->H1, h1);
 	init(n->oW3, nOut, h2, n->H2, h2);
-	if (cudaMemcpy(n->P, p.data(), p.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess) {
+	if (cudaMemcpyAsync(n->P, p.data(), p.size() * 4, cudaMemcpyHostToDevice, n->s) != cudaSuccess ||
+			cudaStreamSynchronize(n->s) != cudaSuccess) {
 		cbm_mlp_destroy(n);
 		return mfail(CBM_ERR_CUDA, "uploading parameters");
 	}
@@ -635,7 +638,8 @@ int cbm_mlp_get_params(cbm_mlp *n, float *dst, uint64_t count)
 	if (!n || !dst) return mfail(CBM_ERR_ARG, "null argument");
 	if (count != n->nP) return mfail(CBM_ERR_ARG, "parameter count mismatch");
 	cudaSetDevice(n->device);
-	MCK(cudaMemcpy(dst, n->P, count * 4, cudaMemcpyDeviceToHost), "reading parameters");
+	MCK(cudaMemcpyAsync(dst, n->P, count * 4, cudaMemcpyDeviceToHost, n->s), "reading parameters");
+	MCK(cudaStreamSynchronize(n->s), "reading parameters");
 	return CBM_OK;
 }
 
@@ -644,9 +648,10 @@ int cbm_mlp_set_params(cbm_mlp *n, const float *src, uint64_t count)
 	if (!n || !src) return mfail(CBM_ERR_ARG, "null argument");
 	if (count != n->nP) return mfail(CBM_ERR_ARG, "parameter count mismatch");
 	cudaSetDevice(n->device);
-	MCK(cudaMemcpy(n->P, src, count * 4, cudaMemcpyHostToDevice), "writing parameters");
-	MCK(cudaMemset(n->Mo, 0, count * 4), "resetting Adam");
-	MCK(cudaMemset(n->Ve, 0, count * 4), "resetting Adam");
+	MCK(cudaMemcpyAsync(n->P, src, count * 4, cudaMemcpyHostToDevice, n->s), "writing parameters");
+	MCK(cudaMemsetAsync(n->Mo, 0, count * 4, n->s), "resetting Adam");
+	MCK(cudaMemsetAsync(n->Ve, 0, count * 4, n->s), "resetting Adam");
+	MCK(cudaStreamSynchronize(n->s), "writing parameters");  // src is the caller's again
 	n->adamStep = 0;
 	return CBM_OK;
 }

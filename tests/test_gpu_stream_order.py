@@ -72,3 +72,24 @@ def test_simulator_beside_default_stream_work(tmp_path):
         with busy_default_stream():
             got = run()
         assert [a == b for a, b in zip(got, want)] == [True] * len(want), k
+
+
+def test_surrogate_beside_default_stream_work():
+    """Parameters set, then trained on at once: Adam starts from zero moments."""
+    from cerebellum_simulation_b200.surrogate import MLP
+    rng = np.random.Generator(np.random.PCG64(8))
+    x = rng.uniform(-1, 1, (512, 24)).astype(np.float32)
+    t = rng.uniform(0, 2, (512, 10)).astype(np.float32)
+
+    def run(busy):
+        net = MLP(24, 96, 64, 10, max_batch=128, seed=2)
+        start = net.get_params()
+        net.train(x, t, batch=128, epochs=2, lr=1e-2, seed=1)  # leaves moments behind
+        with busy_default_stream() if busy else contextlib.nullcontext():
+            net.set_params(start)
+            net.train(x, t, batch=128, epochs=2, lr=1e-2, seed=1)
+            return net.get_params().tobytes()
+
+    want = run(False)
+    for _ in range(3):
+        assert run(True) == want
