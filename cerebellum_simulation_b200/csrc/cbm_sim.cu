@@ -10,6 +10,8 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <type_traits>
+#include <utility>
 
 #include "cbm_kernels.cuh"
 #include "cbm_rng.hpp"
@@ -193,75 +195,132 @@ std::string Network::buildPassMaps(uint32_t R)
 	return uploadDesc();
 }
 
-std::string Network::buildEventPass(uint32_t target, uint32_t SC, cudaStream_t s)
+// The per-tile pass's tables in the tiling for `target` and SC, on the device from
+// the slot tables, beside those in use (which may serve: o->fresh says); nothing
+// that the pass in use reads is touched.
+std::string Network::planEventPass(uint32_t target, uint32_t SC, EventTables *o, cudaStream_t s)
 {
-	// a new tiling drops the spikes the last step left for the next: the ring
-	// is refilled from the spike buffers (setEventMode) whenever it is entered
-	CKS(setEventMode(false, s));
-	const uint32_t rows0 = h_.evRows, wd0 = h_.evWdShift;
-	if (!eventTiling(target, SC, &h_)) return "no tiling of the per-tile GR pass covers the cells";
-	if (!h_.evCnt) {
-		h_.evCnt = alloc<uint8_t>(2ull * h_.numGR);
-		if (!h_.evCnt) return "device allocation failed";
-	}
-	const uint32_t N = h_.numGR, nSrc = h_.numMF + h_.numGO;
-	if (h_.evStart && h_.evRows == rows0 && h_.evWdShift == wd0) return uploadDesc();
-
-	// event tables in the tiling's order, built on the device from the slot tables
-	for (void *q : {(void *)h_.evStart, (void *)h_.evEntry, (void *)h_.outCell, (void *)h_.outMore, (void *)h_.evPfDelay,
-			(void *)h_.spkBits})
-		if (q) release(q);
-	h_.evStart = nullptr; h_.evEntry = nullptr; h_.outCell = h_.outMore = nullptr; h_.evPfDelay = nullptr; h_.spkBits = nullptr;
-	const uint32_t blocks = eventBlocks(), grid = (N + 255) / 256;
+	o->net = h_;
+	DevNet &d = o->net;
+	if (!eventTiling(target, SC, &d)) return "no tiling of the per-tile GR pass covers the cells";
+	void *tmp = nullptr;
+	if (d.evTilesX > 1) CKS(scratch(&tmp));  // taking the tables reorders the arrays through it
+	o->fresh = !h_.evStart || h_.evRows != d.evRows || h_.evWdShift != d.evWdShift;
+	if (!o->fresh) return "";
+	const uint32_t N = h_.numGR, nSrc = h_.numMF + h_.numGO, blocks = eventBlocks(), grid = (N + 255) / 256;
 	const size_t nStart = (size_t)blocks * (nSrc + 1);
-	h_.spkBits = alloc<uint32_t>(2ull * (N / 32));
-	uint32_t *start = alloc<uint32_t>(nStart), *next = alloc<uint32_t>(nStart), *base = alloc<uint32_t>(blocks);
-	if (!h_.spkBits || !start || !next || !base) return "device allocation failed";
-	CKS(uploadDesc());
-	evCountKernel<<<grid, 256, 0, s>>>(devPtr(), start);
+	// one allocation for what is sized now, one for the lists, one that goes again
+	uint8_t *base = nullptr;
+	size_t bytes = 0;
+	auto take = [&](auto *&p, size_t count) {
+		p = base ? (std::remove_reference_t<decltype(p)>)(base + bytes) : nullptr;
+		bytes += (count * sizeof(*p) + 255) & ~(size_t)255;
+	};
+	uint32_t *start, *next, *blockBase, *rows;
+	uint4 *oc, *om;
+	uint16_t *entry;
+	uint8_t *pd;
+	DevNet *desc;
+	auto tables = [&]() {
+		bytes = 0;
+		take(start, nStart);
+		take(oc, N);
+		take(pd, N);
+		take(d.spkBits, 2ull * (N / 32));
+		take(d.evCnt, 2ull * N);
+	};
+	auto building = [&]() {
+		bytes = 0;
+		take(desc, 1);
+		take(next, nStart);
+		take(blockBase, blocks);
+		take(rows, 2);  // rows of outMore, and how many are filled
+	};
+	building();
+	o->building = base = alloc<uint8_t>(bytes, false);
+	if (!base) return "device allocation failed";
+	building();
+	base = nullptr;
+	tables();
+	o->arena[0] = base = alloc<uint8_t>(bytes, false);
+	if (!base) return "device allocation failed";
+	tables();
+	CK(cudaMemcpyAsync(desc, &d, sizeof(DevNet), cudaMemcpyHostToDevice, s), "event tables");
+	CK(cudaMemsetAsync(start, 0, nStart * sizeof(uint32_t), s), "event tables");
+	CK(cudaMemsetAsync(rows, 0, 2 * sizeof(uint32_t), s), "event tables");
+	evCountKernel<<<grid, 256, 0, s>>>(desc, start);
 	evScanKernel<<<blocks, 256, 0, s>>>(start, nSrc);
+	evOutKernel<<<grid, 256, 0, s>>>(desc, nullptr, nullptr, rows);
 	std::vector<uint32_t> hb(blocks);
+	uint32_t nRows = 0;
 	CK(cudaMemcpy2DAsync(hb.data(), 4, start + nSrc, 4ull * (nSrc + 1), 4, blocks, cudaMemcpyDeviceToHost, s), "event tables");
+	CK(cudaMemcpyAsync(&nRows, rows, 4, cudaMemcpyDeviceToHost, s), "event tables");
 	CK(cudaStreamSynchronize(s), "event tables");
 	uint64_t total = 0;
 	for (uint32_t &x : hb) { const uint32_t n = x; x = (uint32_t)total; total += n; }
 	if (total > 0x1FFFFFFFull) return "too many GR synapses for the event tables";
-	uint16_t *entry = alloc<uint16_t>(8 * total, false);
-	if (!entry) return "device allocation failed";
+	if (nRows > 0xFFFFFFu) return "too many GR->GO synapses for the event tables";
+	auto lists = [&]() {
+		bytes = 0;
+		take(entry, 8 * total);
+		take(om, std::max(1u, nRows));
+	};
+	base = nullptr;
+	lists();
+	o->arena[1] = base = alloc<uint8_t>(bytes, false);
+	if (!base) return "device allocation failed";
+	lists();
 	evUnusedKernel<<<1184, 256, 0, s>>>((uint32_t *)entry, 4 * total, kEvUnused | (kEvUnused << 16));
-	CK(cudaMemcpyAsync(base, hb.data(), 4ull * blocks, cudaMemcpyHostToDevice, s), "event tables");
-	evBaseKernel<<<blocks, 256, 0, s>>>(start, next, base, nSrc);
-	evFillKernel<<<grid, 256, 0, s>>>(devPtr(), next, entry);
+	CK(cudaMemcpyAsync(blockBase, hb.data(), 4ull * blocks, cudaMemcpyHostToDevice, s), "event tables");
+	evBaseKernel<<<blocks, 256, 0, s>>>(start, next, blockBase, nSrc);
+	evFillKernel<<<grid, 256, 0, s>>>(desc, next, entry);
+	evOutKernel<<<grid, 256, 0, s>>>(desc, oc, om, rows + 1);
+	evOrderKernel<<<grid, 256, 0, s>>>(desc, h_.pfDelay, pd, 1, 1, true);
+	CK(cudaGetLastError(), "event tables");
+	CK(cudaStreamSynchronize(s), "event tables");
 	// items of 64 cells for a usual list (its mean and two deviations)
 	auto items = [&](uint32_t slots, uint32_t sources) {
 		const double mean = (double)std::min(N, kEvCells) * slots / sources;
 		return std::min(16u, std::max(1u, (uint32_t)std::ceil((mean + 2 * std::sqrt(mean)) / 64)));
 	};
-	h_.evPerMF = items(h_.nMFSlots, h_.numMF);
-	h_.evPerGO = items(h_.nGOSlots, h_.numGO);
-	uint4 *oc = alloc<uint4>(N, false);
-	uint8_t *pd = alloc<uint8_t>(N, false);
-	uint32_t *rows = alloc<uint32_t>(2), nRows = 0;  // zeroed
-	if (!oc || !pd || !rows) return "device allocation failed";
-	evOutKernel<<<grid, 256, 0, s>>>(devPtr(), nullptr, nullptr, rows);
-	CK(cudaMemcpyAsync(&nRows, rows, 4, cudaMemcpyDeviceToHost, s), "event tables");
-	CK(cudaStreamSynchronize(s), "event tables");
-	if (nRows > 0xFFFFFFu) return "too many GR->GO synapses for the event tables";
-	uint4 *om = alloc<uint4>(std::max(1u, nRows), false);
-	if (!om) return "device allocation failed";
-	evOutKernel<<<grid, 256, 0, s>>>(devPtr(), oc, om, rows + 1);
-	evOrderKernel<<<grid, 256, 0, s>>>(devPtr(), h_.pfDelay, pd, 1, 1, true);
-	h_.outCell = oc;
-	h_.outMore = om;
-	h_.evPfDelay = pd;
-	CK(cudaGetLastError(), "event tables");
-	CK(cudaStreamSynchronize(s), "event tables");
-	release(next);
-	release(base);
-	release(rows);
-	h_.evStart = start;
-	h_.evEntry = (const uint4 *)entry;
-	return uploadDesc();
+	d.evPerMF = items(h_.nMFSlots, h_.numMF);
+	d.evPerGO = items(h_.nGOSlots, h_.numGO);
+	d.evStart = start;
+	d.evEntry = (const uint4 *)entry;
+	d.outCell = oc;
+	d.outMore = om;
+	d.evPfDelay = pd;
+	return "";
+}
+
+// Give back what a plan holds and did not hand over.
+void Network::dropEventPass(EventTables *o)
+{
+	for (void **p : {&o->arena[0], &o->arena[1], &o->building}) {
+		if (*p) release(*p);
+		*p = nullptr;
+	}
+}
+
+// The state into the per-tile pass's form, in a plan's tiling.
+std::string Network::takeEventPass(EventTables *o, cudaStream_t s)
+{
+	if (o->fresh) {
+		// the spikes that the last step left for the next are not carried over:
+		// entering the new form refills the ring from the spike buffers
+		CKS(setEventMode(false, s));
+		const DevNet &d = o->net;
+		h_.evWdShift = d.evWdShift; h_.evRows = d.evRows; h_.evTilesX = d.evTilesX; h_.evTiles = d.evTiles;
+		h_.evPCs = d.evPCs; h_.evBC = d.evBC; h_.evSC = d.evSC;
+		h_.evPerMF = d.evPerMF; h_.evPerGO = d.evPerGO;
+		h_.evStart = d.evStart; h_.evEntry = d.evEntry; h_.outCell = d.outCell; h_.outMore = d.outMore;
+		h_.evPfDelay = d.evPfDelay; h_.spkBits = d.spkBits; h_.evCnt = d.evCnt;
+		for (int k = 0; k < 2; k++) std::swap(evArena_[k], o->arena[k]);  // the old ones go with the plan
+		CKS(uploadDesc());
+	}
+	CKS(setEventMode(true, s));
+	streamsSlots_ = false;
+	return "";
 }
 
 // Device scratch of 8 bytes a GR, kept for the network's life (reordering and
@@ -1454,8 +1513,16 @@ std::string Simulator::create(const std::vector<State *> &states, const std::vec
 		if (sscanf(env, "%d,%d,%d,%d,%d", &g.W, &g.RW, &g.S, &g.B, &g.M) != 5) return "CBM_PASS_TMA must be W,RW,S,B,M";
 		return usePassGeometry(g);
 	}
-	const std::vector<PassGeometry> cands = passCandidates();
-	return usePassGeometry(cands.front());
+	// the default; where its tables do not fit in memory, or do not cover the network,
+	// the next that runs (the plain pass needs none)
+	std::string first;
+	for (const PassGeometry &c : passCandidates()) {
+		const std::string e = usePassGeometry(c);
+		if (e.empty()) return "";
+		if (first.empty()) first = e;
+		if (!passBroken_.empty()) break;
+	}
+	return first;
 }
 
 // Cells a tile of the per-tile pass should hold, a multiple of rounds of SC:
@@ -1528,6 +1595,26 @@ std::vector<PassGeometry> Simulator::passCandidates() const
 std::string Simulator::usePassGeometry(const PassGeometry &g)
 {
 	CK(cudaSetDevice(device_), "selecting the device");
+	// what can be refused, or want memory, comes first, beside the pass in use: it
+	// goes on as it was
+	PassPlan p;
+	p.events.resize(nets_.size());
+	std::string e = planPass(g, &p);
+	if (e.empty()) {
+		e = takePass(&p);
+		if (!e.empty()) passBroken_ = "switching the GR pass failed: " + e;
+		dropGraphs();  // captured graphs hold the old kernel
+	} else {
+		cudaGetLastError();  // reported here, not by the next launch's check
+	}
+	for (size_t i = 0; i < nets_.size(); i++) nets_[i]->dropEventPass(&p.events[i]);
+	if (p.blocks.ptr) cudaFree(p.blocks.ptr);
+	return e;
+}
+
+// The kernel, its launch and its tables for a geometry, or why it cannot run.
+std::string Simulator::planPass(const PassGeometry &g, PassPlan *p)
+{
 	uint32_t minRows = UINT32_MAX, maxSlots = 0;
 	bool capable = !nets_.empty();
 	for (Network *n : nets_) {
@@ -1535,186 +1622,149 @@ std::string Simulator::usePassGeometry(const PassGeometry &g)
 		minRows = std::min(minRows, n->passRows());
 		maxSlots = std::max({maxSlots, n->dev().nMFSlots, n->dev().nGOSlots, n->dev().nOutSlots});
 	}
-	// leaving the vector pass: the last step's PF->PC reduction is still pair
-	// sums, and the small-cell update goes back to partial sums
-	if (passVec_ && g.kind != 3)
-		for (Network *n : nets_) CKS(n->setPcSumMode(false, s0_));
-	// everything but the per-tile pass counts GR->GO spikes when they arrive
-	auto arriveMode = [&]() -> std::string {
-		for (Network *n : nets_) {
-			CKS(n->setEventMode(false, s0_));
-			n->streamsSlots_ = true;
-		}
-		return "";
-	};
-	if (g.kind == 3 && nets_.size() > 1) {
+	p->geom = g;
+	if (g.kind == 0) return "";
+	int numSMs = 0, perSM = 0;
+	CK(cudaDeviceGetAttribute(&numSMs, cudaDevAttrMultiProcessorCount, device_), "SM count");
+	if (g.kind == 3) {
 		for (Network *n : nets_)
 			if (!passVecCapable(n->dev())) return "the vector GR pass runs networks of its compiled shape";
-		const void *fn = passVecBatchKernel();
-		if (!dVecUnitOffset_.ptr) {
-			std::vector<uint32_t> units(1, 0), pcs(1, 0);
-			for (Network *n : nets_) {
-				units.push_back(units.back() + n->dev().numGR / 128u);
-				pcs.push_back(pcs.back() + n->dev().numPC);
-			}
-			auto up = [&](DeviceBuf &b, const std::vector<uint32_t> &v) -> std::string {
-				CK(cudaMalloc(&b.ptr, v.size() * sizeof(uint32_t)), "allocating vector-pass tables");
-				b.bytes = v.size() * sizeof(uint32_t);
-				CK(cudaMemcpyAsync(b.ptr, v.data(), b.bytes, cudaMemcpyHostToDevice, s0_), "uploading vector-pass tables");
-				return "";
-			};
-			CKS(up(dVecUnitOffset_, units));
-			CKS(up(dVecPcOffset_, pcs));
-			CKS(up(dVecClaim_, std::vector<uint32_t>(4, 0)));
-		}
-		int perSM = 0, numSMs = 0;
-		CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fn, 32 * kVecWarps, 0), "pass occupancy");
-		CK(cudaDeviceGetAttribute(&numSMs, cudaDevAttrMultiProcessorCount, device_), "SM count");
-		uint32_t units = 0;
+		p->W = kVecWarps - 1;
+		p->threads = 32u * kVecWarps;
+		uint32_t claim = kVecBatchClaim, units = 0, sms = (uint32_t)numSMs;
 		for (Network *n : nets_) units += n->dev().numGR / 128u;
-		const uint32_t claims = (units + kVecBatchClaim - 1) / kVecBatchClaim;
-		passGrid_ = std::max<uint32_t>(1, std::min<uint32_t>((claims + kVecWarps - 1) / kVecWarps,
-				(uint32_t)std::max(1, perSM) * (uint32_t)numSMs));
-		CK(cudaMemsetAsync(dVecClaim_.ptr, 0, dVecClaim_.bytes, s0_), "pass claim counters");
-		for (Network *n : nets_) CKS(n->setPcSumMode(true, s0_));
-		CKS(arriveMode());
-		passTmaFn_ = fn;
-		passVec_ = true;
-		passPersistent_ = false;
-		passTmaW_ = kVecWarps - 1;
-		passTmaThreads_ = 32u * kVecWarps;
-		passTmaR_ = passTmaS_ = 0;
-		passTmaSmem_ = 0;
-		passGeom_ = g;
-		dropGraphs();
-		return "";
-	}
-	if (g.kind == 3) {
-		if (nets_.size() != 1 || !passVecCapable(nets_[0]->dev()))
-			return "the vector GR pass runs networks of its compiled shape";
-		Network &n = *nets_[0];
-		const size_t smem = passVecSmemBytes(n.dev());
-		const void *fn = passVecKernel();
-		CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "pass smem");
-		int perSM = 0, numSMs = 0;
-		CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fn, 32 * kVecWarps, smem), "pass occupancy");
-		CK(cudaDeviceGetAttribute(&numSMs, cudaDevAttrMultiProcessorCount, device_), "SM count");
-		// units claimed at a time (CBM_VEC_CLAIM, tuning; default kVecClaim)
-		vecClaim_ = kVecClaim;
-		if (const char *env = getenv("CBM_VEC_CLAIM")) {
-			const int c = atoi(env);
-			if (c < 1 || c > 64) return "CBM_VEC_CLAIM must be 1..64";
-			vecClaim_ = (uint32_t)c;
+		if (nets_.size() > 1) {
+			p->fn = passVecBatchKernel();
+			if (!dVecClaim_.ptr) {
+				std::vector<uint32_t> unit(1, 0), pcs(1, 0);
+				for (Network *n : nets_) {
+					unit.push_back(unit.back() + n->dev().numGR / 128u);
+					pcs.push_back(pcs.back() + n->dev().numPC);
+				}
+				auto up = [&](DeviceBuf &b, const std::vector<uint32_t> &v) -> std::string {
+					if (b.ptr) return "";
+					b.bytes = v.size() * sizeof(uint32_t);
+					CK(cudaMalloc(&b.ptr, b.bytes), "allocating vector-pass tables");
+					CK(cudaMemcpyAsync(b.ptr, v.data(), b.bytes, cudaMemcpyHostToDevice, s0_), "uploading vector-pass tables");
+					return "";
+				};
+				CKS(up(dVecUnitOffset_, unit));
+				CKS(up(dVecPcOffset_, pcs));
+				CKS(up(dVecClaim_, std::vector<uint32_t>(4, 0)));
+			}
+		} else {
+			const DevNet &h = nets_[0]->dev();
+			p->smem = passVecSmemBytes(h);
+			p->fn = passVecKernel();
+			CK(cudaFuncSetAttribute(p->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem), "pass smem");
+			// units claimed at a time (CBM_VEC_CLAIM, tuning; default kVecClaim)
+			claim = kVecClaim;
+			if (const char *env = getenv("CBM_VEC_CLAIM")) {
+				const int c = atoi(env);
+				if (c < 1 || c > 64) return "CBM_VEC_CLAIM must be 1..64";
+				claim = (uint32_t)c;
+			}
+			p->claim = claim;
+			// every CTA resident from the start: the small-cell kernel's two
+			// CTAs hold an SM each while the pass runs
+			sms = (uint32_t)std::max(1, numSMs - 2);
 		}
-		// every CTA resident from the start: the small-cell kernel's two
-		// CTAs hold an SM each while the pass runs
-		const uint32_t claims = (n.dev().numGR / 128u + vecClaim_ - 1) / vecClaim_;
-		const uint32_t sms = (uint32_t)std::max(1, numSMs - 2);
-		passGrid_ = std::max<uint32_t>(1, std::min<uint32_t>((claims + kVecWarps - 1) / kVecWarps,
-				(uint32_t)std::max(1, perSM) * sms)) + passVecReduceCTAs(n.dev());
-		// claim counters from zero (another pass kind may have run meanwhile)
-		CK(cudaMemsetAsync(n.dev().passClaim, 0, 4 * sizeof(uint32_t), s0_), "pass claim counters");
-		CKS(n.setPcSumMode(true, s0_));
-		CKS(arriveMode());
-		passTmaFn_ = fn;
-		passVec_ = true;
-		passPersistent_ = false;
-		passTmaW_ = kVecWarps - 1;
-		passTmaThreads_ = 32u * kVecWarps;
-		passTmaR_ = passTmaS_ = 0;
-		passTmaSmem_ = smem;
-		passGeom_ = g;
-		dropGraphs();
-		return "";
-	}
-	passVec_ = false;
-	if (g.kind == 0) {
-		CKS(arriveMode());
-		passTmaFn_ = nullptr;
-		passPersistent_ = false;
-		passTmaW_ = passTmaR_ = passTmaS_ = 0;
-		passGeom_ = g;
-		dropGraphs();
+		CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, p->fn, (int)p->threads, p->smem), "pass occupancy");
+		const uint32_t claims = (units + claim - 1) / claim;
+		p->grid = std::max<uint32_t>(1, std::min<uint32_t>((claims + kVecWarps - 1) / kVecWarps,
+				(uint32_t)std::max(1, perSM) * sms));
+		if (nets_.size() == 1) p->grid += passVecReduceCTAs(nets_[0]->dev());
 		return "";
 	}
 	if (!capable) return "the TMA GR pass needs tiles of 32-cell rows in every network";
 	// (the per-tile pass has no slot loops: M is accepted and has no effect)
 	if (g.kind != 1 && g.M > 0 && maxSlots > (uint32_t)g.M)
 		return "a network has more synapse slots than the geometry's slot bound";
-	const void *fn = nullptr;
-	uint32_t R = 0, threads = 0, grid = passBlocks_;
-	size_t smem = 0;
-	if (g.kind == 1) {
-		bool oneZone = true;
-		for (Network *n : nets_) oneZone = oneZone && n->dev().numZones == 1;
-		fn = g.RW > 0 && g.S > 0 ? passTmaKernelFor(g.W, (int)stagesOf(g), oneZone) : nullptr;
-		if (!fn) return "per-tile GR-pass geometry not compiled in";
-		if (!passTmaFits(g, &smem)) return "the per-tile GR-pass geometry does not fit every network";
-		const uint32_t SC = 128u * g.W, target = tileTarget(nets_, SC);
-		R = SC / 32u;
-		threads = 32u * (g.W + 1);
-		std::vector<PassBlock> blocks;
-		for (Network *n : nets_) {
-			CKS(n->buildEventPass(target, SC, s0_));
-			CKS(n->setEventMode(true, s0_));
-			n->streamsSlots_ = false;
-		}
-		// the event CTAs first: theirs is the longer chain of latencies
-		passEvents_ = nets_.size() > 1 ? 0u : nets_[0]->eventBlocks();
-		grid = passEvents_ + nets_[0]->dev().evTiles;
-		if (nets_.size() > 1) {
-			for (Network *n : nets_)
-				for (uint32_t b = 0; b < n->eventBlocks(); b++) blocks.push_back({n->devPtr(), b, 1});
-			for (Network *n : nets_)
-				for (uint32_t b = 0; b < n->dev().evTiles; b++) blocks.push_back({n->devPtr(), b, 0});
-			grid = (uint32_t)blocks.size();
-		}
-		if (dPassBlocks_.ptr) cudaFree(dPassBlocks_.ptr);
-		dPassBlocks_ = DeviceBuf();
-		if (!blocks.empty()) {
-			CK(cudaMalloc(&dPassBlocks_.ptr, blocks.size() * sizeof(PassBlock)), "allocating launch tables");
-			dPassBlocks_.bytes = blocks.size() * sizeof(PassBlock);
-			CK(cudaMemcpyAsync(dPassBlocks_.ptr, blocks.data(), dPassBlocks_.bytes, cudaMemcpyHostToDevice, s0_),
-					"uploading launch tables");
-		}
-	} else {
+	p->W = (uint32_t)g.W;
+	p->S = (uint32_t)g.S;
+	p->threads = 32u * (g.W + 1);
+	if (g.kind == 2) {
 		if (nets_.size() != 1) return "the persistent GR pass runs one network";
-		if (nets_[0]->dev().nOutSlots > kOutInline) return "the persistent GR pass streams at most 4 GR->GO slots";
-		fn = passPersistentKernelFor(g.W, g.S, g.B, g.M);
-		if (!fn) return "persistent GR-pass geometry not compiled in";
-		R = (uint32_t)(2 * g.W);
-		if (R > minRows) return "more rows per unit than a tile has";
 		Network &n = *nets_[0];
-		const PassLayout L = passLayout(R, n.dev().nMFSlots, n.dev().nGOSlots, n.dev().nOutSlots, n.dev().numZones);
-		smem = 128 + (size_t)g.S * L.bytes + 16ull * g.S + 4ull * n.dev().numPC * n.dev().numZones +
+		if (n.dev().nOutSlots > kOutInline) return "the persistent GR pass streams at most 4 GR->GO slots";
+		p->fn = passPersistentKernelFor(g.W, g.S, g.B, g.M);
+		if (!p->fn) return "persistent GR-pass geometry not compiled in";
+		p->R = (uint32_t)(2 * g.W);
+		if (p->R > minRows) return "more rows per unit than a tile has";
+		const PassLayout L = passLayout(p->R, n.dev().nMFSlots, n.dev().nGOSlots, n.dev().nOutSlots, n.dev().numZones);
+		p->smem = 128 + (size_t)g.S * L.bytes + 16ull * g.S + 4ull * n.dev().numPC * n.dev().numZones +
 			32ull * (n.dev().mfWords + n.dev().goWords);
-		threads = 32u * (g.W + 1);
+		if (p->smem > 227 * 1024) return "GR-pass geometry needs more shared memory than a CTA has";
+		CK(cudaFuncSetAttribute(p->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem), "pass smem");
+		CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, p->fn, (int)p->threads, p->smem), "pass occupancy");
+		const uint32_t units = n.dev().numPC * n.dev().tilesPerPC * (n.passRows() / p->R);
+		p->grid = std::min<uint32_t>(units, (uint32_t)std::max(1, perSM) * (uint32_t)numSMs);
+		return "";
 	}
-	if (smem > 227 * 1024) return "GR-pass geometry needs more shared memory than a CTA has";
-	if (g.kind == 2) {
-		CKS(nets_[0]->buildPassMaps(R));
-		CKS(arriveMode());
+	bool oneZone = true;
+	for (Network *n : nets_) oneZone = oneZone && n->dev().numZones == 1;
+	p->fn = g.RW > 0 && g.S > 0 ? passTmaKernelFor(g.W, (int)stagesOf(g), oneZone) : nullptr;
+	if (!p->fn) return "per-tile GR-pass geometry not compiled in";
+	if (!passTmaFits(g, &p->smem)) return "the per-tile GR-pass geometry does not fit every network";
+	CK(cudaFuncSetAttribute(p->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem), "pass smem");
+	const uint32_t SC = 128u * g.W, target = tileTarget(nets_, SC);
+	p->R = SC / 32u;
+	for (size_t i = 0; i < nets_.size(); i++) CKS(nets_[i]->planEventPass(target, SC, &p->events[i], s0_));
+	// the event CTAs first: theirs is the longer chain of latencies
+	if (nets_.size() == 1) {
+		p->eventCTAs = nets_[0]->eventBlocks();
+		p->grid = p->eventCTAs + p->events[0].net.evTiles;
+		return "";
 	}
-	CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "pass smem");
-	if (g.kind == 2) {
-		int perSM = 0, numSMs = 0;
-		CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fn, (int)threads, smem), "pass occupancy");
-		CK(cudaDeviceGetAttribute(&numSMs, cudaDevAttrMultiProcessorCount, device_), "SM count");
-		Network &n = *nets_[0];
-		const uint32_t units = n.dev().numPC * n.dev().tilesPerPC * (n.passRows() / R);
-		grid = std::min<uint32_t>(units, (uint32_t)std::max(1, perSM) * (uint32_t)numSMs);
+	std::vector<PassBlock> blocks;
+	for (Network *n : nets_)
+		for (uint32_t b = 0; b < n->eventBlocks(); b++) blocks.push_back({n->devPtr(), b, 1});
+	for (size_t i = 0; i < nets_.size(); i++)
+		for (uint32_t b = 0; b < p->events[i].net.evTiles; b++) blocks.push_back({nets_[i]->devPtr(), b, 0});
+	p->grid = (uint32_t)blocks.size();
+	p->blocks.bytes = blocks.size() * sizeof(PassBlock);
+	CK(cudaMalloc(&p->blocks.ptr, p->blocks.bytes), "allocating launch tables");
+	CK(cudaMemcpyAsync(p->blocks.ptr, blocks.data(), p->blocks.bytes, cudaMemcpyHostToDevice, s0_), "uploading launch tables");
+	return "";
+}
+
+// The networks' state into the form that a planned pass works on, and the pass
+// into use.
+std::string Simulator::takePass(PassPlan *p)
+{
+	const int kind = p->geom.kind;
+	if (kind == 2) CKS(nets_[0]->buildPassMaps(p->R));
+	// the vector pass leaves the last step's PF->PC reduction as pair sums, and the
+	// small-cell update takes sums from it instead of partial sums
+	for (Network *n : nets_) CKS(n->setPcSumMode(kind == 3, s0_));
+	for (size_t i = 0; i < nets_.size(); i++) {
+		if (kind == 1) {
+			CKS(nets_[i]->takeEventPass(&p->events[i], s0_));
+			continue;
+		}
+		// everything but the per-tile pass counts GR->GO spikes when they arrive
+		CKS(nets_[i]->setEventMode(false, s0_));
+		nets_[i]->streamsSlots_ = true;
 	}
-	passTmaFn_ = fn;
-	passPersistent_ = g.kind == 2;
-	passTmaW_ = (uint32_t)g.W;
-	passTmaThreads_ = threads;
-	passTmaR_ = R;
-	passTmaS_ = (uint32_t)g.S;
-	passTmaSmem_ = smem;
-	passGrid_ = grid;
-	passGeom_ = g;
-	// captured graphs hold the old kernel
-	dropGraphs();
+	if (kind == 3) {
+		// claim counters from zero (another pass kind may have run meanwhile)
+		if (nets_.size() > 1) CK(cudaMemsetAsync(dVecClaim_.ptr, 0, dVecClaim_.bytes, s0_), "pass claim counters");
+		else CK(cudaMemsetAsync(nets_[0]->dev().passClaim, 0, 4 * sizeof(uint32_t), s0_), "pass claim counters");
+		if (nets_.size() == 1) vecClaim_ = p->claim;
+	}
+	CK(cudaStreamSynchronize(s0_), "pass switch");
+	passTmaFn_ = p->fn;
+	passVec_ = kind == 3;
+	passPersistent_ = kind == 2;
+	passTmaW_ = p->W;
+	passTmaR_ = p->R;
+	passTmaS_ = p->S;
+	passTmaThreads_ = p->threads;
+	passTmaSmem_ = p->smem;
+	passGrid_ = p->grid;
+	passEvents_ = p->eventCTAs;
+	passGeom_ = p->geom;
+	std::swap(dPassBlocks_, p->blocks);  // the old ones go with the plan
 	return "";
 }
 
@@ -1733,6 +1783,7 @@ std::string Simulator::uploadCtl()
 
 std::string Simulator::enqueueStep(uint32_t k, bool instrument, bool chained)
 {
+	if (!passBroken_.empty()) return passBroken_;
 	const DevNet *const *netsArg = (const DevNet *const *)dNetPtrs_.ptr;
 	const uint32_t *stageArg = (const uint32_t *)dStageBytes_.ptr;
 	const uint32_t *offsArg = (const uint32_t *)dBlockOffset_.ptr;
@@ -2064,6 +2115,7 @@ std::string Simulator::stageMF(size_t i, const uint8_t *mf)
 std::string Simulator::exportField(size_t i, Field f, uint32_t zone, void *dst, size_t bytes)
 {
 	CK(cudaSetDevice(device_), "selecting the device");
+	if (!passBroken_.empty()) return passBroken_;
 	if (bytes > hExportBytes_) {
 		if (hExport_) cudaFreeHost(hExport_);
 		hExport_ = nullptr;

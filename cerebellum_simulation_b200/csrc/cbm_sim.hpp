@@ -48,6 +48,24 @@ struct PassGeometry {
 	int kind = 0, W = 0, RW = 1, S = 0, B = 0, M = 0;
 };
 
+// The per-tile pass's tables of one network in some tiling, until it takes them.
+struct EventTables {
+	DevNet net{};           // the network with the tiling and the tables
+	bool fresh = false;     // tables of their own (else those in use serve)
+	void *arena[2] = {};    // what holds them
+	void *building = nullptr;
+};
+
+// A GR pass that could come into use: its launch, and its tables.
+struct PassPlan {
+	PassGeometry geom;
+	const void *fn = nullptr;  // null: the plain pass
+	uint32_t W = 0, R = 0, S = 0, threads = 0, grid = 0, eventCTAs = 0, claim = 0;
+	size_t smem = 0;
+	DeviceBuf blocks;
+	std::vector<EventTables> events;
+};
+
 // A set of networks that advance together: one network for the drop-in
 // CBMSimCore path, many for the batched sweep.
 class Simulator {
@@ -105,6 +123,8 @@ public:
 	std::vector<PassGeometry> passCandidates() const;
 	const PassGeometry &passGeometryInUse() const { return passGeom_; }
 	std::string usePassGeometry(const PassGeometry &g);
+	std::string planPass(const PassGeometry &g, PassPlan *p);
+	std::string takePass(PassPlan *p);
 	bool passTmaFits(const PassGeometry &g, size_t *smem) const;
 	// Device error word of every network (kErr* bits): non-empty on error.
 	std::string checkDeviceErrors();
@@ -171,6 +191,7 @@ private:
 	bool lastStepPublishes_ = false;  // the last launch was a single step that writes the mailbox
 	uint32_t vecClaim_ = 2;  // its units claimed at a time (single network)
 	PassGeometry passGeom_;
+	std::string passBroken_;  // why no step can run: a pass switch failed half way
 	size_t passTmaSmem_ = 0;
 	cudaGraphExec_t graphExec_ = nullptr;
 	uint32_t graphChunk_ = 0;
@@ -243,8 +264,10 @@ public:
 	// with S stages.
 	bool eventTiling(uint32_t target, uint32_t SC, DevNet *h) const;
 	static size_t eventSmemBytes(const DevNet &h, uint32_t SC, uint32_t S);
-	// Tile the cells and build the event tables unless they are there.
-	std::string buildEventPass(uint32_t target, uint32_t SC, cudaStream_t s);
+	// The event tables of a tiling, taking them into use, and giving them back.
+	std::string planEventPass(uint32_t target, uint32_t SC, EventTables *o, cudaStream_t s);
+	std::string takeEventPass(EventTables *o, cudaStream_t s);
+	void dropEventPass(EventTables *o);
 	// Enter or leave the per-tile pass's form of the state: GR->GO counts
 	// delivered when cells spike instead of when the spikes arrive, the
 	// conductances one step behind with the arrived spikes beside them, and the
@@ -285,6 +308,7 @@ private:
 	std::map<const void *, size_t> allocBytes_;
 	double avgMF_ = 0, avgGO_ = 0, avgOut_ = 0;
 	bool streamsSlots_ = true;  // the GR pass in use streams the synapse tables (not the per-tile pass)
+	void *evArena_[2] = {};     // what holds the event tables in use
 	bool evMode_ = false;       // the state is in the per-tile pass's form (setEventMode)
 	// pinned staging of host MF input: kMFStage slots, each reused once the
 	// copy that last read it has run (mfStageEv_)
