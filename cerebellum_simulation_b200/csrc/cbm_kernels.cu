@@ -752,7 +752,9 @@ __device__ void golgiRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm
 	float *sV = sScale + numGO;
 	float *sTh = sV + numGO;
 	uint8_t *sAp = reinterpret_cast<uint8_t *>(sTh + numGO);
+#pragma unroll 1
 	for (uint32_t i = tid; i < N->mfWords; i += nThr) sMF[i] = mfW[i];
+#pragma unroll 1
 	for (uint32_t i = tid; i < numGO; i += nThr) sMFGO[i] = 0;
 	if (tid < 32) sExp2[tid] = kExp2Tab[tid];
 	__syncthreads();
@@ -760,6 +762,7 @@ __device__ void golgiRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm
 	uint32_t *goIn = N->goCount + (size_t)((t - 1) & (kGoRing - 1u)) * numGO;
 	uint32_t *goBitsOut = N->goBits + (size_t)(t & 1) * N->goWords;
 	const float gIncGRtoGO = N->ctl->gIncGRtoGO;
+#pragma unroll 1
 	for (uint32_t base = 0; base < numGO; base += nThr) {
 		const uint32_t i = base + tid;
 		uint8_t ap = 0;
@@ -808,6 +811,7 @@ __device__ void golgiRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm
 	__syncthreads();
 	// updateMFtoGOOut (innet.cpp:912-931): every spiking MF adds one to each
 	// GO it targets (integer counts: the order of the additions is immaterial)
+#pragma unroll 1
 	for (uint32_t i = tid; i < N->numMF; i += nThr) {
 		if (!spikeBit(sMF, i)) continue;
 		const int n = N->numpMFfromMFtoGO[i];
@@ -817,6 +821,7 @@ __device__ void golgiRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm
 	}
 	// updateGOtoGOOut: GABA inputs in (source, slot) order, depression scale,
 	// electrical coupling (innet.cpp:937-978)
+#pragma unroll 1
 	for (uint32_t d = tid; d < numGO; d += nThr) {
 		uint32_t cnt = 0;
 		float acc = 0;
@@ -833,6 +838,7 @@ __device__ void golgiRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm
 		const uint8_t ap = sAp[d];
 		N->goGABAOutSynScaleGOGO[d] = s + (!ap) * (1 - s) * N->goGABAGOGOSynRec - ap * (s * (1 - N->goGABAGOGOSynDepF));
 		float vc = 0;
+#pragma unroll 1
 		for (int j = 0; j < nc; j++) {
 			const uint32_t n = N->pGOCoupInGOGO[(size_t)d * N->maxnumpGOCoupInGOGO + j];
 			vc = vc + N->coupleRiRjRatioGO * (sV[n] - sV[d]);
@@ -840,16 +846,20 @@ __device__ void golgiRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm
 		N->vCoupleGO[d] = vc;
 	}
 	__syncthreads();
+#pragma unroll 1
 	for (uint32_t i = tid; i < numGO; i += nThr) N->inputMFGO[i] = sMFGO[i];
 	// threshold coupling: the reference's serial sweep reads already-updated
 	// thresholds of lower-indexed neighbours; the level schedule preserves it
+#pragma unroll 1
 	for (uint32_t L = 0; L < N->numCoupLevels; L++) {
 		__syncthreads();
+#pragma unroll 1
 		for (uint32_t e = N->coupLevelStart[L] + tid; e < N->coupLevelStart[L + 1]; e += nThr) {
 			const uint32_t i = N->coupLevelGO[e];
 			const float own = sTh[i];
 			float tc = 0;
 			const int nc = N->numpGOCoupInGOGO[i];
+#pragma unroll 1
 			for (int j = 0; j < nc; j++) {
 				const uint32_t n = N->pGOCoupInGOGO[(size_t)i * N->maxnumpGOCoupInGOGO + j];
 				const float other = n < i ? N->threshCurGO[n] : sTh[n];
@@ -932,11 +942,13 @@ __device__ void zoneRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm,
 	// MF bookkeeping; the updates are independent.
 	// calcPCActivities (mzone.cpp:187-226), one warp per PC; the SC
 	// conductances update elementwise, their sum runs in the reference's order
+#pragma unroll 1
 	for (uint32_t task = warp; task < Z * numPC; task += nWarps) {
 		const uint32_t z = Z == 1 ? 0u : task / numPC, i = Z == 1 ? task : task % numPC;
 		const DevZone &Q = N->zones[z];
 		const float inputSum = in.pcSum[z] ? in.pcSum[z][i] : pcRowTree(in.pcPart[z] + (size_t)i * N->bs, N->bs, lane);
 		const uint32_t nSC = N->numpPCfromSCtoPC;
+#pragma unroll 1
 		for (uint32_t j = lane; j < nSC; j += 32) {
 			const size_t k = (size_t)i * nSC + j;
 			const float g0 = Q.gSCPC[k];
@@ -971,6 +983,7 @@ __device__ void zoneRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm,
 		}
 	}
 	// calcBCActivities (mzone.cpp:228-256)
+#pragma unroll 1
 	for (uint32_t c = tid; c < Z * numBC; c += nThr) {
 		const uint32_t bz = Z == 1 ? 0u : c / numBC, bi = Z == 1 ? c : c % numBC;
 		const DevZone &Q = N->zones[bz];
@@ -992,6 +1005,7 @@ __device__ void zoneRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm,
 		Q.threshBC[bi] = ap * N->threshMaxBC + (!ap) * (th);
 	}
 	// calcSCActivities (innet.cpp:892-911)
+#pragma unroll 1
 	for (uint32_t c = tid; c < numSC; c += nThr) {
 		const uint32_t sApBuf = N->apBufSC[c];
 		const float sthOld = N->threshSC[c];
@@ -1009,13 +1023,16 @@ __device__ void zoneRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm,
 		N->threshSC[c] = ap * N->threshMaxSC + (!ap) * (th);
 	}
 	// updateMFInput's bookkeeping (innet.cpp:800-815)
+#pragma unroll 1
 	for (uint32_t c = tid; c < numMF; c += nThr) {
 		const uint32_t m = spikeBit(sMF, c);
 		N->histMF[c] = N->histMF[c] || (m > 0);
 		N->apBufMF[c] = (N->apBufMF[c] << 1) | (m * 0x00000001u);
 	}
 	barSync(1, aThr);
+#pragma unroll 1
 	for (uint32_t i = tid; i < numBC; i += nThr) N->bcCount[(size_t)R * numBC + i] = 0;
+#pragma unroll 1
 	for (uint32_t i = tid; i < numSC; i += nThr) N->scCount[(size_t)R * numSC + i] = 0;
 	}
 
@@ -1031,6 +1048,7 @@ __device__ void zoneRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm,
 	// last thread down, so that they run on warps that take no NC (or the
 	// last NCs).
 	const uint32_t nIOSyn = Z * numIO * nIONC;
+#pragma unroll 1
 	for (uint32_t c = nThr - 1 - tid; c < nIOSyn; c += nThr) {
 		const uint32_t iz = Z == 1 ? 0u : c / (numIO * nIONC), ik = Z == 1 ? c : c % (numIO * nIONC);
 		const DevZone &Q = N->zones[iz];
@@ -1046,10 +1064,12 @@ __device__ void zoneRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm,
 	// one warp per NC: its MF->NC synaptic conductances (lanes over the
 	// synapses) into the warp's scratch, then the sums and the update, with
 	// no barrier but the warp's own
+#pragma unroll 1
 	for (uint32_t task = warp; task < Z * numNC; task += nWarps) {
 		const uint32_t z = Z == 1 ? 0u : task / numNC, i = Z == 1 ? task : task % numNC;
 		const DevZone &Q = N->zones[z];
 		float *const sNw = ncScratch + (size_t)task * 2 * nMFNC;
+#pragma unroll 1
 		for (uint32_t j = lane; j < nMFNC; j += 32) {
 			const size_t nk = (size_t)i * nMFNC + j;
 			const float nIn = Q.inputMFNC[nk], nWt = Q.mfSynWeightNC[nk];
@@ -1075,6 +1095,7 @@ __device__ void zoneRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm,
 		const float vNC0 = Q.vNC[i], thNC0 = Q.threshNC[i];
 		const uint32_t apBufNC = Q.apBufNC[i];
 		const uint32_t nPCNC = N->numpNCfromPCtoNC;
+#pragma unroll 1
 		for (uint32_t j = lane; j < nPCNC; j += 32) {
 			const size_t k = (size_t)i * nPCNC + j;
 			const float g0 = Q.gPCNC[k], scale = Q.gPCScaleNC[k];
@@ -1108,6 +1129,7 @@ __device__ void zoneRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm,
 	// now, from the group's last warp, which has no IO update (its system
 	// fence overlaps the IO updates)
 	if (ncMailbox && tid == nThr - 32u) publishNC(N, t, ncMailbox);
+#pragma unroll 1
 	for (uint32_t task = tid; task < Z * numIO; task += nThr) {
 		const uint32_t z = Z == 1 ? 0u : task / numIO, i = Z == 1 ? task : task % numIO;
 		const DevZone &Q = N->zones[z];
@@ -1115,6 +1137,7 @@ __device__ void zoneRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm,
 		const float errDrive = task == tid ? errOwn : errDriveOf(N, t, z);
 		const uint32_t apBuf = Q.apBufIO[i];
 		float gNCSum = 0;
+#pragma unroll 1
 		for (uint32_t j = 0; j < nIONC; j++) gNCSum = gNCSum + ioScratch[(size_t)task * nIONC + j];
 		gNCSum = gNCSum / 3.1;
 		float v = v0;
@@ -1146,6 +1169,7 @@ __device__ void zoneRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm,
 	// timer is.  (The draws and the selector as a phase of their own, behind
 	// one more barrier, took 2.7 us of a 16K network's 12.7 us step; so 11.8.)
 	if (warp == 0) {
+#pragma unroll 1
 		for (uint32_t r = lane; r < Z * numNC; r += 32u) {
 			const uint32_t z = Z == 1 ? 0u : r / numNC, i = Z == 1 ? r : r % numNC;
 			const DevZone &Q = N->zones[z];
@@ -1157,6 +1181,7 @@ __device__ void zoneRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm,
 		}
 	} else if (warp == 1) {
 		// (the IO updates have read ioScratch)
+#pragma unroll 1
 		for (uint32_t r = lane; r < Z * numIO * nIONC; r += 32u) {
 			const uint32_t per = numIO * nIONC;
 			const uint32_t z = Z == 1 ? 0u : r / per, k = Z == 1 ? r : r % per;
@@ -1166,6 +1191,7 @@ __device__ void zoneRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm,
 		const uint32_t nMFIn = Z * numNC * nMFNC, nBCPC = Z * numPC, nSCPC = Z * numPC * N->numpPCfromSCtoPC,
 			nPCBC = Z * numBC, nPCNC = Z * numNC * N->numpNCfromPCtoNC, nIO = Z * numIO;
 		const uint32_t total = nMFIn + nBCPC + nSCPC + nPCBC + nPCNC + nIO + Z;
+#pragma unroll 1
 		for (uint32_t task = tid - 64u; task < total; task += oThr - 64u) {
 			uint32_t r = task;
 			if (r < nMFIn) {
@@ -1218,6 +1244,7 @@ __device__ void zoneRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm,
 				const int32_t timer = Q.pfPCPlastTimerIO[i];
 				const float vOwn = Q.vIO[i];
 				float vc = 0;
+#pragma unroll 1
 				for (uint32_t j = 0; j < N->numpIOInIOIO; j++)
 					vc = vc + N->coupleRiRjRatioIO * (Q.vIO[Q.pIOInIOIO[(size_t)i * N->numpIOInIOIO + j]] - vOwn);
 				const int32_t tm = (!ap) * (timer + 1) + ap * N->tsLTDStartAPIO;
@@ -1259,6 +1286,7 @@ __device__ void zoneRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm,
 	// (mzone.cpp:586-600)
 	{
 		const uint32_t nDraw = Z * numIO * nIONC, nW = popStep ? Z * numNC * nMFNC : 0;
+#pragma unroll 1
 		for (uint32_t task = tid; task < nDraw + nW; task += nThr) {
 			uint32_t r = task;
 			if (r < nDraw) {
@@ -1284,6 +1312,7 @@ __device__ void zoneRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm,
 	}
 	if (stepMod(t, N->numTSinMFHist) == 0) {
 		__syncthreads();
+#pragma unroll 1
 		for (uint32_t i = tid; i < numMF; i += nThr) N->histMF[i] = 0;
 	}
 	// the error drive is consumed once (mzone.cpp:334)
@@ -1312,11 +1341,13 @@ __device__ void stageIn(const DevNet *N, uint8_t *base, uint32_t bytes)
 {
 	const uint32_t tid = threadIdx.x, nThr = blockDim.x;
 	const uint8_t *src = reinterpret_cast<const uint8_t *>(N);
+#pragma unroll 1
 	for (uint32_t o = 16u * tid; o < bytes; o += 16u * nThr) cpAsync16(base + o, src + o);
 	cpAsyncWaitAll();
 	__syncthreads();
 	DevNet *sNet = reinterpret_cast<DevNet *>(base);
 	const StageSeg *segs = reinterpret_cast<const StageSeg *>(base + kStageArenaOff + sNet->zoneArenaBytes);
+#pragma unroll 1
 	for (uint32_t k = tid; k < sNet->numZoneSegs; k += nThr)
 		*reinterpret_cast<uint8_t **>(reinterpret_cast<char *>(sNet) + segs[k].fieldOff) =
 			base + kStageArenaOff + segs[k].smemOff;
@@ -1337,6 +1368,7 @@ __device__ void stageInputs(const DevNet *N, uint64_t t, uint8_t *dyn, ZoneIn &i
 	const uint32_t *mfW = N->mfBits + (size_t)stepMod(t - 1, N->mfRing) * N->mfWords;
 	// small pieces as 4-byte words: table, MF bits, BC counts, SC counts
 	const uint32_t e0 = 64, e1 = e0 + N->mfWords, e2 = e1 + N->numBC, e3 = e2 + N->numSC;
+#pragma unroll 1
 	for (uint32_t w = tid; w < e3; w += nThr) {
 		const void *src;
 		uint8_t *dst;
@@ -1363,18 +1395,22 @@ __device__ void stageInputs(const DevNet *N, uint64_t t, uint8_t *dyn, ZoneIn &i
 	// the PF->PC input sums of every zone when the GR pass made them, else
 	// the partial sums: 16-byte pieces when the slot is 16-byte aligned
 	// (numPC * bs a multiple of 4), else words
+#pragma unroll 1
 	for (uint32_t z = 0; z < Z; z++) {
 		if (N->pcSumMode) {
 			const float *src = N->zones[z].pcSum + (size_t)R * numPC;
 			uint8_t *dst = dyn + L.pc + 4ull * z * numPC;
+#pragma unroll 1
 			for (uint32_t w = tid; w < numPC; w += nThr) cpAsync4(dst + 4 * w, src + w);
 			continue;
 		}
 		const float *src = N->zones[z].pcPartial + (size_t)R * nPC;
 		uint8_t *dst = dyn + L.pc + 4ull * z * nPC;
 		if ((nPC & 3u) == 0)
+#pragma unroll 1
 			for (uint32_t w = 4 * tid; w < nPC; w += 4 * nThr) cpAsync16(dst + 4 * w, src + w);
 		else
+#pragma unroll 1
 			for (uint32_t w = tid; w < nPC; w += nThr) cpAsync4(dst + 4 * w, src + w);
 	}
 	cpAsyncWaitAll();
@@ -1382,6 +1418,7 @@ __device__ void stageInputs(const DevNet *N, uint64_t t, uint8_t *dyn, ZoneIn &i
 		in.mf = reinterpret_cast<const uint32_t *>(dyn + L.mf);
 		in.bcSum = reinterpret_cast<const uint32_t *>(dyn + L.bc);
 		in.scSum = reinterpret_cast<const uint32_t *>(dyn + L.sc);
+#pragma unroll 1
 		for (uint32_t z = 0; z < kMaxZones; z++) {
 			in.pcPart[z] = reinterpret_cast<const float *>(dyn + L.pc) + (size_t)(z < Z ? z : 0) * nPC;
 			in.pcSum[z] = N->pcSumMode ? reinterpret_cast<const float *>(dyn + L.pc) + (size_t)(z < Z ? z : 0) * numPC
@@ -1399,6 +1436,7 @@ __device__ void stageOut(const DevNet *N, const uint8_t *base, const DevNet *sNe
 	const uint32_t from = kStageArenaOff + sNet->zoneWbOff, to = kStageArenaOff + sNet->zoneArenaBytes;
 	uint4 *dst = reinterpret_cast<uint4 *>(const_cast<DevNet *>(N));
 	const uint4 *src = reinterpret_cast<const uint4 *>(base);
+#pragma unroll 1
 	for (uint32_t i = from / 16u + threadIdx.x; i < to / 16u; i += blockDim.x) dst[i] = src[i];
 }
 
@@ -1444,6 +1482,7 @@ __device__ void protocolPrepare(const DevNet *__restrict__ N, uint64_t t)
 	uint32_t *bits = const_cast<uint32_t *>(N->mfBits) + (size_t)stepMod(t, N->mfRing) * N->mfWords;
 	const uint64_t ctr = (t + 1) << 20;
 	const uint32_t numMF = N->numMF, words = N->mfWords;
+#pragma unroll 1
 	for (uint32_t base = 0; base < 32u * words; base += blockDim.x) {
 		const uint32_t i = base + threadIdx.x;
 		uint32_t ap = 0;
@@ -1523,6 +1562,7 @@ __device__ void protocolRecordWarp(const DevNet *__restrict__ N, uint64_t t, uin
 		float *const eyeG = P->eyeG, *const eyeVm = P->eyeVm, *const eyelid = P->eyelid;
 		const float vm0 = lane == 0 ? *eyeVm : 0.0f;
 		float gSum = 0;
+#pragma unroll 1
 		for (uint32_t i0 = 0; i0 < numNC; i0 += 32) {
 			const uint32_t i = i0 + lane;
 			float g = 0;
@@ -1533,6 +1573,7 @@ __device__ void protocolRecordWarp(const DevNet *__restrict__ N, uint64_t t, uin
 				eyeG[i] = g;
 			}
 			const uint32_t n = min(32u, numNC - i0);
+#pragma unroll 1
 			for (uint32_t q = 0; q < n; q++) gSum += __shfl_sync(0xffffffffu, g, q);
 		}
 		if (lane == 0) {
@@ -1547,6 +1588,7 @@ __device__ void protocolRecordWarp(const DevNet *__restrict__ N, uint64_t t, uin
 	if (rec) {
 		const uint32_t bin = (uint32_t)ct / binSteps;
 		uint32_t *const ncPSH = P->ncPSH, *const pcPSH = P->pcPSH;
+#pragma unroll 1
 		for (uint32_t i = lane; i < numNC + numPC; i += 32) {
 			if (i < numNC) ncPSH[((size_t)dt * nBins + bin) * numNC + i] += Q.apNC[i];
 			else pcPSH[((size_t)dt * nBins + bin) * numPC + (i - numNC)] += Q.apPC[i - numNC];
@@ -1705,8 +1747,10 @@ __global__ void __launch_bounds__(kTailThreads) protocolPrimeKernel(const DevNet
 __device__ void publishNC(const DevNet *N, uint64_t t, uint8_t *box)
 {
 	const uint32_t numNC = N->numNC;
+#pragma unroll 1
 	for (uint32_t z = 0; z < N->numZones; z++) {
 		const uint8_t *ap = N->zones[z].apNC;
+#pragma unroll 1
 		for (uint32_t i = 0; i < numNC; i++) box[8 + z * numNC + i] = ap[i];
 	}
 	__threadfence_system();
@@ -1718,6 +1762,15 @@ __device__ void publishNC(const DevNet *N, uint64_t t, uint8_t *box)
 // role runs on shared-memory copies of its arrays and inputs when they fit
 // (one bulk copy in and one out per step instead of a global round trip per
 // phase).
+// Bound by latency, a good part of it the fetching of instructions: every piece of
+// the code runs once a step, on a few iterations at most, and what an SM's
+// instruction cache (about 128 KB) still holds from the last step depends on this
+// kernel's and the GR pass's code together.  So the loops of both roles are rolled
+// but where several loads have to be in flight: unrolled by the compiler, the code
+// was a third larger, and beside the event-driven pass's 75 KB each step fetched it
+// from L2, or from DRAM after an L2 flush: a flushed step took 24.0 us on 16K and
+// 64K GR and 25.5 on 1M, so 19.5, 18.7 and 22.8; back to back 11.8 on 16K and 12.7
+// on 1M, so 11.0 and 12.3.
 __global__ void __launch_bounds__(kTailThreads, 1) tailKernel(const DevNet *const *nets, const uint32_t *stageBytes,
 		uint32_t stepOffset, const DevNet *net0, uint32_t stage0, uint8_t *ncMailbox, const __grid_constant__ MFParam mfp)
 {
@@ -1757,6 +1810,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) tailKernel(const DevNet *cons
 			uint64_t *sExp2 = reinterpret_cast<uint64_t *>(tailSmem);
 			uint32_t *sMF = tailSmem + 64;
 			const uint32_t *mfW = mfp.n ? mfp.w : N->mfBits + (size_t)stepMod(t - 1, N->mfRing) * N->mfWords;
+#pragma unroll 1
 			for (uint32_t i = threadIdx.x; i < N->mfWords; i += blockDim.x) sMF[i] = mfW[i];
 			if (threadIdx.x < 32) sExp2[threadIdx.x] = kExp2Tab[threadIdx.x];
 			const uint32_t R = (uint32_t)((t + 1) % 3);
@@ -1764,6 +1818,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) tailKernel(const DevNet *cons
 				in.mf = sMF;
 				in.bcSum = N->bcCount + (size_t)R * N->numBC;
 				in.scSum = N->scCount + (size_t)R * N->numSC;
+#pragma unroll 1
 				for (uint32_t z = 0; z < kMaxZones; z++) {
 					const DevZone &Q = N->zones[z < N->numZones ? z : 0];
 					in.pcPart[z] = Q.pcPartial + (size_t)R * N->numPC * N->bs;
@@ -1781,6 +1836,7 @@ __global__ void __launch_bounds__(kTailThreads, 1) tailKernel(const DevNet *cons
 		if (mfp.n) {
 			// the launch's MF words into the ring, for the kernels after the
 			// step (this step's kernels read the launch's copy)
+#pragma unroll 1
 			for (uint32_t i = threadIdx.x; i < mfp.n; i += blockDim.x) ring[i] = mfp.w[i];
 		}
 		golgiRole(N, t, tailSmem, mfp.n ? mfp.w : ring);
