@@ -63,6 +63,10 @@ constexpr uint32_t kOutMore = 0xFEu;
 // Largest tile of the per-tile pass.
 constexpr uint32_t kEvMaxTile = 16384u;
 
+// The NC mailbox's word: the step in the low bits and, of at most kMailboxNC NCs,
+// their spikes above (more NCs have a byte each behind the word).
+constexpr uint32_t kMailboxNC = 16u, kMailboxShift = 48u;
+
 // A step's MF spike words passed by value to the step's kernels (one
 // network launched a step at a time: the host packs the caller's input and
 // the launch carries it, with no copy ahead of the kernels).  n = 0: the

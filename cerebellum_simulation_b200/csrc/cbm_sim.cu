@@ -2123,19 +2123,21 @@ std::string Simulator::exportField(size_t i, Field f, uint32_t zone, void *dst, 
 		CK(cudaMallocHost((void **)&hExport_, bytes), "pinned allocation");
 		hExportBytes_ = bytes;
 	}
-	if (lastStepPublishes_ && f == F_AP_NC) {
+	if (lastStepPublishes_ && f == F_AP_NC && zone < nets_[i]->dev().numZones && bytes == nets_[i]->fieldBytes(f)) {
 		// after a single step of one network: the small-cell kernel
-		// writes the NC spikes and then the step number into mapped host
-		// memory; wait for the stamp (bounded), without a copy or a stream
+		// writes the NC spikes with or before the step number into mapped
+		// host memory; wait for the stamp (bounded), without a copy or a stream
 		// synchronisation, while the step's GR pass may still run
 		Network &n = *nets_[i];
-		const uint64_t want = n.hostT_;
+		const uint64_t want = n.hostT_, stampBits = (1ull << kMailboxShift) - 1;
+		uint64_t word = 0;
 		const volatile uint64_t *stamp = reinterpret_cast<const volatile uint64_t *>(n.hMailbox_);
-		bool seen = *stamp == want;
+		auto arrived = [&] { return ((word = *stamp) & stampBits) == want; };
+		bool seen = arrived();
 		if (!seen) {
 			const auto t0 = std::chrono::steady_clock::now();
 			for (uint32_t spin = 0; !seen; spin++) {
-				seen = *stamp == want;
+				seen = arrived();
 				if ((spin & 1023u) == 1023u &&
 						std::chrono::steady_clock::now() - t0 > std::chrono::seconds(10))
 					break;
@@ -2145,7 +2147,12 @@ std::string Simulator::exportField(size_t i, Field f, uint32_t zone, void *dst, 
 			std::atomic_thread_fence(std::memory_order_acquire);
 			if (!directCopySinceStep_) markInputSlotsFree();
 			CKS(checkDeviceErrors());
-			memcpy(dst, n.hMailbox_ + 8 + (size_t)zone * n.dev().numNC, bytes);
+			const uint32_t numNC = n.dev().numNC;
+			if (n.dev().numZones * numNC <= kMailboxNC)
+				for (uint32_t k = 0; k < numNC; k++)
+					((uint8_t *)dst)[k] = (uint8_t)((word >> (kMailboxShift + zone * numNC + k)) & 1u);
+			else
+				memcpy(dst, n.hMailbox_ + 8 + (size_t)zone * numNC, bytes);
 			return "";
 		}
 		// no stamp: the synchronising path below reports what happened
