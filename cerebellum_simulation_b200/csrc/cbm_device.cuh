@@ -32,7 +32,7 @@ constexpr uint32_t kErrPassWait = 1u;  // a GR-pass pipeline wait timed out
 // copied in boxes of 32 cells x R rows (x all slots).
 enum PassMap : int {
 	PM_V = 0, PM_GKCA, PM_THRESH, PM_GESUM, PM_GISUM, PM_APBUF,  // 4-byte state, read and rewritten
-	PM_MFIDX, PM_GOIDX, PM_OUTCON, PM_PFDELAY, PM_HIST, PM_OUTCON16, PM_W0,
+	PM_MFIDX, PM_GOIDX, PM_OUTCON, PM_PFDELAY, PM_HIST, PM_W0,
 	PM_COUNT = PM_W0 + kMaxZones
 };
 
@@ -282,7 +282,7 @@ struct DevNet {
 	const uint16_t *mfIdx;    // [nMFSlots][numGR], sentinel numMF
 	const uint16_t *goIdx;    // [nGOSlots][numGR], sentinel numGO
 	const uint32_t *outCon;   // [nOutSlots][numGR]: (GO << 8) | delay bit, kNoDelay when empty
-	const uint16_t *outCon16; // the same as 16-bit entries (kOut16None when empty), or null (> 2047 GO)
+	const uint16_t *outCon16; // the same as 16-bit entries (kOut16None when empty), or null (until the vector pass wants it)
 	// per-tile pass: a tile is evRows rows of 1 << evWdShift cells of the
 	// [numGR / bs][bs] view, evTilesX tiles side by side; evPCs PCs, evBC BC
 	// and evSC SC blocks in a tile.  While it runs, vGR, gKCaGR, threshGR, gESum,

@@ -107,6 +107,7 @@ const void *pcTreeKernelFn();
 // the MF ring for the kernels after the step.
 __global__ void tailKernel(const DevNet *const *nets, const uint32_t *stageBytes, uint32_t stepOffset,
 		const DevNet *net0, uint32_t stage0, uint8_t *ncMailbox, const __grid_constant__ MFParam mfp);
+__global__ void outCon16Kernel(const uint32_t *in, uint16_t *out, size_t n);
 __global__ void protocolPrimeKernel(const DevNet *N);
 // The records of step t = stepsDone(N) + 1 + stepOffset, after both kernels of
 // that step: ECTrialsData on the first trialBlocks blocks, a cell a thread, then

@@ -533,12 +533,19 @@ __global__ void pcTreeKernel(const DevNet *__restrict__ N, uint64_t t)
 	if (threadIdx.x == 0) N->zones[0].pcSum[(size_t)(t % 3) * numPC + pc] = sum;
 }
 
+// The GR->GO slots in 16 bits: (GO << 5) | delay bit, kOut16None when empty.
+__global__ void outCon16Kernel(const uint32_t *in, uint16_t *out, size_t n)
+{
+	for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+		out[i] = (in[i] & 0xFFu) < 32u ? (uint16_t)(((in[i] >> 8) << 5) | (in[i] & 0x1Fu)) : kOut16None;
+}
+
 const void *passVecBatchKernel() { return (const void *)&grPassVecBatchKernel; }
 
 bool passVecCapable(const DevNet &h)
 {
 	return h.nMFSlots == 4 && h.nGOSlots == 3 && h.nOutSlots == 4 && h.numZones == 1 && h.bs >= 64 && h.bs % 64 == 0 && h.numGR % 128 == 0 &&
-		(1u << h.bcShift) >= 64u && (1u << h.scShift) >= 64u && h.outCon16 &&
+		(1u << h.bcShift) >= 64u && (1u << h.scShift) >= 64u && h.numGO <= kOut16MaxGO &&
 		h.P % (2 * h.bs) == 0;
 }
 

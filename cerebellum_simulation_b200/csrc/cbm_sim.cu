@@ -323,6 +323,26 @@ std::string Network::takeEventPass(EventTables *o, cudaStream_t s)
 	return "";
 }
 
+// What only the vector and the persistent pass use: the PF->PC pair sums and, for
+// the vector pass, the 16-bit GR->GO table.  Made when one of them is first picked:
+// with them, every network took 12 bytes a GR more, and creating one a tenth longer.
+std::string Network::planVecPass(bool out16, cudaStream_t s)
+{
+	for (uint32_t z = 0; z < h_.numZones; z++) {
+		if (!h_.zones[z].pairSum) h_.zones[z].pairSum = alloc<float>((size_t)2 * h_.numPC * h_.K * h_.bs);
+		if (!h_.zones[z].pairSum) return "device allocation failed";
+	}
+	if (out16 && !h_.outCon16) {
+		const size_t n = (size_t)std::max(1u, h_.nOutSlots) * h_.numGR;
+		uint16_t *o = alloc<uint16_t>(n, false);
+		if (!o) return "device allocation failed";
+		outCon16Kernel<<<1184, 256, 0, s>>>(h_.outCon, o, n);
+		CK(cudaGetLastError(), "vector-pass tables");
+		h_.outCon16 = o;
+	}
+	return uploadDesc();
+}
+
 // Device scratch of 8 bytes a GR, kept for the network's life (reordering and
 // exports, one at a time in the stream's order).
 std::string Network::scratch(void **p)
@@ -744,14 +764,7 @@ std::string Network::build(State *st, const std::vector<int> &seeds, uint32_t mf
 	h.mfIdx = upload(mfIdx.data(), mfIdx.size());
 	h.goIdx = upload(goIdx.data(), goIdx.size());
 	h.outCon = upload(outCon.data(), outCon.size());
-	h.outCon16 = nullptr;
-	if (c.numGO <= kOut16MaxGO) {
-		// the 16-bit copy the vector pass reads
-		std::vector<uint16_t> out16(outCon.size(), kOut16None);
-		for (size_t i = 0; i < outCon.size(); i++)
-			if ((outCon[i] & 0xFFu) < 32u) out16[i] = (uint16_t)(((outCon[i] >> 8) << 5) | (outCon[i] & 0x1Fu));
-		h.outCon16 = upload(out16.data(), out16.size());
-	}
+	h.outCon16 = nullptr;  // planVecPass
 	h.pfDelay = upload(pfDelay.data(), pfDelay.size());
 
 	auto upF = [&](const char *n, int z = -1) { NamedArray *x = A(n, z); return upload(x->as<float>(), x->count); };
@@ -827,7 +840,7 @@ std::string Network::build(State *st, const std::vector<int> &seeds, uint32_t mf
 		DevZone &Q = h.zones[z];
 		Q.w = upF("pfSynWeightPC", z);
 		Q.pcPartial = alloc<float>((size_t)3 * c.numPC * h.bs);
-		Q.pairSum = alloc<float>((size_t)2 * c.numPC * h.K * h.bs);
+		Q.pairSum = nullptr;  // planVecPass
 		Q.pcSum = alloc<float>((size_t)3 * c.numPC);
 		Q.plastSel = alloc<uint8_t>((size_t)2 * c.numIO);
 		std::vector<uint32_t> ioOfPC(c.numPC);
@@ -1629,6 +1642,7 @@ std::string Simulator::planPass(const PassGeometry &g, PassPlan *p)
 	if (g.kind == 3) {
 		for (Network *n : nets_)
 			if (!passVecCapable(n->dev())) return "the vector GR pass runs networks of its compiled shape";
+		for (Network *n : nets_) CKS(n->planVecPass(true, s0_));
 		p->W = kVecWarps - 1;
 		p->threads = 32u * kVecWarps;
 		uint32_t claim = kVecBatchClaim, units = 0, sms = (uint32_t)numSMs;
@@ -1691,6 +1705,7 @@ std::string Simulator::planPass(const PassGeometry &g, PassPlan *p)
 		if (!p->fn) return "persistent GR-pass geometry not compiled in";
 		p->R = (uint32_t)(2 * g.W);
 		if (p->R > minRows) return "more rows per unit than a tile has";
+		CKS(n.planVecPass(false, s0_));
 		const PassLayout L = passLayout(p->R, n.dev().nMFSlots, n.dev().nGOSlots, n.dev().nOutSlots, n.dev().numZones);
 		p->smem = 128 + (size_t)g.S * L.bytes + 16ull * g.S + 4ull * n.dev().numPC * n.dev().numZones +
 			32ull * (n.dev().mfWords + n.dev().goWords);

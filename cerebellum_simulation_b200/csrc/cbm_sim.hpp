@@ -268,6 +268,7 @@ public:
 	std::string planEventPass(uint32_t target, uint32_t SC, EventTables *o, cudaStream_t s);
 	std::string takeEventPass(EventTables *o, cudaStream_t s);
 	void dropEventPass(EventTables *o);
+	std::string planVecPass(bool out16, cudaStream_t s);
 	// Enter or leave the per-tile pass's form of the state: GR->GO counts
 	// delivered when cells spike instead of when the spikes arrive, the
 	// conductances one step behind with the arrived spikes beside them, and the
