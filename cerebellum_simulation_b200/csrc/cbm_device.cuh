@@ -47,15 +47,13 @@ constexpr uint32_t kOutInline = 4u;
 // Steps in the ring of GR->GO counts: a spike of step t reaches slots t ..
 // t + 31, while the small-cell update of step t reads and clears slot t - 1.
 constexpr uint32_t kGoRing = 64u;
-// Cells of a block of the event lists, an unused entry of a list (a dummy counter
-// behind the block's), an unused item, the items an event CTA lists at a time and
-// its shared memory, and the spiking cells a streaming
-// CTA lists at a time.
-constexpr uint32_t kEvCells = 16384u;
-constexpr uint32_t kEvUnused = kEvCells;
+// Cells of a block of the event lists (a power of two in this range, DevNet::evCells),
+// an unused item, the items an event CTA lists at a time, its shared memory with
+// such blocks, and the spiking cells a streaming CTA lists at a time.
+constexpr uint32_t kEvMinCells = 2048u, kEvMaxCells = 16384u;
 constexpr uint32_t kEvNone = 0xFFFFFFFFu;
 constexpr uint32_t kEvListCap = 1024u;
-constexpr uint32_t kEvRoleBytes = 128u + 16u + kEvCells + 16u + 4u * kEvListCap;
+CBM_LAYOUT_FN uint32_t eventRoleBytes(uint32_t cells) { return 128u + 16u + cells + 16u + 4u * kEvListCap; }
 constexpr uint32_t kEvCellCap = 256u;
 // Delay field of the last entry of a cell's GR->GO row whose synapses go on in
 // another one.
@@ -289,10 +287,11 @@ struct DevNet {
 	// gISum, apBufGR, historyGR and the zones' w are in tile order (tile by tile,
 	// row by row), as the arrays below always are
 	uint32_t evWdShift, evRows, evTilesX, evTiles, evPCs, evBC, evSC;
+	uint32_t evCells;           // cells of an event block
 	uint32_t evPerMF, evPerGO;  // items of 64 cells a usual list is cut into
 	// block b's target cells of source s (MF, then GO), by eights (u16):
 	// evEntry[evStart[b (numMF + numGO + 1) + s] .. evStart[.. + s + 1]),
-	// padded with kEvUnused
+	// padded with evCells (a dummy counter behind the block's)
 	const uint32_t *evStart;
 	const uint4 *evEntry;
 	// a cell's GR->GO synapses, four a row as outCon's entries; a row whose last

@@ -5,7 +5,7 @@
 // PF delay, the arrived spikes), but its synapses matter only when a spike
 // arrives: about 1 % of the MF, 1-12 % of the GO and 0.1-3 % of the GR spike
 // in a step.  So the synapse tables are not streamed.  They are kept by source:
-//   MF->GR and GO->GR: per block of kEvCells cells, each source's list of
+//   MF->GR and GO->GR: per block of evCells cells, each source's list of
 //     target cells (evStart, evEntry).  An event CTA walks the lists of the
 //     step's spiking sources and counts into half a byte per cell and kind in
 //     shared memory; the counts are the integers the per-cell gather of
@@ -88,7 +88,7 @@ __device__ __forceinline__ void countCells(uint8_t *sCnt, const uint4 &e, uint32
 }
 
 // Event CTA `block` of network N in step t: the spikes that arrive at cells
-// [block kEvCells, + kEvCells) in this step.  Bound by latency (spike words,
+// [block evCells, + evCells) in this step.  Bound by latency (spike words,
 // list starts, lists are dependent round trips of 1-1.5 us beside the streaming
 // CTAs) and by the instructions of a few warps (about six a counted cell): so
 // the lists of a usual step are taken in one round, eight lanes and 64 cells an
@@ -98,15 +98,16 @@ __device__ void eventRole(const DevNet *__restrict__ N, uint64_t t, uint32_t blo
 	constexpr uint32_t U = 10;
 	const uint32_t tid = threadIdx.x, nThr = blockDim.x, lane = tid & 31u;
 	uint32_t *ctr = reinterpret_cast<uint32_t *>(smem);          // items
-	uint8_t *sCnt = smem + 16;                                   // [kEvCells]: MF count | GO count << 4; a dummy
-	uint32_t *sItem = reinterpret_cast<uint32_t *>(sCnt + kEvCells + 16);  // [kEvListCap] source | item << 20
+	const uint32_t evCells = N->evCells;
+	uint8_t *sCnt = smem + 16;                                   // [evCells]: MF count | GO count << 4; a dummy
+	uint32_t *sItem = reinterpret_cast<uint32_t *>(sCnt + evCells + 16);  // [kEvListCap] source | item << 20
 	const uint32_t numMF = N->numMF, numGO = N->numGO, numGR = N->numGR;
 	const uint32_t mfWords = N->mfWords, nWords = mfWords + N->goWords;
 	const uint32_t *mfSrc = N->mfBits + (size_t)stepMod(t - 1, N->mfRing) * mfWords;
 	const uint32_t *goSrc = N->goBits + (size_t)((t - 1) & 1) * N->goWords;
 	const uint32_t *const start = N->evStart + (size_t)block * (numMF + numGO + 1u);
 	const uint4 *const entry = N->evEntry;
-	const uint32_t cells = min(kEvCells, numGR - block * kEvCells), perMF = N->evPerMF, perGO = N->evPerGO;
+	const uint32_t cells = min(evCells, numGR - block * evCells), perMF = N->evPerMF, perGO = N->evPerGO;
 	for (uint32_t w0 = 0; w0 < nWords; w0 += nThr) {
 		// a thread a word; MF words come from the launch when it carries them
 		const uint32_t w = w0 + tid;
@@ -117,7 +118,7 @@ __device__ void eventRole(const DevNet *__restrict__ N, uint64_t t, uint32_t blo
 		if (w < nWords && xs - x0 < 32u) word &= (1u << (xs - x0)) - 1u;
 		if (tid == 0) *ctr = 0;
 		if (w0 == 0)
-			for (uint32_t i = tid; i < kEvCells / 16u + 1u; i += nThr) reinterpret_cast<uint4 *>(sCnt)[i] = make_uint4(0, 0, 0, 0);
+			for (uint32_t i = tid; i < evCells / 16u + 1u; i += nThr) reinterpret_cast<uint4 *>(sCnt)[i] = make_uint4(0, 0, 0, 0);
 		__syncthreads();
 		for (;;) {
 			const uint32_t mine = per * (uint32_t)__popc(word);
@@ -179,7 +180,7 @@ __device__ void eventRole(const DevNet *__restrict__ N, uint64_t t, uint32_t blo
 		}
 	}
 	// the counts, for the next pass
-	uint4 *const out = reinterpret_cast<uint4 *>(N->evCnt + (size_t)(t & 1) * numGR + (size_t)block * kEvCells);
+	uint4 *const out = reinterpret_cast<uint4 *>(N->evCnt + (size_t)(t & 1) * numGR + (size_t)block * evCells);
 	for (uint32_t i = tid; i < cells / 16u; i += nThr) out[i] = reinterpret_cast<const uint4 *>(sCnt)[i];
 }
 
@@ -620,7 +621,7 @@ __global__ void evCountKernel(const DevNet *N, uint32_t *cnt)
 {
 	const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
 	if (g >= N->numGR) return;
-	uint32_t *c = cnt + (size_t)(evIndex(N, g) / kEvCells) * (N->numMF + N->numGO + 1u);
+	uint32_t *c = cnt + (size_t)(evIndex(N, g) / N->evCells) * (N->numMF + N->numGO + 1u);
 	for (uint32_t s = 0; s < N->nMFSlots; s++) {
 		const uint32_t i = N->mfIdx[(size_t)s * N->numGR + g];
 		if (i < N->numMF) atomicAdd(&c[i], 1u);
@@ -676,14 +677,14 @@ __global__ void evFillKernel(const DevNet *N, uint32_t *next, uint16_t *entry)
 	const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
 	if (g >= N->numGR) return;
 	const uint32_t p = evIndex(N, g);
-	uint32_t *c = next + (size_t)(p / kEvCells) * (N->numMF + N->numGO + 1u);
+	uint32_t *c = next + (size_t)(p / N->evCells) * (N->numMF + N->numGO + 1u);
 	for (uint32_t s = 0; s < N->nMFSlots; s++) {
 		const uint32_t i = N->mfIdx[(size_t)s * N->numGR + g];
-		if (i < N->numMF) entry[atomicAdd(&c[i], 1u)] = (uint16_t)(p % kEvCells);
+		if (i < N->numMF) entry[atomicAdd(&c[i], 1u)] = (uint16_t)(p % N->evCells);
 	}
 	for (uint32_t s = 0; s < N->nGOSlots; s++) {
 		const uint32_t i = N->goIdx[(size_t)s * N->numGR + g];
-		if (i < N->numGO) entry[atomicAdd(&c[N->numMF + i], 1u)] = (uint16_t)(p % kEvCells);
+		if (i < N->numGO) entry[atomicAdd(&c[N->numMF + i], 1u)] = (uint16_t)(p % N->evCells);
 	}
 }
 

@@ -94,8 +94,10 @@ size_t Network::passSmemBytes() const
 		sizeof(float) * (size_t)h_.numZones * 2 * h_.K * h_.J;
 }
 
-bool Network::eventTiling(uint32_t target, uint32_t SC, DevNet *o) const
+bool Network::eventTiling(const EventGrain &grain, uint32_t SC, DevNet *o) const
 {
+	const uint32_t target = std::max(grain.tile, SC);
+	o->evCells = grain.block;
 	// Sources are numbered in 16 bits, arriving spikes counted in 4 a cell and kind.
 	if (h_.J != 32 || h_.numMF + h_.numGO > 65535u || h_.nMFSlots > 15u || h_.nGOSlots > 15u) return false;
 	// One PC's rows of 32 cells are the narrowest tile; smaller ones widen up
@@ -121,7 +123,7 @@ bool Network::eventTiling(uint32_t target, uint32_t SC, DevNet *o) const
 size_t Network::eventSmemBytes(const DevNet &h, uint32_t SC, uint32_t S)
 {
 	const uint32_t TC = h.evRows << h.evWdShift;
-	return std::max<size_t>(kEvRoleBytes, 128 + eventSmem(std::min(S, TC / SC), eventLayout(SC, h.numZones).bytes, TC,
+	return std::max<size_t>(eventRoleBytes(h.evCells), 128 + eventSmem(std::min(S, TC / SC), eventLayout(SC, h.numZones).bytes, TC,
 			h.numZones, h.evPCs, h.evBC + h.evSC).bytes);
 }
 
@@ -195,19 +197,19 @@ std::string Network::buildPassMaps(uint32_t R)
 	return uploadDesc();
 }
 
-// The per-tile pass's tables in the tiling for `target` and SC, on the device from
+// The per-tile pass's tables in the tiling for a grain and SC, on the device from
 // the slot tables, beside those in use (which may serve: o->fresh says); nothing
 // that the pass in use reads is touched.
-std::string Network::planEventPass(uint32_t target, uint32_t SC, EventTables *o, cudaStream_t s)
+std::string Network::planEventPass(const EventGrain &grain, uint32_t SC, EventTables *o, cudaStream_t s)
 {
 	o->net = h_;
 	DevNet &d = o->net;
-	if (!eventTiling(target, SC, &d)) return "no tiling of the per-tile GR pass covers the cells";
+	if (!eventTiling(grain, SC, &d)) return "no tiling of the per-tile GR pass covers the cells";
 	void *tmp = nullptr;
 	if (d.evTilesX > 1) CKS(scratch(&tmp));  // taking the tables reorders the arrays through it
-	o->fresh = !h_.evStart || h_.evRows != d.evRows || h_.evWdShift != d.evWdShift;
+	o->fresh = !h_.evStart || h_.evRows != d.evRows || h_.evWdShift != d.evWdShift || h_.evCells != d.evCells;
 	if (!o->fresh) return "";
-	const uint32_t N = h_.numGR, nSrc = h_.numMF + h_.numGO, blocks = eventBlocks(), grid = (N + 255) / 256;
+	const uint32_t N = h_.numGR, nSrc = h_.numMF + h_.numGO, blocks = eventBlocks(d), grid = (N + 255) / 256;
 	const size_t nStart = (size_t)blocks * (nSrc + 1);
 	// one allocation for what is sized now, one for the lists, one that goes again
 	uint8_t *base = nullptr;
@@ -270,7 +272,7 @@ std::string Network::planEventPass(uint32_t target, uint32_t SC, EventTables *o,
 	o->arena[1] = base = alloc<uint8_t>(bytes, false);
 	if (!base) return "device allocation failed";
 	lists();
-	evUnusedKernel<<<1184, 256, 0, s>>>((uint32_t *)entry, 4 * total, kEvUnused | (kEvUnused << 16));
+	evUnusedKernel<<<1184, 256, 0, s>>>((uint32_t *)entry, 4 * total, d.evCells | (d.evCells << 16));
 	CK(cudaMemcpyAsync(blockBase, hb.data(), 4ull * blocks, cudaMemcpyHostToDevice, s), "event tables");
 	evBaseKernel<<<blocks, 256, 0, s>>>(start, next, blockBase, nSrc);
 	evFillKernel<<<grid, 256, 0, s>>>(desc, next, entry);
@@ -280,7 +282,7 @@ std::string Network::planEventPass(uint32_t target, uint32_t SC, EventTables *o,
 	CK(cudaStreamSynchronize(s), "event tables");
 	// items of 64 cells for a usual list (its mean and two deviations)
 	auto items = [&](uint32_t slots, uint32_t sources) {
-		const double mean = (double)std::min(N, kEvCells) * slots / sources;
+		const double mean = (double)std::min(N, d.evCells) * slots / sources;
 		return std::min(16u, std::max(1u, (uint32_t)std::ceil((mean + 2 * std::sqrt(mean)) / 64)));
 	};
 	d.evPerMF = items(h_.nMFSlots, h_.numMF);
@@ -311,6 +313,7 @@ std::string Network::takeEventPass(EventTables *o, cudaStream_t s)
 		CKS(setEventMode(false, s));
 		const DevNet &d = o->net;
 		h_.evWdShift = d.evWdShift; h_.evRows = d.evRows; h_.evTilesX = d.evTilesX; h_.evTiles = d.evTiles;
+		h_.evCells = d.evCells;
 		h_.evPCs = d.evPCs; h_.evBC = d.evBC; h_.evSC = d.evSC;
 		h_.evPerMF = d.evPerMF; h_.evPerGO = d.evPerGO;
 		h_.evStart = d.evStart; h_.evEntry = d.evEntry; h_.outCell = d.outCell; h_.outMore = d.outMore;
@@ -1538,17 +1541,22 @@ std::string Simulator::create(const std::vector<State *> &states, const std::vec
 	return first;
 }
 
-// Cells a tile of the per-tile pass should hold, a multiple of rounds of SC:
+// Cells a tile of the per-tile pass should hold (a multiple of rounds of SC):
 // 2048 (64 rows of 32 cells of the 1M-GR network: one wave of four CTAs an SM),
 // down to 512 where that leaves fewer than two tiles an SM (a single small
-// network).
-static uint32_t tileTarget(const std::vector<Network *> &nets, uint32_t SC)
+// network).  And the cells of an event block: 16,384 where that makes 64 blocks or
+// more (1M GR), down to 2048 for fewer cells, whose CTAs would be few beside idle
+// SMs.  An event CTA's time grows with the spikes that arrive (about 3 a ns): on
+// 16K GR, one CTA in all, a step with 94 % of the GOs spiking took 21 us, and 12
+// with the tables streamed; on eight CTAs it takes 12.0.
+static EventGrain eventGrain(const std::vector<Network *> &nets)
 {
 	uint64_t total = 0;
 	for (Network *n : nets) total += n->dev().numGR;
-	uint32_t target = 2048;
-	while (target > 512 && target > SC && total / target < 296) target /= 2;
-	return std::max(target, SC);
+	EventGrain g{2048, kEvMaxCells};
+	while (g.tile > 512 && total / g.tile < 296) g.tile /= 2;
+	while (g.block > kEvMinCells && total / g.block < 64) g.block /= 2;
+	return g;
 }
 
 // Stages of the per-tile pass in a geometry: its rows per warp times its
@@ -1559,11 +1567,12 @@ static uint32_t stagesOf(const PassGeometry &g) { return (uint32_t)std::min(4, g
 // memory fits; *smem receives that.
 bool Simulator::passTmaFits(const PassGeometry &g, size_t *smem) const
 {
-	const uint32_t SC = 128u * g.W, target = tileTarget(nets_, SC);
+	const uint32_t SC = 128u * g.W;
+	const EventGrain grain = eventGrain(nets_);
 	*smem = 0;
 	for (Network *n : nets_) {
 		DevNet h = n->dev();
-		if (!n->eventTiling(target, SC, &h)) return false;
+		if (!n->eventTiling(grain, SC, &h)) return false;
 		*smem = std::max(*smem, Network::eventSmemBytes(h, SC, stagesOf(g)));
 	}
 	return !nets_.empty() && *smem <= 227 * 1024;
@@ -1722,18 +1731,19 @@ std::string Simulator::planPass(const PassGeometry &g, PassPlan *p)
 	if (!p->fn) return "per-tile GR-pass geometry not compiled in";
 	if (!passTmaFits(g, &p->smem)) return "the per-tile GR-pass geometry does not fit every network";
 	CK(cudaFuncSetAttribute(p->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem), "pass smem");
-	const uint32_t SC = 128u * g.W, target = tileTarget(nets_, SC);
+	const uint32_t SC = 128u * g.W;
+	const EventGrain grain = eventGrain(nets_);
 	p->R = SC / 32u;
-	for (size_t i = 0; i < nets_.size(); i++) CKS(nets_[i]->planEventPass(target, SC, &p->events[i], s0_));
+	for (size_t i = 0; i < nets_.size(); i++) CKS(nets_[i]->planEventPass(grain, SC, &p->events[i], s0_));
 	// the event CTAs first: theirs is the longer chain of latencies
 	if (nets_.size() == 1) {
-		p->eventCTAs = nets_[0]->eventBlocks();
+		p->eventCTAs = Network::eventBlocks(p->events[0].net);
 		p->grid = p->eventCTAs + p->events[0].net.evTiles;
 		return "";
 	}
 	std::vector<PassBlock> blocks;
-	for (Network *n : nets_)
-		for (uint32_t b = 0; b < n->eventBlocks(); b++) blocks.push_back({n->devPtr(), b, 1});
+	for (size_t i = 0; i < nets_.size(); i++)
+		for (uint32_t b = 0; b < Network::eventBlocks(p->events[i].net); b++) blocks.push_back({nets_[i]->devPtr(), b, 1});
 	for (size_t i = 0; i < nets_.size(); i++)
 		for (uint32_t b = 0; b < p->events[i].net.evTiles; b++) blocks.push_back({nets_[i]->devPtr(), b, 0});
 	p->grid = (uint32_t)blocks.size();

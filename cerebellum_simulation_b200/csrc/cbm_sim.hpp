@@ -48,6 +48,11 @@ struct PassGeometry {
 	int kind = 0, W = 0, RW = 1, S = 0, B = 0, M = 0;
 };
 
+// About how many cells a tile and an event block of the per-tile pass take.
+struct EventGrain {
+	uint32_t tile, block;
+};
+
 // The per-tile pass's tables of one network in some tiling, until it takes them.
 struct EventTables {
 	DevNet net{};           // the network with the tiling and the tables
@@ -256,16 +261,15 @@ public:
 	std::string setPcSumMode(bool on, cudaStream_t s);
 	bool passTmaCapable() const { return h_.J == 32; }
 	uint32_t passRows() const { return 2 * h_.K; }
-	uint32_t eventBlocks() const { return (h_.numGR + kEvCells - 1) / kEvCells; }
+	static uint32_t eventBlocks(const DevNet &h) { return (h.numGR + h.evCells - 1) / h.evCells; }
 	// Encode the TMA descriptors for boxes of R rows and upload them.
 	std::string buildPassMaps(uint32_t R);
-	// The per-tile pass's tiling for about `target` cells a tile and stages of
-	// SC cells (false: no tiling fits), and its shared memory in that tiling
-	// with S stages.
-	bool eventTiling(uint32_t target, uint32_t SC, DevNet *h) const;
+	// The per-tile pass's tiling for a grain and stages of SC cells (false: no
+	// tiling fits), and its shared memory in that tiling with S stages.
+	bool eventTiling(const EventGrain &grain, uint32_t SC, DevNet *h) const;
 	static size_t eventSmemBytes(const DevNet &h, uint32_t SC, uint32_t S);
 	// The event tables of a tiling, taking them into use, and giving them back.
-	std::string planEventPass(uint32_t target, uint32_t SC, EventTables *o, cudaStream_t s);
+	std::string planEventPass(const EventGrain &grain, uint32_t SC, EventTables *o, cudaStream_t s);
 	std::string takeEventPass(EventTables *o, cudaStream_t s);
 	void dropEventPass(EventTables *o);
 	std::string planVecPass(bool out16, cudaStream_t s);
