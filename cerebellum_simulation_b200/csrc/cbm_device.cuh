@@ -52,8 +52,12 @@ constexpr uint32_t kGoRing = 64u;
 // such blocks, and the spiking cells a streaming CTA lists at a time.
 constexpr uint32_t kEvMinCells = 2048u, kEvMaxCells = 16384u;
 constexpr uint32_t kEvNone = 0xFFFFFFFFu;
+constexpr uint32_t kEvWideGR = 1u << 17;
 constexpr uint32_t kEvListCap = 1024u;
-CBM_LAYOUT_FN uint32_t eventRoleBytes(uint32_t cells) { return 128u + 16u + cells + 16u + 4u * kEvListCap; }
+CBM_LAYOUT_FN uint32_t eventRoleBytes(uint32_t cells, uint32_t planes)
+{
+	return 128u + 16u + planes * (cells + 16u) + 4u * kEvListCap;
+}
 constexpr uint32_t kEvCellCap = 256u;
 // Delay field of the last entry of a cell's GR->GO row whose synapses go on in
 // another one.
@@ -116,18 +120,19 @@ CBM_LAYOUT_FN PassLayout passLayout(uint32_t R, uint32_t nMF, uint32_t nGO, uint
 }
 
 // One stage of the per-tile pass: SC cells of the six state arrays (from 0),
-// then every zone's weights, the PF delays and the arrived spikes.
+// then every zone's weights, the PF delays and the arrived spikes (planes: 1, or 2
+// with a byte a kind).
 struct EventLayout {
 	uint32_t w, pfDelay, cnt, bytes;  // region offsets, stage size
 	uint32_t tx;                      // bytes the stage's copies deliver
 };
-CBM_LAYOUT_FN EventLayout eventLayout(uint32_t SC, uint32_t Z)
+CBM_LAYOUT_FN EventLayout eventLayout(uint32_t SC, uint32_t Z, uint32_t planes)
 {
 	EventLayout L;
 	L.w = 24u * SC;
 	L.pfDelay = L.w + 4u * SC * Z;
 	L.cnt = L.pfDelay + SC;
-	L.bytes = L.tx = L.cnt + SC;  // a multiple of 128
+	L.bytes = L.tx = L.cnt + planes * SC;  // a multiple of 128
 	return L;
 }
 
@@ -288,6 +293,7 @@ struct DevNet {
 	// row by row), as the arrays below always are
 	uint32_t evWdShift, evRows, evTilesX, evTiles, evPCs, evBC, evSC;
 	uint32_t evCells;           // cells of an event block
+	uint32_t evPlanes;          // 1: evCnt holds MF | GO << 4; 2: MF, then GO, a byte each (more than 15 inputs of a kind)
 	uint32_t evPerMF, evPerGO;  // items of 64 cells a usual list is cut into
 	// block b's target cells of source s (MF, then GO), by eights (u16):
 	// evEntry[evStart[b (numMF + numGO + 1) + s] .. evStart[.. + s + 1]),
@@ -300,7 +306,7 @@ struct DevNet {
 	const uint8_t *evPfDelay;  // pfDelay
 	uint32_t outNow;           // some GR->GO synapse has delay 0: spikes are delivered in their own step
 	uint32_t *spkBits;         // [2][tiles][cells / 128][4]: spikes of the step of that parity (bit i of word c: cell 4 i + c)
-	uint8_t *evCnt;            // [2][numGR] spikes that arrived in the step of that parity: MF | GO << 4
+	uint8_t *evCnt;            // [2][evPlanes][numGR] spikes that arrived in the step of that parity
 	uint64_t evFirst;          // the first step of the pass: gESum, gISum are final before it, later one step behind
 	const uint8_t *pfDelay;   // delay bit of the PF->BC/SC/PC output, kNoDelay when none
 

@@ -52,7 +52,7 @@ struct PassBlock {
 // Per-tile GR pass (cbm_pass_event.cu) with W consumer warps and S stages;
 // launched with 32 * (W + 1) threads and (blocks, event CTAs, stepOffset,
 // descriptor of a single network or null, MF words, exit counter); oneZone:
-// every network has one zone.  Returns null for a geometry that is not
+// every network has one zone and at most 15 inputs of a kind a cell.  Returns null for a geometry that is not
 // compiled in.
 const void *passTmaKernelFor(int W, int S, bool oneZone);
 // The compiled per-tile geometries, in table order.

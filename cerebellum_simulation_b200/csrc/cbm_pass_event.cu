@@ -93,14 +93,20 @@ __device__ __forceinline__ void countCells(uint8_t *sCnt, const uint4 &e, uint32
 // CTAs) and by the instructions of a few warps (about six a counted cell): so
 // the lists of a usual step are taken in one round, eight lanes and 64 cells an
 // item (a long list is several), ten items a group in flight.
-__device__ void eventRole(const DevNet *__restrict__ N, uint64_t t, uint32_t block, uint8_t *smem, const MFParam &mfp)
+// WIDE: the network may have two planes of counts.
+template <bool WIDE>
+__device__ __forceinline__ void eventRole(const DevNet *__restrict__ N, uint64_t t, uint32_t block, uint8_t *smem, const MFParam &mfp)
 {
 	constexpr uint32_t U = 10;
 	const uint32_t tid = threadIdx.x, nThr = blockDim.x, lane = tid & 31u;
 	uint32_t *ctr = reinterpret_cast<uint32_t *>(smem);          // items
 	const uint32_t evCells = N->evCells;
-	uint8_t *sCnt = smem + 16;                                   // [evCells]: MF count | GO count << 4; a dummy
-	uint32_t *sItem = reinterpret_cast<uint32_t *>(sCnt + evCells + 16);  // [kEvListCap] source | item << 20
+	const uint32_t planes = WIDE ? N->evPlanes : 1u, plane = evCells + 16u;
+	uint8_t *sCnt = smem + 16;                                   // [planes][evCells, a dummy behind]
+	uint32_t *sItem = reinterpret_cast<uint32_t *>(sCnt + planes * plane);  // [kEvListCap] source | item << 20
+	// where a GO spike counts, and as what
+	uint8_t *const sCntGO = planes == 2u ? sCnt + plane : sCnt;
+	const uint32_t incGO = planes == 2u ? 1u : 16u;
 	const uint32_t numMF = N->numMF, numGO = N->numGO, numGR = N->numGR;
 	const uint32_t mfWords = N->mfWords, nWords = mfWords + N->goWords;
 	const uint32_t *mfSrc = N->mfBits + (size_t)stepMod(t - 1, N->mfRing) * mfWords;
@@ -118,7 +124,7 @@ __device__ void eventRole(const DevNet *__restrict__ N, uint64_t t, uint32_t blo
 		if (w < nWords && xs - x0 < 32u) word &= (1u << (xs - x0)) - 1u;
 		if (tid == 0) *ctr = 0;
 		if (w0 == 0)
-			for (uint32_t i = tid; i < evCells / 16u + 1u; i += nThr) reinterpret_cast<uint4 *>(sCnt)[i] = make_uint4(0, 0, 0, 0);
+			for (uint32_t i = tid; i < planes * (plane / 16u); i += nThr) reinterpret_cast<uint4 *>(sCnt)[i] = make_uint4(0, 0, 0, 0);
 		__syncthreads();
 		for (;;) {
 			const uint32_t mine = per * (uint32_t)__popc(word);
@@ -166,11 +172,13 @@ __device__ void eventRole(const DevNet *__restrict__ N, uint64_t t, uint32_t blo
 #pragma unroll
 				for (uint32_t u = 0; u < U; u++) {
 					if (a[u] >= b[u]) continue;
-					const uint32_t inc = (gos >> u) & 1u ? 16u : 1u;
-					countCells(sCnt, e[u], inc);
+					const bool isGO = (gos >> u) & 1u;
+					const uint32_t inc = isGO ? incGO : 1u;
+					uint8_t *const cnt = WIDE && isGO ? sCntGO : sCnt;
+					countCells(cnt, e[u], inc);
 					// a list's last item takes what is left of it
 					if ((lasts >> u) & 1u)
-						for (a[u] += 8u; a[u] < b[u]; a[u] += 8u) countCells(sCnt, __ldg(entry + a[u]), inc);
+						for (a[u] += 8u; a[u] < b[u]; a[u] += 8u) countCells(cnt, __ldg(entry + a[u]), inc);
 				}
 			}
 			__syncthreads();
@@ -180,8 +188,10 @@ __device__ void eventRole(const DevNet *__restrict__ N, uint64_t t, uint32_t blo
 		}
 	}
 	// the counts, for the next pass
-	uint4 *const out = reinterpret_cast<uint4 *>(N->evCnt + (size_t)(t & 1) * numGR + (size_t)block * evCells);
-	for (uint32_t i = tid; i < cells / 16u; i += nThr) out[i] = reinterpret_cast<const uint4 *>(sCnt)[i];
+	for (uint32_t q = 0; q < planes; q++) {
+		uint4 *const out = reinterpret_cast<uint4 *>(N->evCnt + (size_t)((t & 1) * planes + q) * numGR + (size_t)block * evCells);
+		for (uint32_t i = tid; i < cells / 16u; i += nThr) out[i] = reinterpret_cast<const uint4 *>(sCnt + q * plane)[i];
+	}
 }
 
 // One warp of a streaming CTA: the GR->GO synapses of its tile's cells that
@@ -259,7 +269,7 @@ template <int c> __device__ __forceinline__ float byteFloat(uint32_t x)
 // the last step.  The launch's first CTAs take the event role: evBlocks of them
 // with one network, those marked in `blocks` in a batch.
 // Waits are bounded (kPassWaitLimitNs); a time-out sets kErrPassWait.
-// ZS: the number of zones, or 0 to read it at run time.
+// ZS: the number of zones, with one plane of counts, or 0 to read both at run time.
 template <int W, int S, int MINB, int ZS>
 __global__ void __launch_bounds__(32 * (W + 1), MINB) grPassTmaKernel(const PassBlock *blocks, uint32_t evBlocks,
 		uint32_t stepOffset, const DevNet *net0, const __grid_constant__ MFParam mfp, uint32_t *exitCount)
@@ -291,7 +301,7 @@ __global__ void __launch_bounds__(32 * (W + 1), MINB) grPassTmaKernel(const Pass
 	extern __shared__ uint8_t passSmemRaw[];
 	uint8_t *const smem = passSmemRaw + ((128u - (tma::smemAddr(passSmemRaw) & 127u)) & 127u);
 	if (events) {
-		eventRole(N, stepsDone(N) + 1 + stepOffset, tile, smem, mfp);
+		eventRole<ZS == 0>(N, stepsDone(N) + 1 + stepOffset, tile, smem, mfp);
 		if (exitCount) __syncthreads();
 		passExitWait(exitCount);
 		return;
@@ -311,7 +321,8 @@ __global__ void __launch_bounds__(32 * (W + 1), MINB) grPassTmaKernel(const Pass
 	const uint64_t t = stepsDone(N) + 1 + stepOffset;
 	const uint32_t Z = ZS ? ZS : N->numZones, rowsPC = 2u * N->K, wdShift = N->evWdShift, Wd = 1u << wdShift;
 	const uint32_t TC = N->evRows << wdShift, nStages = TC / SC;
-	const EventLayout L = eventLayout(SC, Z);
+	const uint32_t planes = ZS ? 1u : N->evPlanes;
+	const EventLayout L = eventLayout(SC, Z, planes);
 	const EventSmem M = eventSmem(min((uint32_t)S, nStages), L.bytes, TC, Z, N->evPCs, N->evBC + N->evSC);
 	float *sStep = reinterpret_cast<float *>(smem + M.step);      // [evPCs][Z] plasticity steps
 	uint32_t *sBC = reinterpret_cast<uint32_t *>(smem + M.bc);
@@ -331,7 +342,7 @@ __global__ void __launch_bounds__(32 * (W + 1), MINB) grPassTmaKernel(const Pass
 	if (warp == W) {
 		bool ok = true;
 		uint32_t issued = 0;
-		const uint8_t *const evCnt = N->evCnt + (size_t)((t - 1) & 1) * N->numGR;
+		const uint8_t *const evCnt = N->evCnt + (size_t)((t - 1) & 1) * planes * N->numGR;
 		auto issue = [&]() {  // the next stage
 			if (lane == 0) {
 				uint8_t *b = stages + (size_t)(issued % S) * L.bytes;
@@ -347,6 +358,7 @@ __global__ void __launch_bounds__(32 * (W + 1), MINB) grPassTmaKernel(const Pass
 				for (uint32_t z = 0; z < Z; z++) tma::loadBulk(b + L.w + z * 4u * SC, N->zones[z].w + c, 4u * SC, bar);
 				tma::loadBulk(b + L.pfDelay, N->evPfDelay + c, SC, bar);
 				tma::loadBulk(b + L.cnt, evCnt + c, SC, bar);
+				if (planes == 2u) tma::loadBulk(b + L.cnt + SC, evCnt + N->numGR + c, SC, bar);
 			}
 			issued++;
 		};
@@ -422,7 +434,11 @@ __global__ void __launch_bounds__(32 * (W + 1), MINB) grPassTmaKernel(const Pass
 			// updateGRInOPGPU of the last step: its MF spikes, and the GO
 			// spikes of the one before (kernels.cu:169-199)
 			if (pending) {
-				const uint32_t mf = c4 & 0x0F0F0F0Fu, go = (c4 >> 4) & 0x0F0F0F0Fu;
+				uint32_t mf = c4 & 0x0F0F0F0Fu, go = (c4 >> 4) & 0x0F0F0F0Fu;
+				if (planes == 2u) {
+					mf = c4;
+					go = *reinterpret_cast<const uint32_t *>(b + L.cnt + SC + e);
+				}
 				gE[0] = gE[0] * gDecMF + gIncMF * byteFloat<0>(mf); gI[0] = gI[0] * gDecGO + gIncGO * byteFloat<0>(go);
 				gE[1] = gE[1] * gDecMF + gIncMF * byteFloat<1>(mf); gI[1] = gI[1] * gDecGO + gIncGO * byteFloat<1>(go);
 				gE[2] = gE[2] * gDecMF + gIncMF * byteFloat<2>(mf); gI[2] = gI[2] * gDecGO + gIncGO * byteFloat<2>(go);
@@ -577,8 +593,9 @@ __global__ void conductancesKernel(const DevNet *N, uint64_t T, float *outE, flo
 {
 	const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
 	if (p >= N->numGR) return;
-	const uint32_t c = N->evCnt[(size_t)(T & 1) * N->numGR + p];
-	const int mf = (int)(c & 15u), go = (int)(c >> 4);
+	const uint8_t *cnt = N->evCnt + (size_t)(T & 1) * N->evPlanes * N->numGR + p;
+	const uint32_t c = *cnt;
+	const int mf = (int)(N->evPlanes == 2u ? c : c & 15u), go = (int)(N->evPlanes == 2u ? cnt[N->numGR] : c >> 4);
 	if (outE) outE[p] = N->gESum[p] * N->gDecMFtoGR + N->gIncMFtoGR * (mf);
 	if (outI) outI[p] = N->gISum[p] * N->gDecGOtoGR + N->gIncGOtoGR * (go);
 }

@@ -98,8 +98,13 @@ bool Network::eventTiling(const EventGrain &grain, uint32_t SC, DevNet *o) const
 {
 	const uint32_t target = std::max(grain.tile, SC);
 	o->evCells = grain.block;
-	// Sources are numbered in 16 bits, arriving spikes counted in 4 a cell and kind.
-	if (h_.J != 32 || h_.numMF + h_.numGO > 65535u || h_.nMFSlots > 15u || h_.nGOSlots > 15u) return false;
+	// Arriving spikes are counted in 4 bits a cell and kind, or in 8.  With 8, from
+	// kEvWideGR cells on: with 20 MF inputs a cell the plain pass takes 10.2 us on
+	// 16K GR, the one that streamed the tables took 11.0; on 256K 18.2 and 17.0, on
+	// 1M 72.7 and 37.9; counting, 12.1 and 15.2.
+	const uint32_t slots = std::max(h_.nMFSlots, h_.nGOSlots);
+	o->evPlanes = slots > 15u ? 2u : 1u;
+	if (h_.J != 32 || slots > 255u || (slots > 15u && h_.numGR < kEvWideGR)) return false;
 	// One PC's rows of 32 cells are the narrowest tile; smaller ones widen up
 	// to 128 cells, then take several PCs (all powers of two).  A round of SC
 	// cells has an even number of rows, so no pair of the reduction straddles two.
@@ -123,7 +128,8 @@ bool Network::eventTiling(const EventGrain &grain, uint32_t SC, DevNet *o) const
 size_t Network::eventSmemBytes(const DevNet &h, uint32_t SC, uint32_t S)
 {
 	const uint32_t TC = h.evRows << h.evWdShift;
-	return std::max<size_t>(eventRoleBytes(h.evCells), 128 + eventSmem(std::min(S, TC / SC), eventLayout(SC, h.numZones).bytes, TC,
+	return std::max<size_t>(eventRoleBytes(h.evCells, h.evPlanes), 128 + eventSmem(std::min(S, TC / SC),
+			eventLayout(SC, h.numZones, h.evPlanes).bytes, TC,
 			h.numZones, h.evPCs, h.evBC + h.evSC).bytes);
 }
 
@@ -229,7 +235,7 @@ std::string Network::planEventPass(const EventGrain &grain, uint32_t SC, EventTa
 		take(oc, N);
 		take(pd, N);
 		take(d.spkBits, 2ull * (N / 32));
-		take(d.evCnt, 2ull * N);
+		take(d.evCnt, 2ull * d.evPlanes * N);
 	};
 	auto building = [&]() {
 		bytes = 0;
@@ -313,7 +319,7 @@ std::string Network::takeEventPass(EventTables *o, cudaStream_t s)
 		CKS(setEventMode(false, s));
 		const DevNet &d = o->net;
 		h_.evWdShift = d.evWdShift; h_.evRows = d.evRows; h_.evTilesX = d.evTilesX; h_.evTiles = d.evTiles;
-		h_.evCells = d.evCells;
+		h_.evCells = d.evCells; h_.evPlanes = d.evPlanes;
 		h_.evPCs = d.evPCs; h_.evBC = d.evBC; h_.evSC = d.evSC;
 		h_.evPerMF = d.evPerMF; h_.evPerGO = d.evPerGO;
 		h_.evStart = d.evStart; h_.evEntry = d.evEntry; h_.outCell = d.outCell; h_.outMore = d.outMore;
@@ -384,7 +390,7 @@ std::string Network::setEventMode(bool on, cudaStream_t s)
 		// every arrival still to come, the last step's spikes included; the
 		// conductances are final
 		CK(cudaMemsetAsync(h_.spkBits, 0, 8ull * (h_.numGR / 32), s), "pass switch");
-		CK(cudaMemsetAsync(h_.evCnt, 0, 2ull * h_.numGR, s), "pass switch");
+		CK(cudaMemsetAsync(h_.evCnt, 0, 2ull * h_.evPlanes * h_.numGR, s), "pass switch");
 		goRingFillKernel<<<grid, 256, 0, s>>>(devPtr(), hostT_);
 		h_.evFirst = hostT_ + 1;
 	} else {
@@ -1725,8 +1731,9 @@ std::string Simulator::planPass(const PassGeometry &g, PassPlan *p)
 		p->grid = std::min<uint32_t>(units, (uint32_t)std::max(1, perSM) * (uint32_t)numSMs);
 		return "";
 	}
-	bool oneZone = true;
-	for (Network *n : nets_) oneZone = oneZone && n->dev().numZones == 1;
+	bool oneZone = true;  // and one plane of counts
+	for (Network *n : nets_)
+		oneZone = oneZone && n->dev().numZones == 1 && n->dev().nMFSlots <= 15u && n->dev().nGOSlots <= 15u;
 	p->fn = g.RW > 0 && g.S > 0 ? passTmaKernelFor(g.W, (int)stagesOf(g), oneZone) : nullptr;
 	if (!p->fn) return "per-tile GR-pass geometry not compiled in";
 	if (!passTmaFits(g, &p->smem)) return "the per-tile GR-pass geometry does not fit every network";
