@@ -54,9 +54,14 @@ constexpr uint32_t kEvMinCells = 2048u, kEvMaxCells = 16384u;
 constexpr uint32_t kEvNone = 0xFFFFFFFFu;
 constexpr uint32_t kEvWideGR = 1u << 17;
 constexpr uint32_t kEvListCap = 1024u;
-CBM_LAYOUT_FN uint32_t eventRoleBytes(uint32_t cells, uint32_t planes)
+// Words of a block's list starts (whole 16-byte pieces), and the most that an event
+// CTA copies to shared memory.
+CBM_LAYOUT_FN uint32_t eventStartWords(uint32_t sources) { return (sources + 4u) & ~3u; }
+constexpr uint32_t kEvStartCap = 6144u;
+CBM_LAYOUT_FN uint32_t eventRoleBytes(uint32_t cells, uint32_t planes, uint32_t sources)
 {
-	return 128u + 16u + planes * (cells + 16u) + 4u * kEvListCap;
+	const uint32_t starts = eventStartWords(sources);
+	return 128u + 16u + planes * (cells + 16u) + 4u * kEvListCap + (starts <= kEvStartCap ? 4u * starts : 0u);
 }
 constexpr uint32_t kEvCellCap = 256u;
 // Delay field of the last entry of a cell's GR->GO row whose synapses go on in
@@ -294,9 +299,10 @@ struct DevNet {
 	uint32_t evWdShift, evRows, evTilesX, evTiles, evPCs, evBC, evSC;
 	uint32_t evCells;           // cells of an event block
 	uint32_t evPlanes;          // 1: evCnt holds MF | GO << 4; 2: MF, then GO, a byte each (more than 15 inputs of a kind)
-	uint32_t evPerMF, evPerGO;  // items of 64 cells a usual list is cut into
+	uint32_t evLaneShift;       // 1 << evLaneShift lanes take an item of a list, eight cells each
+	uint32_t evPerMF, evPerGO;  // items a usual list is cut into
 	// block b's target cells of source s (MF, then GO), by eights (u16):
-	// evEntry[evStart[b (numMF + numGO + 1) + s] .. evStart[.. + s + 1]),
+	// evEntry[evStart[b eventStartWords + s] .. evStart[.. + s + 1]),
 	// padded with evCells (a dummy counter behind the block's)
 	const uint32_t *evStart;
 	const uint4 *evEntry;

@@ -88,16 +88,21 @@ __device__ __forceinline__ void countCells(uint8_t *sCnt, const uint4 &e, uint32
 }
 
 // Event CTA `block` of network N in step t: the spikes that arrive at cells
-// [block evCells, + evCells) in this step.  Bound by latency (spike words,
-// list starts, lists are dependent round trips of 1-1.5 us beside the streaming
-// CTAs) and by the instructions of a few warps (about six a counted cell): so
-// the lists of a usual step are taken in one round, eight lanes and 64 cells an
-// item (a long list is several), ten items a group in flight.
+// [block evCells, + evCells) in this step.  Bound by latency (spike words and
+// lists are dependent round trips of 1-1.5 us beside the streaming CTAs) and by
+// the instructions of a few warps (about six a counted cell): so the lists of a
+// usual step are taken in one round, as many lanes an item as a usual list has
+// eights of cells (up to eight; a longer list is several items), eight items a group
+// of lanes in flight (ten: 75 KB of code instead of 71, a 1M-GR step 0.2-0.4 us
+// slower).  Its time grows with the sources that spike, where streaming the tables
+// did not: with all Golgi cells spiking a step takes 10.3 us on 16K GR, 16.4 on 256K,
+// 23.5 on 1M and 103 on dense 4M (streaming: 12, 12, 13 and 81), with 20 % of them
+// 10.8, 11.4, 13.7 and 62.6 (12, 12, 15 and 83).
 // WIDE: the network may have two planes of counts.
 template <bool WIDE>
 __device__ __forceinline__ void eventRole(const DevNet *__restrict__ N, uint64_t t, uint32_t block, uint8_t *smem, const MFParam &mfp)
 {
-	constexpr uint32_t U = 10;
+	constexpr uint32_t U = 8;
 	const uint32_t tid = threadIdx.x, nThr = blockDim.x, lane = tid & 31u;
 	uint32_t *ctr = reinterpret_cast<uint32_t *>(smem);          // items
 	const uint32_t evCells = N->evCells;
@@ -111,9 +116,19 @@ __device__ __forceinline__ void eventRole(const DevNet *__restrict__ N, uint64_t
 	const uint32_t mfWords = N->mfWords, nWords = mfWords + N->goWords;
 	const uint32_t *mfSrc = N->mfBits + (size_t)stepMod(t - 1, N->mfRing) * mfWords;
 	const uint32_t *goSrc = N->goBits + (size_t)((t - 1) & 1) * N->goWords;
-	const uint32_t *const start = N->evStart + (size_t)block * (numMF + numGO + 1u);
+	const uint32_t *const start = N->evStart + (size_t)block * eventStartWords(numMF + numGO);
 	const uint4 *const entry = N->evEntry;
+	const uint32_t laneShift = N->evLaneShift, lanes = 1u << laneShift, l = tid & (lanes - 1u);
 	const uint32_t cells = min(evCells, numGR - block * evCells), perMF = N->evPerMF, perGO = N->evPerGO;
+	// the block's list starts on their way to shared memory beside the spike words
+	// (one dependent round trip less), where they are few enough
+	uint32_t *const sStart = sItem + kEvListCap;
+	const uint32_t nStart = eventStartWords(numMF + numGO);
+	const bool staged = nStart <= kEvStartCap;
+	if (staged)
+#pragma unroll 1
+		for (uint32_t i = 4u * tid; i < nStart; i += 4u * nThr)
+			asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tma::smemAddr(sStart + i)), "l"(start + i) : "memory");
 	for (uint32_t w0 = 0; w0 < nWords; w0 += nThr) {
 		// a thread a word; MF words come from the launch when it carries them
 		const uint32_t w = w0 + tid;
@@ -137,19 +152,38 @@ __device__ __forceinline__ void eventRole(const DevNet *__restrict__ N, uint64_t
 			uint32_t base = 0;
 			if (lane == 31u && at) base = atomicAdd(ctr, at);
 			at += __shfl_sync(0xffffffffu, base, 31) - mine;
-			if (at + mine <= kEvListCap) {
-				for (; word; word &= word - 1u) {
-					const uint32_t x = x0 + (uint32_t)__ffs((int)word) - 1u;
-					for (uint32_t q = 0; q < per; q++) sItem[at++] = (go ? numMF + x : x) | (q << 20);
+			const uint32_t src0 = go ? numMF + x0 : x0;
+			const bool fits = at + mine <= kEvListCap;
+			// a lane lists its word's spikes; where some word has many, the warp takes
+			// the words in turn, a lane a bit (a lane alone stores 32 times, all lanes to
+			// one bank: 10,000 cycles a round with every source spiking)
+			if (__any_sync(0xffffffffu, fits && __popc(word) > 4)) {
+				for (uint32_t pend = __ballot_sync(0xffffffffu, fits && word); pend; pend &= pend - 1u) {
+					const uint32_t k = (uint32_t)__ffs((int)pend) - 1u;
+					const uint32_t wk = __shfl_sync(0xffffffffu, word, k), sk = __shfl_sync(0xffffffffu, src0, k);
+					const uint32_t pk = __shfl_sync(0xffffffffu, per, k), ak = __shfl_sync(0xffffffffu, at, k);
+					if ((wk >> lane) & 1u) {
+						uint32_t *const o = sItem + ak + pk * (uint32_t)__popc(wk & ((1u << lane) - 1u));
+#pragma unroll 1
+						for (uint32_t q = 0; q < pk; q++) o[q] = (sk + lane) | (q << 20);
+					}
 				}
-			} else {
+				if (fits) word = 0;
+			} else if (fits) {
+#pragma unroll 1
+				for (; word; word &= word - 1u)
+#pragma unroll 1
+					for (uint32_t q = 0; q < per; q++) sItem[at++] = (src0 + (uint32_t)__ffs((int)word) - 1u) | (q << 20);
+			}
+			if (!fits) {
 				// a word whose items do not fit waits for another round (kEvListCap
 				// holds those of one word)
 				for (; at < kEvListCap; at++) sItem[at] = kEvNone;
 			}
+			if (staged) asm volatile("cp.async.wait_all;" ::: "memory");
 			const bool again = __syncthreads_or(word != 0);
 			const uint32_t n = min(*ctr, kEvListCap);
-			const uint32_t groups = nThr / 8u, grp = tid / 8u, l = tid % 8u;
+			const uint32_t groups = nThr >> laneShift, grp = tid >> laneShift;
 			for (uint32_t i0 = grp; i0 < n; i0 += U * groups) {
 				uint32_t a[U], b[U], gos = 0, lasts = 0;
 				uint4 e[U];
@@ -162,8 +196,8 @@ __device__ __forceinline__ void eventRole(const DevNet *__restrict__ N, uint64_t
 						const uint32_t src = x & 0xFFFFFu, q = x >> 20;
 						if (src >= numMF) gos |= 1u << u;
 						if (q + 1u == (src >= numMF ? perGO : perMF)) lasts |= 1u << u;
-						a[u] = __ldg(start + src) + 8u * q + l;
-						b[u] = __ldg(start + src + 1u);
+						a[u] = (staged ? sStart[src] : __ldg(start + src)) + (q << laneShift) + l;
+						b[u] = staged ? sStart[src + 1u] : __ldg(start + src + 1u);
 					}
 				}
 #pragma unroll
@@ -178,7 +212,7 @@ __device__ __forceinline__ void eventRole(const DevNet *__restrict__ N, uint64_t
 					countCells(cnt, e[u], inc);
 					// a list's last item takes what is left of it
 					if ((lasts >> u) & 1u)
-						for (a[u] += 8u; a[u] < b[u]; a[u] += 8u) countCells(cnt, __ldg(entry + a[u]), inc);
+						for (a[u] += lanes; a[u] < b[u]; a[u] += lanes) countCells(cnt, __ldg(entry + a[u]), inc);
 				}
 			}
 			__syncthreads();
@@ -638,7 +672,7 @@ __global__ void evCountKernel(const DevNet *N, uint32_t *cnt)
 {
 	const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
 	if (g >= N->numGR) return;
-	uint32_t *c = cnt + (size_t)(evIndex(N, g) / N->evCells) * (N->numMF + N->numGO + 1u);
+	uint32_t *c = cnt + (size_t)(evIndex(N, g) / N->evCells) * eventStartWords(N->numMF + N->numGO);
 	for (uint32_t s = 0; s < N->nMFSlots; s++) {
 		const uint32_t i = N->mfIdx[(size_t)s * N->numGR + g];
 		if (i < N->numMF) atomicAdd(&c[i], 1u);
@@ -655,7 +689,7 @@ __global__ void evCountKernel(const DevNet *N, uint32_t *cnt)
 __global__ void evScanKernel(uint32_t *cnt, uint32_t nSrc)
 {
 	__shared__ uint32_t part[256];
-	uint32_t *c = cnt + (size_t)blockIdx.x * (nSrc + 1u);
+	uint32_t *c = cnt + (size_t)blockIdx.x * eventStartWords(nSrc);
 	const uint32_t per = (nSrc + 255u) / 256u, from = threadIdx.x * per, to = min(nSrc, from + per);
 	uint32_t sum = 0;
 	for (uint32_t i = from; i < to; i++) sum += (c[i] + 7u) / 8u;
@@ -674,7 +708,7 @@ __global__ void evScanKernel(uint32_t *cnt, uint32_t nSrc)
 // start[block][*] += base[block], and next = the list's first entry.
 __global__ void evBaseKernel(uint32_t *start, uint32_t *next, const uint32_t *base, uint32_t nSrc)
 {
-	uint32_t *c = start + (size_t)blockIdx.x * (nSrc + 1u), *k = next + (size_t)blockIdx.x * (nSrc + 1u);
+	uint32_t *c = start + (size_t)blockIdx.x * eventStartWords(nSrc), *k = next + (size_t)blockIdx.x * eventStartWords(nSrc);
 	for (uint32_t i = threadIdx.x; i <= nSrc; i += blockDim.x) {
 		c[i] += base[blockIdx.x];
 		k[i] = 8u * c[i];
@@ -694,7 +728,7 @@ __global__ void evFillKernel(const DevNet *N, uint32_t *next, uint16_t *entry)
 	const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
 	if (g >= N->numGR) return;
 	const uint32_t p = evIndex(N, g);
-	uint32_t *c = next + (size_t)(p / N->evCells) * (N->numMF + N->numGO + 1u);
+	uint32_t *c = next + (size_t)(p / N->evCells) * eventStartWords(N->numMF + N->numGO);
 	for (uint32_t s = 0; s < N->nMFSlots; s++) {
 		const uint32_t i = N->mfIdx[(size_t)s * N->numGR + g];
 		if (i < N->numMF) entry[atomicAdd(&c[i], 1u)] = (uint16_t)(p % N->evCells);

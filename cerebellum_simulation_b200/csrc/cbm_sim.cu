@@ -128,7 +128,7 @@ bool Network::eventTiling(const EventGrain &grain, uint32_t SC, DevNet *o) const
 size_t Network::eventSmemBytes(const DevNet &h, uint32_t SC, uint32_t S)
 {
 	const uint32_t TC = h.evRows << h.evWdShift;
-	return std::max<size_t>(eventRoleBytes(h.evCells, h.evPlanes), 128 + eventSmem(std::min(S, TC / SC),
+	return std::max<size_t>(eventRoleBytes(h.evCells, h.evPlanes, h.numMF + h.numGO), 128 + eventSmem(std::min(S, TC / SC),
 			eventLayout(SC, h.numZones, h.evPlanes).bytes, TC,
 			h.numZones, h.evPCs, h.evBC + h.evSC).bytes);
 }
@@ -216,7 +216,8 @@ std::string Network::planEventPass(const EventGrain &grain, uint32_t SC, EventTa
 	o->fresh = !h_.evStart || h_.evRows != d.evRows || h_.evWdShift != d.evWdShift || h_.evCells != d.evCells;
 	if (!o->fresh) return "";
 	const uint32_t N = h_.numGR, nSrc = h_.numMF + h_.numGO, blocks = eventBlocks(d), grid = (N + 255) / 256;
-	const size_t nStart = (size_t)blocks * (nSrc + 1);
+	const uint32_t row = eventStartWords(nSrc);
+	const size_t nStart = (size_t)blocks * row;
 	// one allocation for what is sized now, one for the lists, one that goes again
 	uint8_t *base = nullptr;
 	size_t bytes = 0;
@@ -261,7 +262,7 @@ std::string Network::planEventPass(const EventGrain &grain, uint32_t SC, EventTa
 	evOutKernel<<<grid, 256, 0, s>>>(desc, nullptr, nullptr, rows);
 	std::vector<uint32_t> hb(blocks);
 	uint32_t nRows = 0;
-	CK(cudaMemcpy2DAsync(hb.data(), 4, start + nSrc, 4ull * (nSrc + 1), 4, blocks, cudaMemcpyDeviceToHost, s), "event tables");
+	CK(cudaMemcpy2DAsync(hb.data(), 4, start + nSrc, 4ull * row, 4, blocks, cudaMemcpyDeviceToHost, s), "event tables");
 	CK(cudaMemcpyAsync(&nRows, rows, 4, cudaMemcpyDeviceToHost, s), "event tables");
 	CK(cudaStreamSynchronize(s), "event tables");
 	uint64_t total = 0;
@@ -286,13 +287,17 @@ std::string Network::planEventPass(const EventGrain &grain, uint32_t SC, EventTa
 	evOrderKernel<<<grid, 256, 0, s>>>(desc, h_.pfDelay, pd, 1, 1, true);
 	CK(cudaGetLastError(), "event tables");
 	CK(cudaStreamSynchronize(s), "event tables");
-	// items of 64 cells for a usual list (its mean and two deviations)
-	auto items = [&](uint32_t slots, uint32_t sources) {
-		const double mean = (double)std::min(N, d.evCells) * slots / sources;
-		return std::min(16u, std::max(1u, (uint32_t)std::ceil((mean + 2 * std::sqrt(mean)) / 64)));
+	// the lanes that the usual list of either kind keeps busy (its mean, in eights of
+	// cells), and the items that take its mean and two deviations
+	auto mean = [&](uint32_t slots, uint32_t sources) { return (double)std::min(N, d.evCells) * slots / sources; };
+	const double mf = mean(h_.nMFSlots, h_.numMF), go = mean(h_.nGOSlots, h_.numGO);
+	d.evLaneShift = 0;
+	while (d.evLaneShift < 3 && std::max(mf, go) > 8.0 * (1u << d.evLaneShift)) d.evLaneShift++;
+	auto items = [&](double m) {
+		return std::min(16u, std::max(1u, (uint32_t)std::ceil((m + 2 * std::sqrt(m)) / (8u << d.evLaneShift))));
 	};
-	d.evPerMF = items(h_.nMFSlots, h_.numMF);
-	d.evPerGO = items(h_.nGOSlots, h_.numGO);
+	d.evPerMF = items(mf);
+	d.evPerGO = items(go);
 	d.evStart = start;
 	d.evEntry = (const uint4 *)entry;
 	d.outCell = oc;
@@ -321,7 +326,7 @@ std::string Network::takeEventPass(EventTables *o, cudaStream_t s)
 		h_.evWdShift = d.evWdShift; h_.evRows = d.evRows; h_.evTilesX = d.evTilesX; h_.evTiles = d.evTiles;
 		h_.evCells = d.evCells; h_.evPlanes = d.evPlanes;
 		h_.evPCs = d.evPCs; h_.evBC = d.evBC; h_.evSC = d.evSC;
-		h_.evPerMF = d.evPerMF; h_.evPerGO = d.evPerGO;
+		h_.evLaneShift = d.evLaneShift; h_.evPerMF = d.evPerMF; h_.evPerGO = d.evPerGO;
 		h_.evStart = d.evStart; h_.evEntry = d.evEntry; h_.outCell = d.outCell; h_.outMore = d.outMore;
 		h_.evPfDelay = d.evPfDelay; h_.spkBits = d.spkBits; h_.evCnt = d.evCnt;
 		for (int k = 0; k < 2; k++) std::swap(evArena_[k], o->arena[k]);  // the old ones go with the plan
@@ -1552,7 +1557,7 @@ std::string Simulator::create(const std::vector<State *> &states, const std::vec
 // down to 512 where that leaves fewer than two tiles an SM (a single small
 // network).  And the cells of an event block: 16,384 where that makes 64 blocks or
 // more (1M GR), down to 2048 for fewer cells, whose CTAs would be few beside idle
-// SMs.  An event CTA's time grows with the spikes that arrive (about 3 a ns): on
+// SMs.  An event CTA's time grows with the spikes that arrive (eventRole): on
 // 16K GR, one CTA in all, a step with 94 % of the GOs spiking took 21 us, and 12
 // with the tables streamed; on eight CTAs it takes 12.0.
 static EventGrain eventGrain(const std::vector<Network *> &nets)
