@@ -635,9 +635,10 @@ __global__ void conductancesKernel(const DevNet *N, uint64_t T, float *outE, flo
 }
 
 // Geometries the host can pick: (consumer warps, stages, minimum resident CTAs
-// per SM).
-#define CBM_PASS_TMA_CONFIGS(X) X(4, 2, 4) X(4, 3, 4) X(4, 4, 4) X(8, 4, 2) X(8, 3, 2) X(8, 2, 2) X(2, 4, 4) \
-	X(1, 4, 4)
+// per SM).  The first that fits is the default.  Four stages serve tiles of four
+// stages and more whose state streams from HBM, eight warps the largest tiles, two
+// and one warp tiles below 512 cells, which four cannot take.
+#define CBM_PASS_TMA_CONFIGS(X) X(4, 2, 4) X(4, 4, 4) X(8, 3, 2) X(2, 4, 4) X(1, 4, 4)
 
 int passTmaConfigCount()
 {

@@ -1468,6 +1468,30 @@ Simulator::~Simulator()
 	for (cudaEvent_t e : tailEv_) cudaEventDestroy(e);
 }
 
+// Stages that the per-tile pass runs with in a geometry: of the compiled ones for
+// its warps (cbm_pass_event.cu) those nearest its rows per warp times its stages.
+static uint32_t stagesOf(const PassGeometry &g)
+{
+	return g.W == 8 ? 3u : g.W == 4 && g.RW * g.S <= 2 ? 2u : 4u;
+}
+
+// Whether CBM_PASS_TMA may name a geometry: the tuples it has always taken (rows
+// per warp and resident CTAs among them, which the pass has no use for any more),
+// and those that the autotuner reports.
+static bool namedGeometry(const PassGeometry &g)
+{
+	static const int known[][5] = {{8, 1, 3, 2, 4}, {8, 1, 3, 3, 4}, {8, 1, 4, 2, 4}, {8, 1, 2, 3, 4}, {4, 1, 4, 4, 4},
+		{4, 2, 3, 3, 4}, {4, 2, 4, 2, 4}, {4, 2, 2, 4, 4}, {8, 1, 3, 2, 0}, {4, 1, 4, 1, 0}, {2, 1, 4, 1, 0}, {1, 1, 4, 1, 0}};
+	for (const int *k : known)
+		if (g.W == k[0] && g.RW == k[1] && g.S == k[2] && g.B == k[3] && g.M == k[4]) return true;
+	for (int i = 0; i < passTmaConfigCount(); i++) {
+		int W, S, B;
+		passTmaConfig(i, &W, &S, &B);
+		if (g.W == W && g.RW == 1 && g.S == S && g.B == B && (g.M == 0 || g.M == 4)) return true;
+	}
+	return false;
+}
+
 std::string Simulator::create(const std::vector<State *> &states, const std::vector<std::vector<int>> &seeds,
 		int device, uint32_t mfRing, const std::vector<uint32_t> *mfSeeds)
 {
@@ -1538,6 +1562,15 @@ std::string Simulator::create(const std::vector<State *> &states, const std::vec
 		if (!strcmp(env, "0")) { g.kind = 0; return usePassGeometry(g); }
 		g.kind = 1;
 		if (sscanf(env, "%d,%d,%d,%d,%d", &g.W, &g.RW, &g.S, &g.B, &g.M) != 5) return "CBM_PASS_TMA must be W,RW,S,B,M";
+		if (!namedGeometry(g)) return "per-tile GR-pass geometry not compiled in";
+		// bounds of the slot loops and tiles that the named geometries had; the pass
+		// keeps to them
+		for (Network *n : nets_) {
+			const DevNet &h = n->dev();
+			if (g.M > 0 && std::max({h.nMFSlots, h.nGOSlots, std::min(h.nOutSlots, kOutInline)}) > (uint32_t)g.M)
+				return "a network has more synapse slots than the geometry's slot bound";
+			if ((uint32_t)(g.W * g.RW) > n->passRows()) return "more rows per stage than a tile has";
+		}
 		return usePassGeometry(g);
 	}
 	// the default; where its tables do not fit in memory, or do not cover the network,
@@ -1559,7 +1592,7 @@ std::string Simulator::create(const std::vector<State *> &states, const std::vec
 // more (1M GR), down to 2048 for fewer cells, whose CTAs would be few beside idle
 // SMs.  An event CTA's time grows with the spikes that arrive (eventRole): on
 // 16K GR, one CTA in all, a step with 94 % of the GOs spiking took 21 us, and 12
-// with the tables streamed; on eight CTAs it takes 12.0.
+// with the tables streamed; on eight CTAs it takes 10.2.
 static EventGrain eventGrain(const std::vector<Network *> &nets)
 {
 	uint64_t total = 0;
@@ -1569,10 +1602,6 @@ static EventGrain eventGrain(const std::vector<Network *> &nets)
 	while (g.block > kEvMinCells && total / g.block < 64) g.block /= 2;
 	return g;
 }
-
-// Stages of the per-tile pass in a geometry: its rows per warp times its
-// stages, in the compiled range.
-static uint32_t stagesOf(const PassGeometry &g) { return (uint32_t)std::min(4, g.RW * g.S); }
 
 // Whether every network has a tiling for the geometry and its CTA's shared
 // memory fits; *smem receives that.
@@ -1711,11 +1740,11 @@ std::string Simulator::planPass(const PassGeometry &g, PassPlan *p)
 		return "";
 	}
 	if (!capable) return "the TMA GR pass needs tiles of 32-cell rows in every network";
-	// (the per-tile pass has no slot loops: M is accepted and has no effect)
+	// (the per-tile pass has no slot loops)
 	if (g.kind != 1 && g.M > 0 && maxSlots > (uint32_t)g.M)
 		return "a network has more synapse slots than the geometry's slot bound";
 	p->W = (uint32_t)g.W;
-	p->S = (uint32_t)g.S;
+	p->S = g.kind == 1 ? stagesOf(g) : (uint32_t)g.S;
 	p->threads = 32u * (g.W + 1);
 	if (g.kind == 2) {
 		if (nets_.size() != 1) return "the persistent GR pass runs one network";
@@ -1739,7 +1768,7 @@ std::string Simulator::planPass(const PassGeometry &g, PassPlan *p)
 	bool oneZone = true;  // and one plane of counts
 	for (Network *n : nets_)
 		oneZone = oneZone && n->dev().numZones == 1 && n->dev().nMFSlots <= 15u && n->dev().nGOSlots <= 15u;
-	p->fn = g.RW > 0 && g.S > 0 ? passTmaKernelFor(g.W, (int)stagesOf(g), oneZone) : nullptr;
+	p->fn = g.RW > 0 && g.S > 0 ? passTmaKernelFor(g.W, (int)p->S, oneZone) : nullptr;
 	if (!p->fn) return "per-tile GR-pass geometry not compiled in";
 	if (!passTmaFits(g, &p->smem)) return "the per-tile GR-pass geometry does not fit every network";
 	CK(cudaFuncSetAttribute(p->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem), "pass smem");
