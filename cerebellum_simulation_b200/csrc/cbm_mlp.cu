@@ -345,14 +345,15 @@ __global__ void prepareKernel(const float *x, uint32_t rows, uint32_t nIn, uint3
 }
 
 // Adam (Kingma and Ba, 2015) on n parameters, bias-corrected step t, and the
-// parameters' BF16 copy.
+// parameters' BF16 copy.  Not on the gradients of a product that failed, which the
+// host hears of at the end of the epoch.
 __global__ void adamKernel(float *p, const float *g, float *m, float *v, size_t n, float lr, float b1, float b2,
-		float eps, float c1, float c2, __nv_bfloat16 *h)
+		float eps, float c1, float c2, __nv_bfloat16 *h, const uint32_t *err)
 {
 	pdlLaunchDependents();
 	pdlWait();
 	const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= n) return;
+	if (i >= n || *err) return;
 	const float gi = g[i];
 	const float mi = b1 * m[i] + (1 - b1) * gi, vi = b2 * v[i] + (1 - b2) * gi * gi;
 	m[i] = mi;
@@ -745,7 +746,8 @@ int cbm_mlp_train(cbm_mlp *n, const float *x, const float *target, unsigned coun
 				const float b1 = 0.9f, b2 = 0.999f;
 				const float c1 = 1.0f - (float)std::pow(b1, (double)n->adamStep), c2 = 1.0f - (float)std::pow(b2, (double)n->adamStep);
 				MTRY(launch(n, adamKernel, dim3((unsigned)((n->nP + kThreads - 1) / kThreads)), 0, "Adam", n->P,
-						(const float *)n->G, n->Mo, n->Ve, n->nP, lr, b1, b2, 1e-8f, c1, c2, n->Wh));
+						(const float *)n->G, n->Mo, n->Ve, n->nP, lr, b1, b2, 1e-8f, c1, c2, n->Wh,
+						(const uint32_t *)n->err));
 			}
 			MCK(cudaMemcpyAsync(n->hLoss[h], n->loss, 4ull * k, cudaMemcpyDeviceToHost, n->s), "loss");
 			MCK(cudaEventRecord(n->done[h], n->s), "training");
