@@ -707,11 +707,11 @@ int cbm_mlp_train(cbm_mlp *n, const float *x, const float *target, unsigned coun
 	const size_t halfRows = std::max<size_t>(n->maxBatch, kRows / 8);
 	MCK(cudaStreamSynchronize(n->s), "training");  // a call that failed may have left copies from them
 	for (int h = 0; h < 2; h++) {
-		if (n->done[h]) continue;
-		MCK(cudaMallocHost((void **)&n->hX[h], 4 * halfRows * n->nIn), "pinned rows");
-		MCK(cudaMallocHost((void **)&n->hT[h], 4 * halfRows * n->nOut), "pinned targets");
-		MCK(cudaMallocHost((void **)&n->hLoss[h], 4 * halfRows), "pinned losses");
-		MCK(cudaEventCreateWithFlags(&n->done[h], cudaEventDisableTiming), "event");
+		// (each by itself: a call that failed between them left the others)
+		if (!n->hX[h]) MCK(cudaMallocHost((void **)&n->hX[h], 4 * halfRows * n->nIn), "pinned rows");
+		if (!n->hT[h]) MCK(cudaMallocHost((void **)&n->hT[h], 4 * halfRows * n->nOut), "pinned targets");
+		if (!n->hLoss[h]) MCK(cudaMallocHost((void **)&n->hLoss[h], 4 * halfRows), "pinned losses");
+		if (!n->done[h]) MCK(cudaEventCreateWithFlags(&n->done[h], cudaEventDisableTiming), "event");
 	}
 	double epochLoss = 0;
 	for (unsigned e = 0; e < epochs; e++) {

@@ -1,7 +1,8 @@
 // Training after a product that failed on the device reports the error and leaves
 // the parameters as they were.  The failure is an error word set from the host:
 // cudaMemcpyAsync below stands in for the runtime's and notes where the library
-// reads that word from.
+// reads that word from.  Pinned memory that runs out between the two training halves
+// fails one call, is had by the next, and all of it is given back.
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
@@ -22,6 +23,24 @@ extern "C" cudaError_t cudaMemcpyAsync(void *dst, const void *src, size_t n, cud
 	return real(dst, src, n, kind, s);
 }
 
+static int pinned = 0, pinnedLeft = -1;
+
+extern "C" cudaError_t cudaMallocHost(void **p, size_t n)
+{
+	static const auto real = (cudaError_t(*)(void **, size_t))dlsym(RTLD_NEXT, "cudaMallocHost");
+	if (pinnedLeft == 0) return cudaErrorMemoryAllocation;
+	if (pinnedLeft > 0) pinnedLeft--;
+	pinned++;
+	return real(p, n);
+}
+
+extern "C" cudaError_t cudaFreeHost(void *p)
+{
+	static const auto real = (cudaError_t(*)(void *))dlsym(RTLD_NEXT, "cudaFreeHost");
+	pinned--;
+	return real(p);
+}
+
 #define CHECK(c) do { if (!(c)) { fprintf(stderr, "%s:%d: %s\n", __FILE__, __LINE__, #c); return 1; } } while (0)
 
 int main()
@@ -37,6 +56,13 @@ int main()
 	std::vector<float> p(cbm_mlp_num_params(n)), q(p.size());
 	float loss = 0;
 	CHECK(cbm_mlp_get_params(n, p.data(), p.size()) == 0);
+	for (int k : {2, 1, 0}) {
+		pinnedLeft = k;
+		CHECK(cbm_mlp_train(n, x.data(), t.data(), rows, batch, 1, 1e-2f, 3, &loss) != 0);
+		pinnedLeft = -1;
+	}
+	CHECK(cbm_mlp_get_params(n, q.data(), q.size()) == 0);
+	CHECK(memcmp(p.data(), q.data(), 4 * p.size()) == 0);
 	CHECK(cbm_mlp_train(n, x.data(), t.data(), rows, batch, 1, 1e-2f, 3, &loss) == 0);
 	CHECK(cbm_mlp_get_params(n, q.data(), q.size()) == 0);
 	CHECK(memcmp(p.data(), q.data(), 4 * p.size()) != 0);  // it trains
@@ -47,5 +73,6 @@ int main()
 	CHECK(cbm_mlp_get_params(n, p.data(), p.size()) == 0);
 	CHECK(memcmp(p.data(), q.data(), 4 * p.size()) == 0);  // none of it was applied
 	cbm_mlp_destroy(n);
+	CHECK(pinned == 0);
 	return 0;
 }
