@@ -295,6 +295,42 @@ def cpu_reference(state_path, mf, steps, threads, warmup=0):
     return res
 
 
+def cpu_oracle(state_path, mf, steps, warmup=0):
+    """The step's C restatement (oracle/libcbm_oracle.so: the reference's host code in
+    its own operation order, no OpenMP) on one host core, for machines where the
+    reference harness is not built: at most 20 timed steps, like cpu_reference's
+    otherwise.  Returns None when the library is not built either."""
+    import ctypes
+    path = os.path.join(ROOT, "oracle", "libcbm_oracle.so")
+    if not os.path.exists(path):
+        return None
+    steps = min(steps, 20)
+    if len(mf) < warmup + steps:
+        raise ValueError(f"the CPU sample needs {warmup + steps} MF rows, the stream has {len(mf)}")
+    lib = ctypes.CDLL(path)
+    lib.cbm_oracle_load.restype = ctypes.c_void_p
+    lib.cbm_oracle_load.argtypes = [ctypes.c_char_p, ctypes.c_char_p, ctypes.c_size_t]
+    lib.cbm_oracle_free.argtypes = [ctypes.c_void_p]
+    lib.cbm_oracle_set_seeds.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
+    lib.cbm_oracle_run.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint64, ctypes.c_void_p]
+    err = ctypes.create_string_buffer(256)
+    o = lib.cbm_oracle_load(os.fsencode(state_path), err, 256)
+    if not o:
+        raise RuntimeError(f"the oracle refused the state: {err.value.decode()}")
+    rows = np.ascontiguousarray(mf[:warmup + steps], dtype=np.uint8)
+    seeds = np.array([7], dtype=np.int32)
+    lib.cbm_oracle_set_seeds(o, seeds.ctypes.data)
+    lib.cbm_oracle_run(o, rows.ctypes.data, warmup, None)
+    t0 = time.perf_counter()
+    lib.cbm_oracle_run(o, rows[warmup:].ctypes.data, steps, None)
+    s = time.perf_counter() - t0
+    lib.cbm_oracle_free(o)
+    return {"value": steps / s, "unit": "steps/s", "cores": 1, "kind": "oracle",
+            "sample": f"{steps} steps of the same 1M-GR network and MF input (ms {warmup}-{warmup + steps} of "
+                      f"trial 1, after {warmup} untimed steps), C restatement of the reference's step, one core "
+                      "(the reference harness is not built here)"}
+
+
 WORKLOAD = ("1M-GR eyelid network: 1,048,576 GR (4 MF + 3 GO inputs, 4 GO targets each), 1024 GO, 1024 MF, "
             "32 PC x 32,768 PF, 128 BC, 512 SC, 8 NC, 4 IO; CS 2000-2500 of 5000-step trials, US at CS offset, "
             "PF->PC LTD/LTP on")
@@ -583,7 +619,8 @@ def main_dense4m(args):
             p = os.path.join(d, "c3.state")
             st.writeState(p)
             try:
-                cpu = cpu_reference(p, mf, 40, os.cpu_count() or 1, warmup=5)
+                cpu = (cpu_reference(p, mf, 40, os.cpu_count() or 1, warmup=5) or
+                       cpu_oracle(p, mf, 5, warmup=2))
             except (RuntimeError, ValueError) as e:
                 cpu = {"error": str(e)}
             if cpu and "error" not in cpu:
@@ -752,7 +789,8 @@ def main():
             p = os.path.join(d, "c2.state")
             st.writeState(p)
             try:
-                cpu = cpu_reference(p, mf, CPU_STEPS, os.cpu_count() or 1, warmup=CPU_WARMUP)
+                cpu = (cpu_reference(p, mf, CPU_STEPS, os.cpu_count() or 1, warmup=CPU_WARMUP) or
+                       cpu_oracle(p, mf, CPU_STEPS, warmup=CPU_WARMUP))
             except (RuntimeError, ValueError) as e:
                 cpu_error = str(e)
 
