@@ -1137,7 +1137,7 @@ __device__ void zoneRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm,
 		const float errDrive = task == tid ? errOwn : errDriveOf(N, t, z);
 		const uint32_t apBuf = Q.apBufIO[i];
 		float gNCSum = 0;
-#pragma unroll 1
+#pragma unroll 4
 		for (uint32_t j = 0; j < nIONC; j++) gNCSum = gNCSum + ioScratch[(size_t)task * nIONC + j];
 		gNCSum = gNCSum / 3.1;
 		float v = v0;
@@ -1244,7 +1244,7 @@ __device__ void zoneRole(const DevNet *__restrict__ N, uint64_t t, uint32_t *sm,
 				const int32_t timer = Q.pfPCPlastTimerIO[i];
 				const float vOwn = Q.vIO[i];
 				float vc = 0;
-#pragma unroll 1
+#pragma unroll 4
 				for (uint32_t j = 0; j < N->numpIOInIOIO; j++)
 					vc = vc + N->coupleRiRjRatioIO * (Q.vIO[Q.pIOInIOIO[(size_t)i * N->numpIOInIOIO + j]] - vOwn);
 				const int32_t tm = (!ap) * (timer + 1) + ap * N->tsLTDStartAPIO;
@@ -1782,6 +1782,10 @@ __device__ void publishNC(const DevNet *N, uint64_t t, uint8_t *box)
 // from L2, or from DRAM after an L2 flush: a flushed step took 24.0 us on 16K and
 // 64K GR and 25.5 on 1M, so 19.5, 18.7 and 22.8; back to back 11.8 on 16K and 12.7
 // on 1M, so 11.0 and 12.3.
+// The IO sums stay unrolled by four: rolled, their loads went one by one, and a step with
+// 32 IOs took 13.8 us (12.9 before the loops were rolled; so 12.8), two zones of 16 IOs
+// 26.7 (24.6; 25.0), one network of 32 NCs and 8 IOs 14.0 (14.2; 13.3).  More warps for
+// the release draws or probabilities were no faster there: the outputs had fewer.
 __global__ void __launch_bounds__(kTailThreads, 1) tailKernel(const DevNet *const *nets, const uint32_t *stageBytes,
 		uint32_t stepOffset, const DevNet *net0, uint32_t stage0, uint8_t *ncMailbox, const __grid_constant__ MFParam mfp)
 {
