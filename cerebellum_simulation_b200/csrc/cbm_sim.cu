@@ -576,18 +576,17 @@ size_t Network::tailSmemBytes() const
 
 double Network::bytesPerStepAlgorithmic() const
 {
-	return (72.0 + 4.0 * avgMF_ + 4.0 * avgGO_ + 8.0 * avgOut_) * h_.numGR;
+	// what no pass can do without: six 4-byte state arrays in and out, the PF delay,
+	// every zone's weight; history read + write and weight writes on plasticity steps
+	return (49.0 + 4.0 * h_.numZones + (16.0 + 4.0 * h_.numZones) / h_.tsPerHistBinGR) * h_.numGR;
 }
 
 double Network::bytesPerStepLayout() const
 {
-	// GR state read and written (6 x 4 B each way), the PF delay byte, the
-	// PF->PC weight of every zone; history read + write and weight writes on
-	// plasticity steps; the synapse tables (u16 MF and GO indices, u32 GR->GO
-	// slots) where the pass streams them, else the counts of arrived spikes
-	const double slots = streamsSlots_ ? 2.0 * h_.nMFSlots + 2.0 * h_.nGOSlots + 4.0 * h_.nOutSlots : 2.0;
-	const double perGR = 48.0 + slots + 1.0 + 4.0 * h_.numZones + (16.0 + 4.0 * h_.numZones) / h_.tsPerHistBinGR;
-	return perGR * h_.numGR;
+	// beside those the synapse tables (u16 MF and GO indices, u32 GR->GO slots) where the
+	// pass streams them, else the counts of arrived spikes, read and written
+	const double slots = streamsSlots_ ? 2.0 * h_.nMFSlots + 2.0 * h_.nGOSlots + 4.0 * h_.nOutSlots : 2.0 * h_.evPlanes;
+	return bytesPerStepAlgorithmic() + slots * h_.numGR;
 }
 
 std::string checkNetwork(const State &st)
@@ -750,13 +749,10 @@ std::string Network::build(State *st, const std::vector<int> &seeds, uint32_t mf
 	const uint32_t *pfMask = A("pGRDelayMaskfromGRtoBSP")->as<uint32_t>();
 	const uint32_t strideGO = c.maxnumpGRfromGOtoGR, strideOut = c.maxnumpGRfromGRtoGO;
 	uint32_t nMF = 0, nGO = 0, nOut = 0;
-	uint64_t sumMF = 0, sumGO = 0, sumOut = 0;
 	for (uint32_t g = 0; g < N; g++) {
 		nMF = std::max<uint32_t>(nMF, numMFin[g]); nGO = std::max<uint32_t>(nGO, numGOin[g]);
 		nOut = std::max<uint32_t>(nOut, numOut[g]);
-		sumMF += numMFin[g]; sumGO += numGOin[g]; sumOut += numOut[g];
 	}
-	avgMF_ = (double)sumMF / N; avgGO_ = (double)sumGO / N; avgOut_ = (double)sumOut / N;
 	h.nMFSlots = nMF; h.nGOSlots = nGO; h.nOutSlots = nOut;
 	std::vector<uint16_t> mfIdx((size_t)std::max(1u, nMF) * N, (uint16_t)c.numMF);
 	std::vector<uint16_t> goIdx((size_t)std::max(1u, nGO) * N, (uint16_t)c.numGO);

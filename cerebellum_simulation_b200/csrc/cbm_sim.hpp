@@ -288,7 +288,7 @@ public:
 	static constexpr size_t kTailSmemBudget = 200 * 1024;
 	uint32_t mfWords() const { return h_.mfWords; }
 	uint32_t mfRing() const { return h_.mfRing; }
-	double bytesPerStepAlgorithmic() const;  // 72 + 4 n_mf + 4 n_go + 8 n_out per GR
+	double bytesPerStepAlgorithmic() const;  // what no pass can do without (see cbm_sim_algorithmic_bytes_per_step)
 	double bytesPerStepLayout() const;       // what this layout moves (see cbm_sim_layout_bytes_per_step)
 
 	HostCtl ctl{};
@@ -311,7 +311,6 @@ private:
 	DevProtocol hProto_{};  // host copy of the protocol descriptor
 	std::vector<void *> allocs_;
 	std::map<const void *, size_t> allocBytes_;
-	double avgMF_ = 0, avgGO_ = 0, avgOut_ = 0;
 	bool streamsSlots_ = true;  // the GR pass in use streams the synapse tables (not the per-tile pass)
 	void *evArena_[2] = {};     // what holds the event tables in use
 	bool evMode_ = false;       // the state is in the per-tile pass's form (setEventMode)

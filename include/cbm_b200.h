@@ -421,14 +421,16 @@ int cbm_sim_run_flushed_kernels(cbm_sim *sim, uint64_t nsteps, uint64_t flushByt
  * last cbm_sim_run that timed the GR pass (0 before). */
 int cbm_sim_last_tail_ms(cbm_sim *sim, float *ms);
 
-/* Algorithmic HBM bytes of one step: (72 + 4 n_mf + 4 n_go + 8 n_out) per GR
- * with the network's mean synapse counts. */
+/* HBM bytes that no pass over the GRs can do without in one step: the six 4-byte
+ * state arrays read and written, the PF delay and every zone's weight read,
+ * history read and written and weights written every tsPerHistBinGR steps,
+ * averaged.  A GR's synapses need be touched only when a spike arrives: they are
+ * not counted. */
 double cbm_sim_algorithmic_bytes_per_step(cbm_sim *sim);
 
-/* Bytes the GR pass moves per step with this library's layout (16-bit
- * synapse indices, 8-bit delays, packed GR->GO targets): reads and writes of
- * the GR state, indices, delays and weights, history and weight writes every
- * tsPerHistBinGR steps averaged.  No counterpart in the reference. */
+/* Bytes the GR pass in use streams per step: those above, and the synapse tables
+ * (16-bit indices, packed GR->GO targets) or, with the per-tile pass, the counts of
+ * arrived spikes.  No counterpart in the reference. */
 double cbm_sim_layout_bytes_per_step(cbm_sim *sim);
 
 /* Which GR-pass kernel runs: *kind 0 = plain (one warp-row per load), 1 =
