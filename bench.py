@@ -217,6 +217,12 @@ def measured_peak():
     return 6650.0, "fallback"
 
 
+def mailbox_bytes(num_nc):
+    """What a single step writes to mapped host memory: the step stamp with the NC
+    spikes in it (up to 16), or with a byte for each behind it."""
+    return 8 if num_nc <= 16 else 8 + num_nc
+
+
 def profiled_traffic():
     """Per-launch DRAM bytes of the GR pass from the committed ncu summary."""
     p = os.path.join(ROOT, "profiles", "gr_pass_1M_eyelid.md")
@@ -609,8 +615,7 @@ def main_dense4m(args):
         sim3.calcActivity()
         zone.exportAPNC()
     e2e_ms = sim3.timer_stop()
-    # the NC spikes and the 8-byte step stamp the small-cell kernel writes to mapped host memory
-    h2d, d2h = sim3.mf_words() * 4, st.con("numNC") + 8
+    h2d, d2h = sim3.mf_words() * 4, mailbox_bytes(st.con("numNC"))
     sim3.close()
 
     cpu = None
@@ -780,7 +785,7 @@ def main():
     e2e_ms, = replicas.max_over_ranks(dist, [e2e_ms], device=f"cuda:{device}")
     e2e = replicas.throughput(world, n_e2e, e2e_ms)
     h2d = sim3.mf_words() * 4
-    d2h = st.con("numNC") + 8  # NC spikes and the step stamp, written to mapped host memory
+    d2h = mailbox_bytes(st.con("numNC"))
     sim3.close()
 
     cpu, cpu_error = None, None

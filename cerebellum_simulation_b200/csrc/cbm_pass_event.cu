@@ -7,8 +7,8 @@
 // in a step.  So the synapse tables are not streamed.  They are kept by source:
 //   MF->GR and GO->GR: per block of evCells cells, each source's list of
 //     target cells (evStart, evEntry).  An event CTA walks the lists of the
-//     step's spiking sources and counts into half a byte per cell and kind in
-//     shared memory; the counts are the integers the per-cell gather of
+//     step's spiking sources and counts into half a byte per cell and kind (a
+//     byte with more than 15 inputs of a kind) in shared memory; the counts are the integers the per-cell gather of
 //     kernels.cu:169-199 gives.
 //   GR->GO: a cell's spike adds its synapses to the counts of the step they
 //     arrive in, t + delay, in a ring of kGoRing steps (outCell).  The
@@ -23,14 +23,14 @@
 // cells are consecutive, so a CTA streams a few long pieces by bulk copies.
 //
 // What bounds it: on up to 1M GR, latency (a CTA's prologue, its 2-4 rounds and
-// its sums, 8-9 us, which the small-cell kernel's 11 us cover); beyond, the
-// streaming (63 us a step on the dense 4M network, 38 us of them the bytes at the
-// measured copy bandwidth).
+// its sums, 11-13 us beside the small-cell kernel's 11); beyond, the streaming
+// (53 us of the dense 4M network's 67 us step, 38 of them the bytes at the measured
+// copy bandwidth) and there the Golgi CTA beside it.
 // Streaming the tables instead (14 B of indices and 8-16 B of GR->GO slots a
-// cell, with seven gathers and four delay tests), a step took 83 us on the
-// dense 4M-GR network (here 65), 80 us on 64 networks of 16K GR, whose 128-cell
-// tiles were prologue only (24), 78 us on six of 256K-2M (58), 16.5 us on 1M GR
-// (13.6).  Other homes for the lists that were measured: each CTA's
+// cell, with seven gathers and four delay tests), a step took 93 us on the
+// dense 4M-GR network (here 67), 92 us on 64 networks of 16K GR, whose 128-cell
+// tiles were prologue only (33), 83 us on six of 256K-2M (62), 15.6 us on 1M GR
+// (13.1).  Other homes for the lists that were measured: each CTA's
 // own 2048 cells (a GO's list has 1.5 cells there on the 4M network: as long
 // again as the streaming), and counts in global memory (random reductions there
 // slow the streaming stores: 29 us a step on the 1M network).
