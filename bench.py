@@ -303,14 +303,14 @@ def cpu_reference(state_path, mf, steps, threads, warmup=0):
 
 def cpu_oracle(state_path, mf, steps, warmup=0):
     """The step's C restatement (oracle/libcbm_oracle.so: the reference's host code in
-    its own operation order, no OpenMP) on one host core, for machines where the
-    reference harness is not built: at most 20 timed steps, like cpu_reference's
-    otherwise.  Returns None when the library is not built either."""
+    its own operation order, the GR loops under OpenMP) on host cores, for machines
+    where the reference harness is not built: at most 40 timed steps, like
+    cpu_reference's otherwise.  Returns None when the library is not built either."""
     import ctypes
     path = os.path.join(ROOT, "oracle", "libcbm_oracle.so")
     if not os.path.exists(path):
         return None
-    steps = min(steps, 20)
+    steps = min(steps, 40)
     if len(mf) < warmup + steps:
         raise ValueError(f"the CPU sample needs {warmup + steps} MF rows, the stream has {len(mf)}")
     lib = ctypes.CDLL(path)
@@ -331,10 +331,11 @@ def cpu_oracle(state_path, mf, steps, warmup=0):
     lib.cbm_oracle_run(o, rows[warmup:].ctypes.data, steps, None)
     s = time.perf_counter() - t0
     lib.cbm_oracle_free(o)
-    return {"value": steps / s, "unit": "steps/s", "cores": 1, "kind": "oracle",
+    threads = ctypes.CDLL("libgomp.so.1").omp_get_max_threads()  # the OpenMP runtime the oracle is linked to
+    return {"value": steps / s, "unit": "steps/s", "cores": threads, "kind": "oracle",
             "sample": f"{steps} steps of the same 1M-GR network and MF input (ms {warmup}-{warmup + steps} of "
-                      f"trial 1, after {warmup} untimed steps), C restatement of the reference's step, one core "
-                      "(the reference harness is not built here)"}
+                      f"trial 1, after {warmup} untimed steps), C restatement of the reference's step, OpenMP {threads} "
+                      "threads (the reference harness is not built here)"}
 
 
 WORKLOAD = ("1M-GR eyelid network: 1,048,576 GR (4 MF + 3 GO inputs, 4 GO targets each), 1024 GO, 1024 MF, "
@@ -625,7 +626,7 @@ def main_dense4m(args):
             st.writeState(p)
             try:
                 cpu = (cpu_reference(p, mf, 40, os.cpu_count() or 1, warmup=5) or
-                       cpu_oracle(p, mf, 5, warmup=2))
+                       cpu_oracle(p, mf, 40, warmup=5))
             except (RuntimeError, ValueError) as e:
                 cpu = {"error": str(e)}
             if cpu and "error" not in cpu:
