@@ -185,8 +185,8 @@ __device__ void colSums(const GemmJob &J, float *s)
 // waiting for its loads and its MMAs, on one or two CTAs took 30-62 us a product;
 // transposed copies of the operands, the ReLU derivative and the loss were
 // launches of their own.  A 64-256-256-50 network's gradients over 200 rows took
-// 518 us and take 139, a training minibatch of 256 took 482 and takes 67, a
-// forward pass over 4096 rows 3620 and 205 (copies to and from the host included).
+// 523 us and take 143, a training minibatch of 256 took 484 and takes 68, a
+// forward pass over 4096 rows 3670 and 215 (copies to and from the host included).
 __global__ void __launch_bounds__(kThreads) gemmKernel(const __grid_constant__ GemmJobs jobs, uint32_t *err)
 {
 	pdlLaunchDependents();

@@ -68,7 +68,7 @@ template <int V> __device__ __forceinline__ Words<V> loadWords(const uint32_t *p
 // and one thread a column then adds the terms in order from shared memory.  A
 // thread a column walking its rows, and the tree as a launch of its own behind
 // scratch in global memory, took 14.3 us on 32 PCs of 32,768 fibres; this takes
-// 8.2, launch included.
+// 8.4, launch included.
 template <int V>
 __global__ void __launch_bounds__(kThreads) pfpcSumsKernel(const uint32_t *apBuf, const uint32_t *mask, const float *w,
 		uint32_t P, uint32_t bs, uint32_t cols, float *sums)
